@@ -316,7 +316,11 @@ void solver_setup(Krylov& k, int32_t n_pad, int device);
 // Runs the grid barrier with one block that never arrives on `blocks`
 // blocks; reports how many gave up, the status word and the kernel time.
 int selftest_wait_limit(int blocks, int* gave_up, int* status, float* ms);
+// ----------------------------------------------------------------- cg64.cu
+// Blocks the FP64 solve may use on the device (0: it does not fit).
+int cg64_grid(int device);
 // Solves A x = b; returns through DevStats (iterations, residual, status).
+// A.val32 is scratch of this solve.
 void launch_solve_fp64(const Consts& c, const Ppe& A, const Krylov& k, double tol,
                        int64_t max_iter, DevStats* ds, cudaStream_t st);
 // warm: x already holds the initial guess (launch_mixed_setup), else the

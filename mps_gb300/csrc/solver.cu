@@ -1,6 +1,7 @@
 // Pressure Poisson solve (src/mps.cpp:417-470).
 //
-// Both solvers are persistent cooperative kernels: one launch per solve, the
+// The mixed-precision solvers (the FP64 one is in cg64.cu) are persistent
+// cooperative kernels: one launch per solve, the
 // blocks stay resident and meet at grid barriers between the phases of an
 // iteration, and the convergence test runs on the device.  A dot product is
 // reduced per block, written as one partial per block, and summed in a fixed
@@ -8,12 +9,6 @@
 // before it releases the others; results are therefore run-to-run
 // deterministic and every block takes the same branch.
 //
-//  * FP64 (k_cg64): the Jacobi-preconditioned CG that Eigen's
-//    ConjugateGradient runs with its defaults (zero start, stop when
-//    ||r||^2 < max(tol^2 ||b||^2, DBL_MIN) on the recursive residual, cap 2n),
-//    over the SELL-32 FP64 matrix; three phases per iteration as Eigen's loop
-//    is written.  Roofline: HBM (12 B per stored entry and iteration) and FP64
-//    issue (one DFMA per entry).
 //  * MIXED (k_cg_mixed): iterative refinement.  x and the residual
 //    r = b - A x stay FP64 (FP64 matrix); each correction A d = r is solved
 //    by Jacobi CG in the Chronopoulos-Gear arrangement (one fused reduction
@@ -500,106 +495,6 @@ __device__ __forceinline__ void off_rows(const Ppe& A, const MatFree& mf, int K,
     }
     o = fa ? spmv32_sell_row(A, K, i, v, vi) : compact_row_sum(A, mf, K, i, v, vi);
     o2 = i2 < 0 ? 0.f : (fb ? spmv32_sell_row(A, K, i2, v, vi2) : compact_row_sum(A, mf, K, i2, v, vi2));
-}
-
-// ----------------------------------------------------------------- FP64 CG
-// A step whose matrix failed the symmetry test skips its solve (the
-// reference exits there); every block reads the flag, set before the launch.
-__device__ __forceinline__ bool solve_skipped(DevStats* ds) {
-    if (!(*(volatile int32_t*)&ds->status & ST_ASYMMETRIC)) return false;
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        ds->cg_iterations = 0;
-        ds->refinements = 0;
-        ds->cg_rel_residual = -1.0;
-    }
-    return true;
-}
-
-__global__ void __launch_bounds__(kBlock, 1) k_cg64(Ppe A, Krylov kv, SolveArgs a, DevStats* ds) {
-    if (solve_skipped(ds)) return;
-    GridBar gb = whole_grid(kv);
-    const int lane = threadIdx.x & 31;
-    const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-
-    double acc[1] = {0.0}, tot[1];
-    for (int sl = gwarp; sl < a.nslices; sl += nwarps) {
-        int i = sl * 32 + lane;
-        if (i >= a.n) continue;
-        double d = A.diag[i];
-        kv.inv_diag[i] = d != 0.0 ? 1.0 / d : 1.0;
-        double b = A.src[i];
-        kv.x[i] = 0.0;
-        kv.r[i] = b;
-        acc[0] = fma(b, b, acc[0]);
-    }
-    if (!reduce_sync<1, kBlock>(gb, acc, tot, ds)) return;
-    const double rhs2 = tot[0];
-    int64_t it = 0;
-    double rn2 = rhs2;
-    bool conv = true;
-    if (rhs2 > 0.0) {
-        const double thr = fmax(a.tol * a.tol * rhs2, DBL_MIN);
-        if (!(rn2 < thr)) {
-            double a1[1] = {0.0}, t1[1];
-            for (int sl = gwarp; sl < a.nslices; sl += nwarps) {
-                int i = sl * 32 + lane;
-                if (i >= a.n) continue;
-                double r = kv.r[i];
-                double p = kv.inv_diag[i] * r;
-                kv.p[i] = p;
-                a1[0] = fma(r, p, a1[0]);
-            }
-            if (!reduce_sync<1, kBlock>(gb, a1, t1, ds)) return;
-            double abs_new = t1[0];
-            while (it < a.max_iter) {
-                double a2[1] = {0.0}, t2[1];
-                for (int sl = gwarp; sl < a.nslices; sl += nwarps) {
-                    int i = sl * 32 + lane;
-                    if (i >= a.n) continue;
-                    double pi = kv.p[i];
-                    double q = spmv64_row(A, a.K, sl, lane, i, kv.p, pi);
-                    kv.q[i] = q;
-                    a2[0] = fma(pi, q, a2[0]);
-                }
-                if (!reduce_sync<1, kBlock>(gb, a2, t2, ds)) return;
-                const double alpha = abs_new / t2[0];
-                double a3[2] = {0.0, 0.0}, t3[2];
-                for (int sl = gwarp; sl < a.nslices; sl += nwarps) {
-                    int i = sl * 32 + lane;
-                    if (i >= a.n) continue;
-                    kv.x[i] = fma(alpha, kv.p[i], kv.x[i]);
-                    double r = fma(-alpha, kv.q[i], kv.r[i]);
-                    kv.r[i] = r;
-                    double z = kv.inv_diag[i] * r;
-                    kv.z[i] = z;
-                    a3[0] = fma(r, r, a3[0]);
-                    a3[1] = fma(r, z, a3[1]);
-                }
-                if (!reduce_sync<2, kBlock>(gb, a3, t3, ds)) return;
-                rn2 = t3[0];
-                if (rn2 < thr) break;
-                const double beta = t3[1] / abs_new;
-                abs_new = t3[1];
-                for (int sl = gwarp; sl < a.nslices; sl += nwarps) {
-                    int i = sl * 32 + lane;
-                    if (i >= a.n) continue;
-                    kv.p[i] = fma(beta, kv.p[i], kv.z[i]);
-                }
-                it++;
-                if (!grid_sync(gb, ds)) return;
-            }
-        }
-        conv = rn2 < thr;
-    } else {
-        rn2 = 0.0;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        ds->cg_iterations = it;
-        ds->refinements = 0;
-        ds->cg_rel_residual = rhs2 > 0.0 ? sqrt(rn2 / rhs2) : 0.0;
-        if (!conv) atomicOr(&ds->status, ST_NOT_CONVERGED);
-    }
 }
 
 // --------------------------------------------------------------- mixed IR
@@ -1763,7 +1658,7 @@ SolveArgs make_args(const Consts& c, double tol, int64_t max_iter) {
 }  // namespace
 
 void solver_setup(Krylov& k, int32_t /*n_pad*/, int device) {
-    int g1 = coop_grid((const void*)k_cg64, device, kBlock, 0, 1);
+    int g1 = cg64_grid(device);
     int g2 = coop_grid((const void*)k_cg_mixed, device, kMixedBlock, 0, 1);
     int g3 = coop_grid((const void*)k_cg_mixed_ov, device, kMixedBlock, 0, 1);
     k.grid = std::min({g1, g2, g3});
@@ -1777,17 +1672,6 @@ void launch_mixed_setup(const Consts& c, const SortScratch& sc, const Ppe& A, Ma
     mf.numY = c.numY;
     mf.nkeys = c.nkeys;
     k_mixed_setup<<<(c.n + 255) / 256, 256, 0, st>>>(c, A, mf, k, ids, warm ? 1 : 0, &ds->sym_fp);
-    ++g_launches;
-}
-
-void launch_solve_fp64(const Consts& c, const Ppe& A, const Krylov& k, double tol,
-                       int64_t max_iter, DevStats* ds, cudaStream_t st) {
-    SolveArgs a = make_args(c, tol, max_iter);
-    Ppe AA = A;
-    Krylov kk = k;
-    void* args[] = {&AA, &kk, &a, &ds};
-    cudaMemsetAsync(k.barrier, 0, sizeof(unsigned int), st);
-    cudaLaunchCooperativeKernel((const void*)k_cg64, dim3(k.grid), dim3(kBlock), args, 0, st);
     ++g_launches;
 }
 
