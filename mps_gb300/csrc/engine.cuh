@@ -269,6 +269,7 @@ struct Mg {
     int32_t enabled;
     int32_t nlev;   // coarse levels 1..nlev
     int32_t ngrid;  // levels 1..ngrid run grid-wide; ngrid+1..nlev run in block 0
+    int32_t lred;   // overlapped solve: levels lred..nlev run in every block (solver.cu, split cycle)
     MgLevel lev[kMgMaxLevels];
     float* e0;      // level-0 correction (per slot)
     float* res0;    // level-0 residual (per slot)
@@ -310,6 +311,7 @@ struct Krylov {
     unsigned int* barrier;  // monotonically increasing arrival counter
     double* totals;         // unused scratch (8 doubles)
     int32_t grid;           // cooperative grid size
+    int32_t cluster;        // blocks of a one-cluster solve (0: the device runs none)
     int32_t block;
 };
 void solver_setup(Krylov& k, int32_t n_pad, int device);

@@ -201,7 +201,7 @@ __device__ __forceinline__ bool reduce_sync(GridBar& gb, const double (&v)[M], d
 // of a block-and-grid reduction in FP64 cost ~7 us per iteration on the
 // critical path; the pair sums keep ~44 bits, far more than an FP32 Krylov
 // iteration needs.
-struct F2 {
+struct __align__(8) F2 {  // (8-byte stores: cluster_reduce_f2)
     float hi, lo;
 };
 
@@ -297,6 +297,88 @@ __device__ __forceinline__ bool reduce_sync_f2(GridBar& gb, const F2 (&v)[M], fl
     if (!grid_sync(gb, ds)) return false;
     sum_partials_f2<M>(gb, part, tot);
     return true;
+}
+
+// ------------------------------------------------------- one-cluster solves
+// The blocks of a small scene's solve are one thread-block cluster: its
+// hardware barrier takes a fraction of a grid barrier's trips through L2, and
+// the sums of an iteration go straight into the other blocks' shared memory.
+// Blocks of a cluster are always co-resident, and every block takes the same
+// branches (bitwise the same totals), so the barrier needs no wait limit.
+constexpr int kClusterMax = 16;
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ void st_remote(const F2* local, int rank, F2 v) {
+    unsigned a = (unsigned)__cvta_generic_to_shared(local), r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(r), "f"(v.hi), "f"(v.lo) : "memory");
+}
+
+// reduce_sync_f2 within a cluster: every block stores its M pairs into its
+// slot of every block, and after the barrier each block adds the slots in
+// rank order.  Two slot sets in turn, as with the partials in global memory.
+template <int M, int BS>
+__device__ __forceinline__ void cluster_reduce_f2(GridBar& gb, const F2 (&v)[M], float (&tot)[M]) {
+    constexpr int kW = BS / 32;
+    __shared__ F2 sh[M][kW];
+    __shared__ F2 slots[2][M][kClusterMax];
+    __shared__ float s_tot[M];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, par = gb.parity;
+    gb.parity ^= 1;
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+        F2 a = v[m];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a = f2_add(a, f2_shfl_down(a, o));
+        if (lane == 0) sh[m][warp] = a;
+    }
+    __syncthreads();
+    if (warp < M) {
+        F2 a = lane < kW ? sh[warp][lane] : F2{0.f, 0.f};
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a = f2_add(a, f2_shfl_down(a, o));
+        a = F2{__shfl_sync(0xffffffffu, a.hi, 0), __shfl_sync(0xffffffffu, a.lo, 0)};
+        if (lane < gb.size) st_remote(&slots[par][warp][gb.rank], lane, a);
+    }
+    cluster_barrier();
+    if (warp < M) {
+        F2 a = lane < gb.size ? slots[par][warp][lane] : F2{0.f, 0.f};
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a = f2_add(a, f2_shfl_down(a, o));
+        if (lane == 0) s_tot[warp] = a.hi + a.lo;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < M; m++) tot[m] = s_tot[m];
+}
+
+// The barrier and the sums of a solve's blocks: a grid's (CL false) or a cluster's.
+template <bool CL>
+__device__ __forceinline__ bool solve_sync(GridBar& gb, DevStats* ds) {
+    if constexpr (CL) {
+        cluster_barrier();
+        return true;
+    } else {
+        return grid_sync(gb, ds);
+    }
+}
+template <bool CL, int BS>
+__device__ __forceinline__ bool solve_reduce(GridBar& gb, const double (&v)[1], double (&tot)[1], DevStats* ds) {
+    const double* part = publish_partials<1, BS>(gb, v);
+    if (!solve_sync<CL>(gb, ds)) return false;
+    sum_partials<1>(gb, part, tot);
+    return true;
+}
+template <bool CL, int BS>
+__device__ __forceinline__ bool solve_reduce_f2(GridBar& gb, const F2 (&v)[3], float (&tot)[3], DevStats* ds) {
+    if constexpr (CL) {
+        cluster_reduce_f2<3, BS>(gb, v, tot);
+        return true;
+    } else {
+        return reduce_sync_f2<3, BS>(gb, v, tot, ds);
+    }
 }
 
 // ------------------------------------------------------------------ SpMV
@@ -742,6 +824,346 @@ __device__ __forceinline__ void mg_level1_plain(const Mg& mg, const MatFree& mf,
             }
         }
     }
+}
+
+// ------------------------------------------------------------- split cycle
+// The cell levels of the overlapped solve's V-cycle with as few exchanges
+// between blocks as the data needs.  Down to level lr = mg.lred the levels are
+// restricted grid-wide, one barrier each.  From lr on every block runs the
+// levels for itself in shared memory (a few thousand cells: less than the
+// barriers they would take).  On the way up a block smooths only the cells
+// that its own rows' corrections depend on: the 3x3 cells around its rows' and,
+// on the levels above, the parents of those and of their neighbours.  So the
+// way up has no barrier at all, and level 1's correction ends in shared memory,
+// where the rows read it.  Same arithmetic per cell as mg_cell_levels (a cell
+// smoothed by two blocks gets the same bits in both).  Bound by the latency of
+// its chain of phases; measured per inner iteration, with a barrier for each
+// level and direction before: 45,000 particles (3 barriers instead of 9) 41 ->
+// 27 us, 100,000 50 -> 37 us, 1M (6 instead of 14) 117 -> 108 us, of which the
+// cycle takes 76 -> 54 us.
+//
+// Shared memory (floats): per level >= lr its r, e and t, one level after
+// another (cells without unknowns stay 0 from the kernel's start), then per
+// level lr-1 .. 1 the block's corrected cells, and at the end the lists of the
+// cells that the block smooths.  Corrected cells that do not fit (a block whose
+// unknowns lie far apart) go to the level's t array in global memory: blocks
+// that overlap there store the same bits, and each reads only what it stored.
+// A list that does not fit is replaced by the level's list of all cells.
+constexpr int kCycleList = 4608;
+struct CyclePatch {
+    int list[kMgMaxLevels], count[kMgMaxLevels];  // the block's cells of the level (list -1: all with unknowns)
+    int lo[kMgMaxLevels], off[kMgMaxLevels];      // levels < lr: first cell and first float (-1: global) of the patch
+    // Operator data kept in shared memory for the solve, as far as it fits
+    // (first float, -1: read from global memory): the dense inverse; per level
+    // > lr the restriction weights of its cells, dn = [16 weights, invd, (x, y)]
+    // by position in the level's list; per level the stencils of the block's
+    // cells, up = [9 taps, invd, (x, y)] by position in the block's list.  The
+    // cycle's phases are short chains of dependent loads, several times as
+    // long from L2 behind the operator pass's traffic as from here.
+    int dense, dn[kMgMaxLevels], up[kMgMaxLevels];
+};
+
+// Plans the block's patches: marks the 3x3 cells around its unknowns in a bit
+// per cell, lists the marked cells with unknowns, marks the parents of those
+// and their neighbours on the next level, and so on.  All threads.
+template <int BS>
+__device__ __forceinline__ void plan_patches(const Ppe& A, const Mg& mg, const MatFree& mf, int sl0, int sl1, int n,
+                                             float* __restrict__ sm, int floats, CyclePatch& cp) {
+    __shared__ int s_cnt, s_lo, s_hi;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned* bits = reinterpret_cast<unsigned*>(sm);
+    int* list = reinterpret_cast<int*>(sm + floats - kCycleList);
+    const int room = floats - kCycleList;
+    int next = 0;  // the next patch's first float
+    for (int l = mg.lred; l <= mg.nlev; l++) next += 3 * mg.lev[l].nx * mg.lev[l].ny;
+    int used = 0;  // list entries
+    bool all = false;
+    for (int l = 1; l < mg.nlev; l++) {
+        const MgLevel& L = mg.lev[l];
+        const int cells = L.nx * L.ny, words = (cells + 31) >> 5;
+        int cnt = __ldg(mg.nact + l), lo = 0, hi = cells - 1;
+        if (!all) {
+            if (tid == 0) {
+                s_cnt = 0;
+                s_lo = cells;
+                s_hi = -1;
+            }
+            // (a grid of more cells than bits: in windows)
+            for (int w0 = 0; w0 < words; w0 += room) {
+                const int nw = min(words - w0, room);
+                for (int k = tid; k < nw; k += BS) bits[k] = 0u;
+                __syncthreads();
+                auto mark = [&](int x, int y) {
+                    const int I = x * L.ny + y - w0 * 32;
+                    if (I < 0 || I >= nw * 32) return;
+                    const unsigned m = 1u << (I & 31);
+                    if (!(*(volatile unsigned*)(bits + (I >> 5)) & m)) atomicOr(bits + (I >> 5), m);
+                };
+                if (l == 1) {
+                    for (int sl = sl0 + warp; sl < sl1; sl += BS / 32) {
+                        const int i = sl * 32 + lane;
+                        const int key = i < n && A.diag32[i] > 0.f ? __ldg(mf.skey + i) : -1;
+                        const int before = __shfl_up_sync(0xffffffffu, key, 1);
+                        if (key >= 0 && (lane == 0 || key != before)) {  // an unknown's cell is interior
+                            const int x = key / L.ny, y = key - x * L.ny;
+#pragma unroll
+                            for (int d = 0; d < 9; d++) mark(x + d / 3 - 1, y + d % 3 - 1);
+                        }
+                    }
+                } else {
+                    const MgLevel& F = mg.lev[l - 1];
+                    for (int q = tid; q < cp.count[l - 1]; q += BS) {
+                        const int I = list[cp.list[l - 1] + q];
+                        const int x = I / F.ny, y = I - x * F.ny;
+#pragma unroll
+                        for (int d = 0; d < 9; d++)
+                            mark(min(max(x + d / 3 - 1, 0), F.nx - 1) >> 1, min(max(y + d % 3 - 1, 0), F.ny - 1) >> 1);
+                    }
+                }
+                __syncthreads();
+                // 32 words per warp and pass, their cells listed in ascending order
+                // (neighbouring entries share memory sectors)
+                for (int k0 = warp * 32; k0 < nw; k0 += BS) {
+                    const int k = k0 + lane;
+                    const unsigned m = k < nw ? bits[k] : 0u;
+                    const int c0 = (w0 + k) * 32;
+                    unsigned act = 0u;
+                    if (m) {
+                        atomicMin(&s_lo, c0 + __ffs(m) - 1);
+                        atomicMax(&s_hi, c0 + 31 - __clz(m));
+                        for (unsigned q = m; q; q &= q - 1)
+                            if (__ldg(L.invd + c0 + __ffs(q) - 1) > 0.f) act |= q & (0u - q);
+                    }
+                    int pos = __popc(act);
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int y = __shfl_up_sync(0xffffffffu, pos, o);
+                        if (lane >= o) pos += y;
+                    }
+                    const int total = __shfl_sync(0xffffffffu, pos, 31);
+                    int base = 0;
+                    if (lane == 31 && total) base = atomicAdd(&s_cnt, total);
+                    pos += used + __shfl_sync(0xffffffffu, base, 31) - __popc(act);
+                    for (; act; act &= act - 1, pos++)
+                        if (pos < kCycleList) list[pos] = c0 + __ffs(act) - 1;
+                }
+                __syncthreads();
+            }
+            all = used + s_cnt > kCycleList;
+            if (!all) {
+                cnt = s_cnt;
+                lo = s_lo;
+                hi = s_hi;
+            }
+        }
+        const int size = max(hi - lo + 1, 0);
+        __syncthreads();
+        if (tid == 0) {
+            cp.list[l] = all ? -1 : used;
+            cp.count[l] = cnt;
+            cp.lo[l] = lo;
+            cp.off[l] = l < mg.lred && next + size <= room ? next : -1;
+        }
+        if (l < mg.lred && next + size <= room) next += size;
+        if (!all) used += cnt;
+        __syncthreads();
+    }
+    for (int k = tid; k < next; k += BS) sm[k] = 0.f;
+    auto take = [&](int size) {
+        const int at = next + size <= room ? next : -1;
+        if (at >= 0) next += size;
+        return at;
+    };
+    // operator data, coarse levels first
+    const int nd = mg.lev[mg.nlev].nx * mg.lev[mg.nlev].ny;
+    const int dense = take(nd * nd);
+    if (dense >= 0)
+        for (int k = tid; k < nd * nd; k += BS) sm[dense + k] = __ldg(mg.dense + k);
+    if (tid == 0) cp.dense = dense;
+    for (int l = mg.nlev - 1; l >= 1; l--) {
+        const MgLevel &L = mg.lev[l], &C = mg.lev[l + 1];
+        const int na = __ldg(mg.nact + l + 1), nc = C.nx * C.ny, n1 = L.nx * L.ny;
+        const int dn = l >= mg.lred ? take(18 * na) : -1;
+        if (dn >= 0)
+            for (int q = tid; q < na; q += BS) {
+                const int I = __ldg(C.act + q);
+#pragma unroll
+                for (int k = 0; k < 16; k++) sm[dn + k * na + q] = ldc(C.rw, (size_t)k * nc + I);
+                sm[dn + 16 * na + q] = ldc(C.invd, I);
+                sm[dn + 17 * na + q] = __int_as_float((I / C.ny) << 16 | (I % C.ny));
+            }
+        const int cnt = cp.count[l];
+        const int up = cp.list[l] >= 0 ? take(11 * cnt) : -1;
+        if (up >= 0)
+            for (int q = tid; q < cnt; q += BS) {
+                const int I = list[cp.list[l] + q];
+#pragma unroll
+                for (int d = 0; d < 9; d++) sm[up + d * cnt + q] = ldc(L.st, (size_t)d * n1 + I);
+                sm[up + 9 * cnt + q] = ldc(L.invd, I);
+                sm[up + 10 * cnt + q] = __int_as_float((I / L.ny) << 16 | (I % L.ny));
+            }
+        if (tid == 0) {
+            cp.dn[l + 1] = dn;
+            cp.up[l] = up;
+        }
+    }
+}
+
+// Post-smoothing of cell (x, y) with the prolongation folded in: stencil st(d),
+// e and r of its level by cell index, corr = the parents' corrected values.
+template <class S, class E>
+__device__ __forceinline__ float smooth_cell(const Mg& mg, const MgLevel& L, int cny, const float* corr, int x, int y,
+                                             float iv, float ri, S&& st, E&& e) {
+    float w[9], ej[9];
+#pragma unroll
+    for (int d = 0; d < 9; d++) {
+        const int jx = min(max(x + d / 3 - 1, 0), L.nx - 1), jy = min(max(y + d % 3 - 1, 0), L.ny - 1);
+        w[d] = st(d);
+        ej[d] = fmaf(mg.scale, corr[(jx >> 1) * cny + (jy >> 1)], e(jx * L.ny + jy));
+    }
+    float acc = 0.f;
+#pragma unroll
+    for (int d = 0; d < 9; d++) {
+        const int jx = x + d / 3 - 1, jy = y + d % 3 - 1;
+        if (jx >= 0 && jy >= 0 && jx < L.nx && jy < L.ny) acc = fmaf(w[d], ej[d], acc);
+    }
+    return fmaf(mg.omega * iv, ri - acc, ej[4]);
+}
+
+// All of the block's cells of level l: t by cell index, e and r of the level by
+// their accessors.
+template <int NT, class E, class R>
+__device__ __forceinline__ void smooth_level(const Mg& mg, int l, const CyclePatch& cp, const float* sm,
+                                             const int* list, const float* corr, float* t, E&& e, R&& r) {
+    const MgLevel& L = mg.lev[l];
+    const int cny = mg.lev[l + 1].ny, cnt = cp.count[l], n = L.nx * L.ny;
+    if (cp.up[l] >= 0) {
+        const float* W = sm + cp.up[l];
+        for (int q = threadIdx.x; q < cnt; q += NT) {
+            const int xy = __float_as_int(W[10 * cnt + q]);
+            const int x = xy >> 16, y = xy & 0xffff, I = x * L.ny + y;
+            t[I] = smooth_cell(mg, L, cny, corr, x, y, W[9 * cnt + q], r(I), [&](int d) { return W[d * cnt + q]; }, e);
+        }
+    } else {
+        const int* li = cp.list[l] >= 0 ? list + cp.list[l] : L.act;
+        for (int q = threadIdx.x; q < cnt; q += NT) {
+            const int I = li[q];
+            const int x = I / L.ny, y = I - x * L.ny;
+            t[I] = smooth_cell(mg, L, cny, corr, x, y, ldc(L.invd, I), r(I),
+                               [&](int d) { return ldc(L.st, (size_t)d * n + I); }, e);
+        }
+    }
+}
+
+// The cycle, run by the first NT threads of every block of the group, after
+// level 1's residual (and, with lr > 1, its pre-smoothing) was written and a
+// barrier passed.  gcell / gsz: this thread's first entry of the grid-wide
+// cell lists and the group's stride.  Returns false if a barrier gave up.
+template <int NT>
+__device__ __forceinline__ bool mg_split_cycle(const Mg& mg, GridBar& gb, DevStats* ds, int gcell, int gsz,
+                                               float* __restrict__ sm, int floats, const CyclePatch& cp) {
+    const int tid = threadIdx.x, lr = mg.lred;
+    const int* list = reinterpret_cast<const int*>(sm + floats - kCycleList);
+    for (int l = 1; l < lr; l++) {
+        const MgLevel &F = mg.lev[l], &C = mg.lev[l + 1];
+        const int na = __ldg(mg.nact + l + 1);
+        for (int q = gcell; q < na; q += gsz) {
+            const int I = __ldg(C.act + q);
+            const int X = I / C.ny, Y = I - X * C.ny;
+            const float iv = __ldg(C.invd + I);
+            const float rr = restrict_cell(F, C, I, X, Y);
+            C.r[I] = rr;
+            if (l + 1 < lr) C.e[I] = mg.omega * iv * rr;
+        }
+        if (!grid_sync<NT>(gb, ds)) return false;
+    }
+    float* base = sm;  // level l's r, e, t
+    {
+        const MgLevel& L = mg.lev[lr];
+        const int na = __ldg(mg.nact + lr), n = L.nx * L.ny;
+        for (int q = tid; q < na; q += NT) {
+            const int I = __ldg(L.act + q);
+            const float iv = __ldg(L.invd + I), rr = __ldcg(L.r + I);
+            base[I] = rr;
+            base[n + I] = mg.omega * iv * rr;
+        }
+        group_bar<NT>();
+    }
+    for (int l = lr; l < mg.nlev; l++) {
+        const MgLevel &F = mg.lev[l], &C = mg.lev[l + 1];
+        const int nc = C.nx * C.ny, na = __ldg(mg.nact + l + 1);
+        const float* fr = base;
+        base += 3 * F.nx * F.ny;
+        auto cell = [&](int X, int Y, float iv, auto&& weight) {
+            int xs[4], ys[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                xs[k] = min(max(2 * X - 1 + k, 0), F.nx - 1) * F.ny;
+                ys[k] = min(max(2 * Y - 1 + k, 0), F.ny - 1);
+            }
+            float w[16];
+#pragma unroll
+            for (int k = 0; k < 16; k++) w[k] = weight(k);
+            float acc = 0.f;
+#pragma unroll
+            for (int k = 0; k < 16; k++) acc = fmaf(w[k], fr[xs[k >> 2] + ys[k & 3]], acc);
+            base[X * C.ny + Y] = acc;
+            base[nc + X * C.ny + Y] = mg.omega * iv * acc;  // (the coarsest level's is replaced below)
+        };
+        if (cp.dn[l + 1] >= 0) {
+            const float* W = sm + cp.dn[l + 1];
+            for (int q = tid; q < na; q += NT) {
+                const int xy = __float_as_int(W[17 * na + q]);
+                cell(xy >> 16, xy & 0xffff, W[16 * na + q], [&](int k) { return W[k * na + q]; });
+            }
+        } else {
+            for (int q = tid; q < na; q += NT) {
+                const int I = __ldg(C.act + q);
+                cell(I / C.ny, I % C.ny, ldc(C.invd, I), [&](int k) { return ldc(C.rw, (size_t)k * nc + I); });
+            }
+        }
+        group_bar<NT>();
+    }
+    const float* corr;  // the corrected values of level l + 1, by cell index
+    {
+        // coarsest level: its dense inverse, one warp per row (a cell without
+        // unknowns has an identity row and residual 0)
+        const MgLevel& L = mg.lev[mg.nlev];
+        const int n = L.nx * L.ny, lane = tid & 31;
+        const float* D = cp.dense >= 0 ? sm + cp.dense : mg.dense;
+        for (int i = tid >> 5; i < n; i += NT / 32) {
+            float a = 0.f;
+            for (int j = lane; j < n; j += 32) a = fmaf(D[i * n + j], base[j], a);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+            if (lane == 0) base[n + i] = a;
+        }
+        group_bar<NT>();
+        corr = base + n;
+    }
+    for (int l = mg.nlev - 1; l >= lr; l--) {
+        const int n = mg.lev[l].nx * mg.lev[l].ny;
+        base -= 3 * n;
+        smooth_level<NT>(mg, l, cp, sm, list, corr, base + 2 * n, [&](int j) { return base[n + j]; },
+                         [&](int j) { return base[j]; });
+        group_bar<NT>();
+        corr = base + 2 * n;
+    }
+    for (int l = lr - 1; l >= 1; l--) {
+        const MgLevel& L = mg.lev[l];
+        float* t = cp.off[l] >= 0 ? sm + cp.off[l] - cp.lo[l] : L.t;  // by cell index
+        smooth_level<NT>(mg, l, cp, sm, list, corr, t, [&](int j) { return ldv(L.e, j); },
+                         [&](int j) { return ldv(L.r, j); });
+        group_bar<NT>();
+        corr = t;
+    }
+    return true;
+}
+
+// Where level 1's correction lies after the split cycle, by cell index.
+__device__ __forceinline__ const float* split_correction(const Mg& mg, const float* sm, const CyclePatch& cp) {
+    if (mg.lred > 1) return cp.off[1] >= 0 ? sm + cp.off[1] - cp.lo[1] : mg.lev[1].t;
+    return sm + (mg.nlev > 1 ? 2 : 1) * mg.lev[1].nx * mg.lev[1].ny;
 }
 
 // The cell levels of the V-cycle after level 1's residual and pre-smoothing
@@ -1206,17 +1628,14 @@ __global__ void __launch_bounds__(kMixedBlock, 1)
 // and, since A P1 = B (the rows' 3x3-cell sums, k_mg_rowcell),
 //     w = A u = omega (A y) + scale B e1,
 // where A y needs only r, not the cycle.  So after the vector update (which
-// writes y) and one grid barrier, each block splits: its first kCycleThreads
-// threads run the cycle (level-1 sums, the grid-wide levels with grid
-// barriers of that group, the small levels in block 0), the other warps
-// apply the FP32 operator to y for the block's own rows (z = A y).  The
+// writes y) and one barrier, each block splits: its first NV threads run the
+// split cycle (above), the other warps apply the FP32 operator to y for the
+// block's own rows (z = A y).  The
 // block joins, and one pass over its rows forms u, w and the three dot
 // products.  The operator pass (most of an iteration's HBM traffic) is thus
 // off the cycle's chain of dependent phases, and u and w never leave the
 // block (no operator pass reads them).  Same Chronopoulos-Gear recurrences,
 // refinement and stopping rules as solve_mixed.
-//
-// Rows: 32-row slices dealt to blocks 1..G-1 (block 0 runs the small levels).
 constexpr int kCycleThreads = 512;
 // The vector update of the overlapped solve gives each warp one contiguous
 // range of rows that starts and ends at level-1 cell boundaries, walked in
@@ -1236,10 +1655,10 @@ __device__ __forceinline__ int cell_start_at_or_after(const int32_t* __restrict_
     return n;
 }
 
-template <int BS, int NV>
+template <int BS, int NV, bool CL>
 __device__ __forceinline__ void solve_mixed_overlap(const Ppe& A, const MatFree& mf, const Mg& mg,
                                                     const Krylov& kv, const SolveArgs& a, DevStats* ds,
-                                                    GridBar& gb) {
+                                                    GridBar& gb, float* __restrict__ sm, int floats) {
     if (*(volatile int32_t*)&ds->status & ST_ASYMMETRIC) {  // the reference exits here
         if (gb.rank == 0 && threadIdx.x == 0) {
             ds->cg_iterations = 0;
@@ -1255,13 +1674,10 @@ __device__ __forceinline__ void solve_mixed_overlap(const Ppe& A, const MatFree&
     const int gtid = b * BS + tid, gsz = G * BS;
     const int gwarp = gtid >> 5, nwarps = gsz >> 5;
     const int n = a.n, nsl = a.nslices;
-    // The rows (32-row slices) of the operator pass, of the pass that forms
-    // u and w and of the vector update belong to blocks 1..G-1: slices
-    // rb, rb + RB, rb + 2 RB, ...  Block 0 runs the cycle's small levels and
-    // does not also stream rows beside them.
-    const int RB = G > 1 ? G - 1 : 1;
-    const int rb = G > 1 ? b - 1 : 0;
-    const bool has_rows = G == 1 || b > 0;
+    // This block's rows: one run of 32-row slices for the operator pass and the
+    // pass that forms u and w (their corrections then come from one run of
+    // cells), and about the same rows, cut at cell boundaries, for the update.
+    const int sl0 = (int)((int64_t)nsl * b / G), sl1 = (int)((int64_t)nsl * (b + 1) / G);
     // per-slot FP32 work vectors of this arrangement (the additive cycle uses
     // neither the level-0 correction nor the level-0 residual arrays)
     float* __restrict__ y = mg.e0;    // D^-1 r
@@ -1271,11 +1687,10 @@ __device__ __forceinline__ void solve_mixed_overlap(const Ppe& A, const MatFree&
     // level 1's sums fused into the vector update (cell indices fit 24 bits)
     const bool fuse1 = n1 < (1 << 24);
     __shared__ int s_cycle_ok;
+    __shared__ CyclePatch s_cp;
     __shared__ float s_ring[kW][kRing];
-    // the e/t role swaps of the grid-wide levels (lev_view): the cycle group
-    // makes them, the other warps follow with the same mask after each cycle
-    uint32_t swp = 0;
-    const uint32_t cycle_swaps = ((1u << (mg.ngrid + 1)) - 1u) & ~1u;  // levels 1..ngrid
+    plan_patches<BS>(A, mg, mf, sl0, sl1, n, sm, floats, s_cp);
+    __syncthreads();
 
     double acc[1] = {0.0}, tot[1];
     for (int sl = gwarp; sl < nsl; sl += nwarps) {
@@ -1296,12 +1711,12 @@ __device__ __forceinline__ void solve_mixed_overlap(const Ppe& A, const MatFree&
         double bb = A.src[i];
         acc[0] = fma(bb, bb, acc[0]);
     }
-    if (!reduce_sync<1, BS>(gb, acc, tot, ds)) return;
+    if (!solve_reduce<CL, BS>(gb, acc, tot, ds)) return;
     // this warp's rows of the vector update: [rlo, rhi), from the first cell
     // start at or after an even split point to the next warp's
     int rlo = 0, rhi = 0;
-    if (has_rows) {
-        const int nw = RB * kW, wi = rb * kW + warp;
+    {
+        const int nw = G * kW, wi = b * kW + warp;
         rlo = wi == 0 ? 0 : cell_start_at_or_after(mf.skey, (int)((int64_t)n * wi / nw), n);
         rhi = wi + 1 == nw ? n : cell_start_at_or_after(mf.skey, (int)((int64_t)n * (wi + 1) / nw), n);
     }
@@ -1323,7 +1738,7 @@ __device__ __forceinline__ void solve_mixed_overlap(const Ppe& A, const MatFree&
             kv.r[i] = r;
             a0[0] = fma(r, r, a0[0]);
         }
-        if (!reduce_sync<1, BS>(gb, a0, t0, ds)) return;
+        if (!solve_reduce<CL, BS>(gb, a0, t0, ds)) return;
         rn2 = t0[0];
         if (a.warm && refine == 0 && rn2 > rhs2) {
             // a guess worse than zero (a state replaced by mps_upload): start from zero
@@ -1332,7 +1747,7 @@ __device__ __forceinline__ void solve_mixed_overlap(const Ppe& A, const MatFree&
                 kv.r[i] = A.src[i];
             }
             rn2 = rhs2;
-            if (!grid_sync(gb, ds)) return;
+            if (!solve_sync<CL>(gb, ds)) return;
         }
         if (rn2 < thr || refine >= a.max_refine || inner_total >= a.max_iter) break;
         refine++;
@@ -1346,7 +1761,7 @@ __device__ __forceinline__ void solve_mixed_overlap(const Ppe& A, const MatFree&
             kv.s32[i] = 0.f;
             y[i] = kv.inv_diag32[i] * r;
         }
-        if (!grid_sync(gb, ds)) return;
+        if (!solve_sync<CL>(gb, ds)) return;
         float alpha = 0.f, beta = 0.f, gamma_old = 1.f;
         int64_t k = 0;
         for (;;) {
@@ -1356,21 +1771,18 @@ __device__ __forceinline__ void solve_mixed_overlap(const Ppe& A, const MatFree&
             // writes them for the next iteration
             if (k == 0 || !fuse1) {
                 mg_level1_plain(mg, mf, kv.r32, ((warp * G + b) << 5) + lane, gsz,
-                                level1_presmooth(mg, swp));
-                if (!grid_sync(gb, ds)) return;
+                                mg.lev[1].e);
+                if (!solve_sync<CL>(gb, ds)) return;
             }
             // ---- split: the cycle's cell levels on r, the operator on y
             if (warp < kVW) {
-                const int gcell = ((warp * G + b) << 5) + lane;
-                const bool ok = mg_cell_levels<NV>(mg, swp, gb, ds, gcell, G * NV, false);
+                const bool ok = mg_split_cycle<NV>(mg, gb, ds, ((warp * G + b) << 5) + lane, G * NV, sm, floats, s_cp);
                 if (tid == 0) s_cycle_ok = ok;
             } else {
-                for (int q = warp - kVW; has_rows; q += 2 * kZW) {
-                    const int sl1 = rb + RB * q;
-                    if (sl1 >= nsl) break;
-                    const int sl2 = rb + RB * (q + kZW);
-                    const int i = sl1 * 32 + lane;
-                    int i2 = sl2 < nsl ? sl2 * 32 + lane : -1;
+                for (int sla = sl0 + warp - kVW; sla < sl1; sla += 2 * kZW) {
+                    const int slb = sla + kZW;
+                    const int i = sla * 32 + lane;
+                    int i2 = slb < sl1 ? slb * 32 + lane : -1;
                     if (i2 >= n) i2 = -1;
                     if (i >= n) continue;  // the partial last slice (then i2 < 0 too)
                     const int j2 = i2 >= 0 ? i2 : i;
@@ -1382,18 +1794,15 @@ __device__ __forceinline__ void solve_mixed_overlap(const Ppe& A, const MatFree&
                     z[i] = dg0 > 0.f ? fmaf(c0, y0, o) : 0.f;
                     if (i2 >= 0) z[i2] = dg1 > 0.f ? fmaf(c1, y1, o2) : 0.f;
                 }
-                swp ^= cycle_swaps;
             }
             __syncthreads();
             if (!s_cycle_ok) return;
-            const float* __restrict__ e1 = level1_correction(mg, swp);
+            const float* e1 = split_correction(mg, sm, s_cp);
             // ---- u = omega y + scale e1[cell], w = omega z + scale B e1, dot products
             F2 g = {0.f, 0.f}, dl = {0.f, 0.f}, rr = {0.f, 0.f};
-            for (int q = warp; has_rows; q += 2 * kW) {
-                const int sla = rb + RB * q;
-                if (sla >= nsl) break;
-                const int slb = rb + RB * (q + kW);
-                int ii[2] = {sla * 32 + lane, slb < nsl ? slb * 32 + lane : n};
+            for (int sla = sl0 + warp; sla < sl1; sla += 2 * kW) {
+                const int slb = sla + kW;
+                int ii[2] = {sla * 32 + lane, slb < sl1 ? slb * 32 + lane : n};
                 float dg[2], cs[2], ri[2], yi[2], zi[2];
                 int key[2];
 #pragma unroll
@@ -1418,7 +1827,7 @@ __device__ __forceinline__ void solve_mixed_overlap(const Ppe& A, const MatFree&
 #pragma unroll
                         for (int d = 0; d < 9; d++) {
                             bt[d] = d == 4 ? 0.f : __ldg(mg.rowcell + (size_t)d * np + i);
-                            en[d] = __ldcg(e1 + key[h] + (d / 3 - 1) * NY + (d % 3 - 1));
+                            en[d] = e1[key[h] + (d / 3 - 1) * NY + (d % 3 - 1)];
                         }
                         float corr = 0.f;
 #pragma unroll
@@ -1437,7 +1846,7 @@ __device__ __forceinline__ void solve_mixed_overlap(const Ppe& A, const MatFree&
             }
             const F2 v3[3] = {g, dl, rr};
             float t3[3];
-            if (!reduce_sync_f2<3, BS>(gb, v3, t3, ds)) return;
+            if (!solve_reduce_f2<CL, BS>(gb, v3, t3, ds)) return;
             if (t3[2] < ithr || inner_total + k >= a.max_iter) break;
             const float gamma = t3[0], delta = t3[1];
             if (k == 0) {
@@ -1457,7 +1866,7 @@ __device__ __forceinline__ void solve_mixed_overlap(const Ppe& A, const MatFree&
             // and pre-smoothing (the same values as the separate level-1 pass)
             {
                 float* __restrict__ r1 = mg.lev[1].r;
-                float* __restrict__ e1n = level1_presmooth(mg, swp);
+                float* __restrict__ e1n = mg.lev[1].e;
                 float* ring = s_ring[warp];
                 for (int base = rlo; base < rhi; base += 64) {
                     float u[2], p[2], sv[2], w[2], x[2], r[2], id[2];
@@ -1512,13 +1921,13 @@ __device__ __forceinline__ void solve_mixed_overlap(const Ppe& A, const MatFree&
                 }
             }
             k++;
-            if (!grid_sync(gb, ds)) return;
+            if (!solve_sync<CL>(gb, ds)) return;
         }
         inner_total += k;
         // x += d (FP64)
         const double back = sqrt(rn2);
         for (int i = gtid; i < n; i += gsz) kv.x[i] = fma((double)kv.x32[i], back, kv.x[i]);
-        if (!grid_sync(gb, ds)) return;
+        if (!solve_sync<CL>(gb, ds)) return;
     }
     if (gb.rank == 0 && threadIdx.x == 0) {
         ds->cg_iterations = inner_total;
@@ -1528,11 +1937,24 @@ __device__ __forceinline__ void solve_mixed_overlap(const Ppe& A, const MatFree&
     }
 }
 
+template <int NV>
 __global__ void __launch_bounds__(kMixedBlock, 1)
     k_cg_mixed_ov(__grid_constant__ const Ppe A, __grid_constant__ const MatFree mf, __grid_constant__ const Mg mg,
-                  __grid_constant__ const Krylov kv, __grid_constant__ const SolveArgs a, DevStats* ds) {
+                  __grid_constant__ const Krylov kv, __grid_constant__ const SolveArgs a, DevStats* ds, int floats) {
+    extern __shared__ float s_levels[];
     GridBar gb = whole_grid(kv);
-    solve_mixed_overlap<kMixedBlock, kCycleThreads>(A, mf, mg, kv, a, ds, gb);
+    solve_mixed_overlap<kMixedBlock, NV, false>(A, mf, mg, kv, a, ds, gb, s_levels, floats);
+}
+
+// The same solve by one cluster, for small scenes whose level 1 fits a
+// block's shared memory: two cluster barriers per inner iteration.
+__global__ void __launch_bounds__(kMixedBlock, 1)
+    k_cg_mixed_cl(__grid_constant__ const Ppe A, __grid_constant__ const MatFree mf, __grid_constant__ const Mg mg,
+                  __grid_constant__ const Krylov kv, __grid_constant__ const SolveArgs a, DevStats* ds, int floats) {
+    extern __shared__ float s_levels[];
+    GridBar gb = whole_grid(kv);
+    solve_mixed_overlap<kMixedBlock, kCycleThreads, true>(A, mf, mg, kv, a, ds, gb, s_levels, floats);
+    cluster_barrier();  // no block leaves while another may still store into its slots
 }
 
 // Many scenes in one persistent launch: block b belongs to group bmap[b].x
@@ -1657,12 +2079,80 @@ SolveArgs make_args(const Consts& c, double tol, int64_t max_iter) {
 
 }  // namespace
 
+namespace {
+// Largest scene of the one-cluster solve.  Its 16 SMs take, per inner
+// iteration, 18 us at 2,000 rows, 22 at 11,000 and 31 at 21,000 against 24, 28
+// and 31 for the grid of 152 blocks with its barriers: the line lies where the
+// operator pass on 16 SMs has eaten up what the cluster barriers save.
+constexpr int kClusterRows = 24000;
+// Dynamic shared memory of the overlapped solve's blocks (the split cycle's
+// levels, patches and operator data), and the part of it that the levels may
+// take: 136 KB hold all levels of a tank of 11,000 cells.
+constexpr int kSplitSmem = 192 * 1024;
+constexpr int kSplitLevels = 136 * 1024;
+// Above kStreamRows rows the iteration is bound by the operator pass rather
+// than by the cycle's latency, and its loads in flight need the L1 that shared
+// memory takes away: less shared memory (one more grid-wide level) and fewer
+// cycle warps.  1M rows: 171 us per inner iteration with 192 KB and 512
+// threads, 123 with 104 KB, 108 with 256 threads as well; at 100,000 rows
+// 256 threads cost 37 -> 40 us.
+constexpr int kStreamRows = 300000;
+constexpr int kStreamLevels = 40 * 1024;
+constexpr int kStreamCycle = 256;
+constexpr int kStreamSmem = 104 * 1024;
+static_assert(kSplitLevels + 4 * kCycleList < kSplitSmem && kStreamLevels + 4 * kCycleList < kStreamSmem,
+              "the levels and the lists fit; patches and operator data take what is left");
+
+// Cells of levels l .. nlev.
+int level_cells(const Mg& mg, int l) {
+    int64_t n = 0;
+    for (; l <= mg.nlev; l++) n += (int64_t)mg.lev[l].nx * mg.lev[l].ny;
+    return (int)std::min<int64_t>(n, 1 << 26);
+}
+int first_shared_level(const Mg& mg, int n) {
+    int l = 1;
+    const int most = n > kStreamRows ? kStreamLevels : kSplitLevels;
+    while (l < mg.nlev && level_cells(mg, l) * 12 > most) l++;
+    return l;
+}
+
+void cluster_attribute(cudaLaunchAttribute& at, int blocks) {
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = blocks;
+    at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = 1;
+}
+
+// Blocks of the cluster the device can run (0: none of the sizes).
+int cluster_blocks() {
+    const void* fn = (const void*)k_cg_mixed_cl;
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem);
+    cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    for (int blocks = kClusterMax; blocks >= 8; blocks /= 2) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(blocks);
+        cfg.blockDim = dim3(kMixedBlock);
+        cfg.dynamicSmemBytes = kSplitSmem;
+        cudaLaunchAttribute at[1];
+        cluster_attribute(at[0], blocks);
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int fit = 0;
+        if (cudaOccupancyMaxActiveClusters(&fit, fn, &cfg) == cudaSuccess && fit > 0) return blocks;
+        cudaGetLastError();
+    }
+    return 0;
+}
+}  // namespace
+
 void solver_setup(Krylov& k, int32_t /*n_pad*/, int device) {
     int g1 = cg64_grid(device);
     int g2 = coop_grid((const void*)k_cg_mixed, device, kMixedBlock, 0, 1);
-    int g3 = coop_grid((const void*)k_cg_mixed_ov, device, kMixedBlock, 0, 1);
+    int g3 = std::min(coop_grid((const void*)k_cg_mixed_ov<kCycleThreads>, device, kMixedBlock, kSplitSmem, 1),
+                      coop_grid((const void*)k_cg_mixed_ov<kStreamCycle>, device, kMixedBlock, kStreamSmem, 1));
     k.grid = std::min({g1, g2, g3});
     k.block = kBlock;
+    k.cluster = cluster_blocks();
 }
 
 void launch_mixed_setup(const Consts& c, const SortScratch& sc, const Ppe& A, MatFree& mf,
@@ -1836,8 +2326,35 @@ void launch_solve_mixed(const Consts& c, const Ppe& A, const MatFree& mf, const 
     void* args[] = {&AA, &mm, &gg, &kk, &a, &ds};
     cudaMemsetAsync(k.barrier, 0, sizeof(unsigned int), st);
     const bool ov = mg.enabled && mg.overlap;
-    const void* fn = ov ? (const void*)k_cg_mixed_ov : (const void*)k_cg_mixed;
-    cudaLaunchCooperativeKernel(fn, dim3(k.grid), dim3(kMixedBlock), args, 0, st);
+    int floats = kSplitSmem / 4;
+    if (ov && k.cluster > 0 && c.n <= kClusterRows && level_cells(mg, 1) * 12 <= kSplitSmem - 4 * kCycleList) {
+        gg.lred = 1;  // every level in every block: no patches, no barrier of the cycle's own
+        void* cargs[] = {&AA, &mm, &gg, &kk, &a, &ds, &floats};
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(k.cluster);
+        cfg.blockDim = dim3(kMixedBlock);
+        cfg.dynamicSmemBytes = kSplitSmem;
+        cfg.stream = st;
+        cudaLaunchAttribute at[1];
+        cluster_attribute(at[0], k.cluster);
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        cudaLaunchKernelExC(&cfg, (const void*)k_cg_mixed_cl, cargs);
+        ++g_launches;
+        return;
+    }
+    if (ov) {
+        gg.lred = first_shared_level(mg, c.n);
+        const bool stream = c.n > kStreamRows;
+        const int smem = stream ? kStreamSmem : kSplitSmem;
+        floats = smem / 4;
+        void* oargs[] = {&AA, &mm, &gg, &kk, &a, &ds, &floats};
+        const void* fn = stream ? (const void*)k_cg_mixed_ov<kStreamCycle> : (const void*)k_cg_mixed_ov<kCycleThreads>;
+        cudaLaunchCooperativeKernel(fn, dim3(k.grid), dim3(kMixedBlock), oargs, smem, st);
+        ++g_launches;
+        return;
+    }
+    cudaLaunchCooperativeKernel((const void*)k_cg_mixed, dim3(k.grid), dim3(kMixedBlock), args, 0, st);
     ++g_launches;
 }
 
