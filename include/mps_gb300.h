@@ -120,8 +120,8 @@ int mps_set_solver(mps_engine* e, int32_t precision, double tol, int64_t max_ite
  * A u assembled from it and the rows' 3x3-cell sums of A); mode 4: mode 1's
  * preconditioner with the operator applied to u after the cycle (the same
  * iteration in the order of the textbook loop; kept for comparison, and the
- * form every batch scene uses); mode 3: the same with the smoothed
- * transfer P = P1 - omega D^-1 A P1, applied through the rows' 3x3-cell sums
+ * form that batch launches of 256 and 512 threads use); mode 3: the same with
+ * the smoothed transfer P = P1 - omega D^-1 A P1, applied through the rows' 3x3-cell sums
  * of A (fewer iterations, no extra operator pass); mode 2:
  * the multiplicative V(1,1) cycle from the particle level (three operator
  * passes per iteration).  omega = Jacobi weight in (0,1], scale =

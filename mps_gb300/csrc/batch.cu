@@ -15,7 +15,9 @@
 // group-size model blocks_s ~ rows_s^alpha) is chosen by a small autotuner
 // on the first step: every candidate solves that step's systems (the solve
 // is idempotent: it starts from x = 0 and reads only the assembled system),
-// the fastest is kept, and the step then finishes with it.
+// the fastest is kept, and the step then finishes with it.  1024-thread
+// candidates run the overlapped arrangement of the multigrid solve within
+// each group, the others its plain form.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -209,7 +211,6 @@ int mps_batch_create(int32_t n_scenes, const mps_params* params, const int32_t* 
         mps_engine* e = nullptr;
         int rc = mps_create(&params[s], counts[s], pos + 3 * off, vel + 3 * off, type + off, &e);
         if (rc) return bail(rc);
-        e->cycle_overlap = 0;  // the batched solve kernel runs mode 1 in its plain form
         b->eng.push_back(e);
         if ((rc = mps_set_solver(e, MPS_PRECISION_MIXED, b->tol, 0))) return bail(rc);
         off += counts[s];

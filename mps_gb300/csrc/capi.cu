@@ -205,7 +205,7 @@ Mg active_mg(const mps_engine* e) {
     g.enabled = e->mg.enabled && e->mg_requested != 0;
     g.additive = e->mg_requested == 1 || e->mg_requested == 3 || e->mg_requested == 4;
     g.smooth = e->mg_requested == 3;
-    g.overlap = e->mg_requested == 1 && e->cycle_overlap;
+    g.overlap = e->mg_requested == 1;
     return g;
 }
 
