@@ -428,6 +428,37 @@ __device__ __forceinline__ float spmv32_sell_row(const Ppe& A, int K, int row,
     return s;
 }
 
+// Groups [g0, g1) of four entries of such a row, two groups' loads and gathers
+// at a time.
+__device__ __forceinline__ float sell_part_sum(const Ppe& A, int K, int row, int w, int g0, int g1,
+                                               const float* __restrict__ u, float ui) {
+    const int32_t* cp = A.col + (size_t)(row >> 5) * K * 32 + (row & 31);
+    const float4* vq = reinterpret_cast<const float4*>(A.val32) + (qsell_index(row, 0, K) >> 2);
+    float s0 = 0.f, s1 = 0.f;
+    for (int g = g0; g < g1; g += 2) {
+        int c[8];
+        float x[8];
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 a = __ldg(vq + g * 32), b = g + 1 < g1 ? __ldg(vq + (g + 1) * 32) : zero;
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+            const int m = 4 * g + t;  // (the columns past the slice's width are not set)
+            c[t] = m < w && m < 4 * g1 ? __ldg(cp + m * 32) : row;
+        }
+#pragma unroll
+        for (int t = 0; t < 8; t++) x[t] = __ldcg(u + c[t]) - ui;
+        s0 = fmaf(a.x, x[0], s0);
+        s1 = fmaf(a.y, x[1], s1);
+        s0 = fmaf(a.z, x[2], s0);
+        s1 = fmaf(a.w, x[3], s1);
+        s0 = fmaf(b.x, x[4], s0);
+        s1 = fmaf(b.y, x[5], s1);
+        s0 = fmaf(b.z, x[6], s0);
+        s1 = fmaf(b.w, x[7], s1);
+    }
+    return s0 + s1;
+}
+
 // Compact FP32 row: per group of four entries one 16-byte value word and one
 // 4-byte word of index bytes (2 bits: which of the row's three candidate
 // ranges, 6 bits: offset in it); the range starts are stored per row.  The
@@ -1225,13 +1256,14 @@ __device__ __forceinline__ bool mg_vcycle(const Mg& mg, uint32_t& swp, const Ppe
                                           int K, const float* __restrict__ r, float* __restrict__ u,
                                           const float* __restrict__ invd0, int n, GridBar& gb,
                                           DevStats* ds) {
-    const int gtid = gb.rank * BS + threadIdx.x;
     const int gsz = gb.size * BS;
-    // Cells of the grid levels are dealt to blocks in interleaved 32-cell
-    // chunks (coalesced within a warp): the cells with unknowns cover only
-    // the fluid's part of the tank, and a contiguous split would hand them all
-    // to a few blocks while the rest wait at the next barrier.
-    const int gcell = ((threadIdx.x >> 5) * gb.size + gb.rank) * 32 + (threadIdx.x & 31);
+    // Rows, and the cells of the grid levels, are dealt to blocks in
+    // interleaved 32-entry chunks (coalesced within a warp): a contiguous split
+    // would hand a small scene's rows, and the cells with unknowns, which cover
+    // only the fluid's part of the tank, to a few blocks while the rest wait at
+    // the next barrier.
+    const int gtid = ((threadIdx.x >> 5) * gb.size + gb.rank) * 32 + (threadIdx.x & 31);
+    const int gcell = gtid;
     // level 0 residual of the Inner particles (coalesced, one row per thread);
     // the additive form restricts r itself
     const float* src0 = mg.additive ? r : mg.res0;
@@ -1439,7 +1471,8 @@ __device__ __forceinline__ void solve_mixed(const Ppe& A, const MatFree& mf, con
         }
         return;
     }
-    const int gtid = gb.rank * BS + threadIdx.x;
+    // 32-row chunks dealt to the blocks in turn (see mg_vcycle)
+    const int gtid = ((threadIdx.x >> 5) * gb.size + gb.rank) * 32 + (threadIdx.x & 31);
     const int gsz = gb.size * BS;
     const int lane = threadIdx.x & 31;
     const int gwarp = gtid >> 5;
@@ -1515,7 +1548,7 @@ __device__ __forceinline__ void solve_mixed(const Ppe& A, const MatFree& mf, con
             // rows i and i + gsz of this thread together (their operator
             // loads interleaved); rows that are not unknowns (diagonal 0:
             // Surface, Ignored, ghosts) get w = +0
-            for (int i = gtid; i < a.n; i += 2 * gsz) {
+            for (int i = mf.enabled ? gtid : a.n; i < a.n; i += 2 * gsz) {
                 const int i2 = i + gsz < a.n ? i + gsz : -1;
                 // the rows' own words first: in flight with the operator's
                 float ui[2], dg[2], rv[2];
@@ -1537,6 +1570,46 @@ __device__ __forceinline__ void solve_mixed(const Ppe& A, const MatFree& mf, con
                     acc_prod(g, rv[h], ui[h]);
                     acc_prod(dl, w, ui[h]);
                     acc_prod(rr, rv[h], rv[h]);
+                }
+            }
+            if (!mf.enabled) {
+                // rows without the compact form (3-D scenes: ~100 entries a
+                // row).  A small scene leaves most warps without a row, and a
+                // row by one thread is a chain of dependent gathers: `parts`
+                // warps share a slice, each with a run of its groups of four
+                // entries, and the first adds their sums in order.
+                constexpr int kW = BS / 32;
+                const int warp = threadIdx.x >> 5;
+                int parts = 8;
+                while (parts > 1 && (int64_t)parts * a.nslices > (int64_t)gb.size * kW) parts >>= 1;
+                const int per = kW / parts, part = warp & (parts - 1);
+                const int mine = (a.nslices - gb.rank + gb.size - 1) / gb.size;  // the group's slices of this block
+                __shared__ float s_part[kW][32];
+                for (int q0 = 0; q0 < mine; q0 += per) {
+                    const int q = q0 + warp / parts;
+                    const int i = (q * gb.size + gb.rank) * 32 + lane;
+                    const bool row = q < mine && i < a.n;
+                    float ui = 0.f, o = 0.f;
+                    if (row) {
+                        ui = __ldcg(kv.u32 + i);
+                        const int w = __ldg(A.slice_w + (i >> 5)), groups = (w + 3) >> 2;
+                        o = sell_part_sum(A, a.K, i, w, groups * part / parts, groups * (part + 1) / parts, kv.u32, ui);
+                    }
+                    if (parts > 1) {
+                        s_part[warp][lane] = o;
+                        __syncthreads();
+                        if (part == 0)
+                            for (int t = 1; t < parts; t++) o += s_part[warp + t][lane];
+                    }
+                    if (row && part == 0) {
+                        const float dg = A.diag32[i], rv = kv.r32[i];
+                        const float w = dg > 0.f ? fmaf(A.rsum32[i], ui, o) : 0.f;
+                        kv.w32[i] = w;
+                        acc_prod(g, rv, ui);
+                        acc_prod(dl, w, ui);
+                        acc_prod(rr, rv, rv);
+                    }
+                    if (parts > 1) __syncthreads();
                 }
             }
             const F2 v3[3] = {g, dl, rr};

@@ -30,8 +30,9 @@ __device__ __forceinline__ bool outside_domain(const Consts& c, double x, double
 // pre-filter at `bound`: pass 1 collects them in a local list, pass 2 calls
 // f(j), where f runs the exact FP64 test and the work.  Splitting the sweep
 // keeps the FP64 work on compact lists, with nearly all lanes of a warp busy.
-// More survivors than the list holds: f(j) for every candidate (f's exact
-// test then selects the same neighbours in the same order).
+// A full list (3-D particles have ~120 neighbours) is worked off and filled
+// again, which keeps the order; running f on every candidate instead took
+// 0.75 ms on a 9,000-particle 3-D tank.
 constexpr int kNear = 64;
 template <bool PLANAR, class F>
 __device__ __forceinline__ void for_each_near(const Consts& c, const StateBuf& s,
@@ -43,16 +44,13 @@ __device__ __forceinline__ void for_each_near(const Consts& c, const StateBuf& s
     int ns = 0;
     for_each_candidate<PLANAR>(c, cs, key, [&](int j) {
         if (j == k || far32<PLANAR>(s, j, fx, fy, fz, bound)) return;
-        if (ns < kNear) cand[ns] = j;
-        ns++;
+        if (ns == kNear) {
+            for (int q = 0; q < kNear; q++) f(cand[q]);
+            ns = 0;
+        }
+        cand[ns++] = j;
     });
-    if (ns <= kNear) {
-        for (int q = 0; q < ns; q++) f(cand[q]);
-    } else {
-        for_each_candidate<PLANAR>(c, cs, key, [&](int j) {
-            if (j != k) f(j);
-        });
-    }
+    for (int q = 0; q < ns; q++) f(cand[q]);
 }
 
 // Number density at re_p over a particle's current neighbours (d < re_max),
