@@ -47,7 +47,6 @@ namespace mpsg {
 namespace {
 
 constexpr int kT = 256;
-inline int nblk(int n) { return (n + kT - 1) / kT; }
 
 struct Arr3 {
     double* p[3];
@@ -617,27 +616,27 @@ void tape_phase(mps_engine* e, TapePhase ph) {
     StateBuf& s = e->S();
     switch (ph) {
         case TAPE_START:
-            k_tape_state<<<nblk(n), kT, 0, st>>>(n, s.id, s, c.planar, c.z0, arr6(t.st0), t.type0);
+            k_tape_state<<<block_count(n), block_threads(n), 0, st>>>(n, s.id, s, c.planar, c.z0, arr6(t.st0), t.type0);
             break;
         case TAPE_LIST0:
             launch_build_list(c, s, e->sc, e->nb, e->ds, st);
-            k_tape_list<<<nblk(n), kT, 0, st>>>(n, e->nb.n_pad, s.id, e->nb.cnt, e->nb.slot, t.l0cnt,
+            k_tape_list<<<block_count(n), block_threads(n), 0, st>>>(n, e->nb.n_pad, s.id, e->nb.cnt, e->nb.slot, t.l0cnt,
                                                  t.l0id);
             break;
         case TAPE_EXPLICIT:
-            k_tape_state<<<nblk(n), kT, 0, st>>>(n, s.id, s, c.planar, c.z0, arr6(t.st1), t.type1);
+            k_tape_state<<<block_count(n), block_threads(n), 0, st>>>(n, s.id, s, c.planar, c.z0, arr6(t.st1), t.type1);
             break;
         case TAPE_COLLISION:
-            k_tape_state<<<nblk(n), kT, 0, st>>>(n, s.id, s, c.planar, c.z0, arr6(t.st2), nullptr);
+            k_tape_state<<<block_count(n), block_threads(n), 0, st>>>(n, s.id, s, c.planar, c.z0, arr6(t.st2), nullptr);
             k_tape_pairs<<<64, kT, 0, st>>>(e->pairs, e->cand_base + n, e->pair_cap, t.pairs, t.npairs,
                                             t.pair_cap, e->ds);
             break;
         case TAPE_LIST2:
-            k_tape_list<<<nblk(n), kT, 0, st>>>(n, e->nb.n_pad, s.id, e->nb.cnt, e->nb.slot, t.l2cnt,
+            k_tape_list<<<block_count(n), block_threads(n), 0, st>>>(n, e->nb.n_pad, s.id, e->nb.cnt, e->nb.slot, t.l2cnt,
                                                  t.l2id);
             break;
         case TAPE_SOLVE:
-            k_tape_solve<<<nblk(n), kT, 0, st>>>(n, s.id, e->kv.x, s.bc, s.dir, t.praw, t.bc, t.dir);
+            k_tape_solve<<<block_count(n), block_threads(n), 0, st>>>(n, s.id, e->kv.x, s.bc, s.dir, t.praw, t.bc, t.dir);
             break;
     }
 }
@@ -663,13 +662,13 @@ Arr3 a3(double* const* p) { return Arr3{{p[0], p[1], p[2]}}; }
 // engine state <- (x, v, type) arrays in id order
 void restore(mps_trajectory* t, double* const* src, const int8_t* type_src) {
     mps_engine* e = t->e;
-    k_restore_state<<<nblk(t->n), kT, 0, e->st>>>(t->n, e->S().id, e->S(), e->c.planar, arr6(src),
+    k_restore_state<<<block_count(t->n), block_threads(t->n), 0, e->st>>>(t->n, e->S().id, e->S(), e->c.planar, arr6(src),
                                                   type_src);
 }
 
 void snapshot(mps_trajectory* t, double* const* dst, int8_t* type_dst) {
     mps_engine* e = t->e;
-    k_tape_state<<<nblk(t->n), kT, 0, e->st>>>(t->n, e->S().id, e->S(), e->c.planar, e->c.z0,
+    k_tape_state<<<block_count(t->n), block_threads(t->n), 0, e->st>>>(t->n, e->S().id, e->S(), e->c.planar, e->c.z0,
                                                arr6(dst), type_dst);
 }
 
@@ -692,8 +691,8 @@ int set_gravity(mps_trajectory* t, const double* g) {
 int record_sensors(mps_trajectory* t, int step) {
     if (t->nsens == 0) return MPS_OK;
     mps_engine* e = t->e;
-    k_to_id<<<nblk(t->n), kT, 0, e->st>>>(t->n, e->S().id, e->S().p, t->idp);
-    k_pick<<<nblk(t->nsens), kT, 0, e->st>>>(t->nsens, t->sensor, t->idp,
+    k_to_id<<<block_count(t->n), block_threads(t->n), 0, e->st>>>(t->n, e->S().id, e->S().p, t->idp);
+    k_pick<<<block_count(t->nsens), block_threads(t->nsens), 0, e->st>>>(t->nsens, t->sensor, t->idp,
                                              t->sens_out + (size_t)step * t->nsens);
     return MPS_OK;
 }
@@ -702,33 +701,33 @@ int record_sensors(mps_trajectory* t, int step) {
 int reverse_step(mps_trajectory* t, const TapeStep& T, int step) {
     mps_engine* e = t->e;
     const Consts& c = e->c;
-    const int n = t->n, G = nblk(n);
+    const int n = t->n, G = block_count(n);
     cudaStream_t st = e->st;
     Arr3 xb = a3(t->xb), vb = a3(t->vb), ab = a3(t->ab), vt = a3(t->vt), xx = a3(t->xextra);
     // move and pressure gradient
-    k_adj_move<<<G, kT, 0, st>>>(n, c.dt, c.planar, T.type1, xb, vb, ab);
-    k_adj_pplus<<<G, kT, 0, st>>>(n, T.praw, t->pplus);
-    k_adj_minp<<<G, kT, 0, st>>>(n, c, T, t->pplus, t->phat, t->amin);
-    k_adj_grad_local<<<G, kT, 0, st>>>(n, c, T, ab, t->phatbar);
-    k_adj_grad_gather<<<G, kT, 0, st>>>(n, c, T, t->pplus, t->phat, ab, t->phatbar, t->amin, xb,
+    k_adj_move<<<G, block_threads(n), 0, st>>>(n, c.dt, c.planar, T.type1, xb, vb, ab);
+    k_adj_pplus<<<G, block_threads(n), 0, st>>>(n, T.praw, t->pplus);
+    k_adj_minp<<<G, block_threads(n), 0, st>>>(n, c, T, t->pplus, t->phat, t->amin);
+    k_adj_grad_local<<<G, block_threads(n), 0, st>>>(n, c, T, ab, t->phatbar);
+    k_adj_grad_gather<<<G, block_threads(n), 0, st>>>(n, c, T, t->pplus, t->phat, ab, t->phatbar, t->amin, xb,
                                         t->pbar);
     if (t->nsens)
-        k_adj_sensor<<<nblk(t->nsens), kT, 0, st>>>(t->nsens, t->sensor,
+        k_adj_sensor<<<block_count(t->nsens), block_threads(t->nsens), 0, st>>>(t->nsens, t->sensor,
                                                     t->sens_bar + (size_t)step * t->nsens, t->pbar);
     // transpose Poisson solve (A is symmetric): A lambda = masked p_bar
-    k_adj_assemble<<<G, kT, 0, st>>>(n, c, T, t->pbar, e->A);
+    k_adj_assemble<<<G, block_threads(n), 0, st>>>(n, c, T, t->pbar, e->A);
     TCU(cudaMemsetAsync(e->ds, 0, sizeof(DevStats), st));
     launch_solve_fp64(c, e->A, e->kv, 1e-14, 4 * (int64_t)n + 100, e->ds, st);
-    k_adj_ppe_gather<<<G, kT, 0, st>>>(n, c, T, e->kv.x, xb);
+    k_adj_ppe_gather<<<G, block_threads(n), 0, st>>>(n, c, T, e->kv.x, xb);
     // collision pass
-    k_copy6<<<G, kT, 0, st>>>(n, arr6(T.st1), arr6(t->cur));
-    k_zero3<<<G, kT, 0, st>>>(n, xx);
+    k_copy6<<<G, block_threads(n), 0, st>>>(n, arr6(T.st1), arr6(t->cur));
+    k_zero3<<<G, block_threads(n), 0, st>>>(n, xx);
     k_adj_collision<<<1, 1, 0, st>>>(n, c, T, arr6(t->cur), t->rec, xb, vb, xx);
-    k_add3<<<G, kT, 0, st>>>(n, xx, xb);
+    k_add3<<<G, block_threads(n), 0, st>>>(n, xx, xb);
     // explicit part
-    k_adj_explicit_local<<<G, kT, 0, st>>>(n, c.dt, c.planar, T.type0, xb, vb, vt, ab);
+    k_adj_explicit_local<<<G, block_threads(n), 0, st>>>(n, c.dt, c.planar, T.type0, xb, vb, vt, ab);
     k_adj_gsum<<<1, 1024, 0, st>>>(n, ab, t->gbar);
-    k_adj_explicit_gather<<<G, kT, 0, st>>>(n, c, T, ab, vt, xb, vb);
+    k_adj_explicit_gather<<<G, block_threads(n), 0, st>>>(n, c, T, ab, vt, xb, vb);
     TCU(cudaMemcpyAsync(e->hs, e->ds, sizeof(DevStats), cudaMemcpyDeviceToHost, st));
     TCU(cudaStreamSynchronize(st));
     TCU(cudaGetLastError());
@@ -838,7 +837,7 @@ int mps_trajectory_forward(mps_trajectory* t, const double* vel0, const double* 
                 if (vel0[3 * i + 2] != 0.0) return tfail(MPS_ERR_ARG, "a planar engine keeps v_z = 0");
         std::memcpy(t->hstage, vel0, sizeof(double) * 3 * n);
         TCU(cudaMemcpyAsync(e->stage, t->hstage, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st));
-        k_deinterleave3<<<nblk(n), kT, 0, st>>>(n, e->stage, Arr3{{t->ic[3], t->ic[4], t->ic[5]}});
+        k_deinterleave3<<<block_count(n), block_threads(n), 0, st>>>(n, e->stage, Arr3{{t->ic[3], t->ic[4], t->ic[5]}});
     }
     restore(t, t->ic, t->ic_type);
     for (int s = 0; s < t->steps; s++) {
@@ -855,7 +854,7 @@ int mps_trajectory_forward(mps_trajectory* t, const double* vel0, const double* 
     for (int w = 0; w < 2; w++) {
         double* host = w == 0 ? pos_final : vel_final;
         if (!host) continue;
-        k_interleave3<<<nblk(n), kT, 0, st>>>(n, Arr3{{t->fin[3 * w], t->fin[3 * w + 1], t->fin[3 * w + 2]}},
+        k_interleave3<<<block_count(n), block_threads(n), 0, st>>>(n, Arr3{{t->fin[3 * w], t->fin[3 * w + 1], t->fin[3 * w + 2]}},
                                               e->stage);
         TCU(cudaMemcpyAsync(t->hstage, e->stage, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, st));
         TCU(cudaStreamSynchronize(st));
@@ -886,10 +885,10 @@ int mps_trajectory_backward(mps_trajectory* t, const double* d_sensor_pressure,
         if (host) {
             std::memcpy(t->hstage, host, sizeof(double) * 3 * n);
             TCU(cudaMemcpyAsync(e->stage, t->hstage, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st));
-            k_deinterleave3<<<nblk(n), kT, 0, st>>>(n, e->stage, Arr3{{dst[0], dst[1], dst[2]}});
+            k_deinterleave3<<<block_count(n), block_threads(n), 0, st>>>(n, e->stage, Arr3{{dst[0], dst[1], dst[2]}});
             TCU(cudaStreamSynchronize(st));
         } else {
-            k_zero3<<<nblk(n), kT, 0, st>>>(n, Arr3{{dst[0], dst[1], dst[2]}});
+            k_zero3<<<block_count(n), block_threads(n), 0, st>>>(n, Arr3{{dst[0], dst[1], dst[2]}});
         }
     }
     if (t->nsens) {
@@ -921,7 +920,7 @@ int mps_trajectory_backward(mps_trajectory* t, const double* d_sensor_pressure,
     for (int w = 0; w < 2; w++) {
         double* host = w == 0 ? d_pos0 : d_vel0;
         if (!host) continue;
-        k_interleave3<<<nblk(n), kT, 0, st>>>(n, a3(w == 0 ? t->xb : t->vb), e->stage);
+        k_interleave3<<<block_count(n), block_threads(n), 0, st>>>(n, a3(w == 0 ? t->xb : t->vb), e->stage);
         TCU(cudaMemcpyAsync(t->hstage, e->stage, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, st));
         TCU(cudaStreamSynchronize(st));
         std::memcpy(host, t->hstage, sizeof(double) * 3 * n);

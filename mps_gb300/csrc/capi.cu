@@ -265,11 +265,11 @@ void enqueue_pre_solve(mps_engine* e) {
     e->swap();
     launch_build_list_bc_source(c, e->S(), e->sc, e->nb, e->A, e->ds, st);
     if (taping) tape_phase(e, TAPE_LIST2);
-    launch_assemble(c, e->S(), e->nb, e->A, e->ds, st);
+    // solvePoissonEquation's symmetry test (src/mps.cpp:418-442): the assembly
+    // forms the fingerprint, or the mixed solver's setup, which reads the matrix anyway
+    launch_assemble(c, e->S(), e->nb, e->A, e->parent, e->has_surface, !mixed, e->ds, st);
     launch_dirichlet(c, e->S(), e->nb, e->A, e->parent, e->has_surface, e->ds, st);
-    // solvePoissonEquation's symmetry test (src/mps.cpp:418-442); the mixed
-    // solver's setup reads the matrix anyway and forms the fingerprint there
-    if (!mixed) launch_symmetry_check(c, e->S(), e->A, e->ds, st);
+    if (!mixed) launch_symmetry_locate(c, e->S(), e->A, e->ds, st);
 }
 
 // Mixed solver only: FP32 operator and multigrid hierarchy of this step.
@@ -631,7 +631,7 @@ int mps_create(const mps_params* prm, int32_t n, const double* pos, const double
     if ((rc = alloc_state(e, e->buf[0])) || (rc = alloc_state(e, e->buf[1]))) return bail(rc);
     const size_t np = e->n_pad, K = c.K;
     if (e->alloc(&e->sc.key, np) || e->alloc(&e->sc.rank, np) || e->alloc(&e->sc.perm, np) ||
-        e->alloc(&e->sc.skey, np) || e->alloc(&e->sc.cell_count, (size_t)c.nkeys + 2) ||
+        e->alloc(&e->sc.skey, np) || e->alloc(&e->sc.pid, np) || e->alloc(&e->sc.cell_count, (size_t)c.nkeys + 2) ||
         e->alloc(&e->sc.cell_start, (size_t)c.nkeys + 2) ||
         e->alloc(&e->sc.scan_tmp, scan_tmp_ints(std::max(c.nkeys + 1, n + 1))) ||
         e->alloc(&e->nb.cnt, np) || e->alloc(&e->nb.slot, np * K) || e->alloc(&e->nb.dist, np * K) ||

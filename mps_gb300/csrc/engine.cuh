@@ -128,6 +128,7 @@ struct CollPair {
 // ----------------------------------------------------------------- sort.cu
 struct SortScratch {
     int32_t *key, *rank, *perm, *skey;  // per slot
+    int32_t* pid;                       // ids in perm's order
     int32_t *cell_count, *cell_start;   // nkeys + 2
     int32_t *scan_tmp;                  // block sums
 };
@@ -214,18 +215,18 @@ void launch_build_list(const Consts& c, const StateBuf& s, const SortScratch& sc
 // setSourceTerm (src/mps.cpp:262-320; the higher-order source after it).
 void launch_build_list_bc_source(const Consts& c, const StateBuf& s, const SortScratch& sc,
                                  const NbList& nb, const Ppe& A, DevStats* ds, cudaStream_t st);
-void launch_assemble(const Consts& c, const StateBuf& s, const NbList& nb, const Ppe& A,
-                     DevStats* ds, cudaStream_t st);
+// fingerprint: also the symmetry fingerprint of the matrix (over slots) into
+// ds->sym_fp, for launch_symmetry_locate.  Also resets launch_dirichlet's parents.
+void launch_assemble(const Consts& c, const StateBuf& s, const NbList& nb, const Ppe& A, int32_t* parent,
+                     int8_t* has_surface, bool fingerprint, DevStats* ds, cudaStream_t st);
 void launch_dirichlet(const Consts& c, const StateBuf& s, const NbList& nb, const Ppe& A,
                       int32_t* parent, int8_t* has_surface, DevStats* ds, cudaStream_t st);
 // --------------------------------------------------------------- symcheck.cu
 // The symmetry test of solvePoissonEquation (src/mps.cpp:418-442) on the
-// assembled matrix: a one-pass fingerprint, and the first asymmetric pair
-// when it is not zero; raises ST_ASYMMETRIC, which makes the solvers skip.
-void launch_symmetry_check(const Consts& c, const StateBuf& s, const Ppe& A, DevStats* ds,
-                           cudaStream_t st);
-// The second half alone, after a kernel that accumulated the fingerprint
-// (the mixed setup does, over slots, while it reads the matrix).
+// assembled matrix, after a kernel that accumulated its fingerprint (the
+// assembly for the FP64 solver, the mixed setup for the mixed one, over slots):
+// where that is not zero, finds the first asymmetric pair and raises
+// ST_ASYMMETRIC, which makes the solvers skip.
 void launch_symmetry_locate(const Consts& c, const StateBuf& s, const Ppe& A, DevStats* ds,
                             cudaStream_t st);
 // x_prev (may be null) receives the solution by particle id.

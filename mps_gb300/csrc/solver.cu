@@ -2101,20 +2101,25 @@ __global__ void k_mixed_setup(Consts c, Ppe A, MatFree mf, Krylov kv, const int3
         // of index bytes (padding: range 0, offset 0, value 0)
         for (int m0 = 0; m0 < wq; m0 += 4) {
             float v4[4];
+            double v[4];
+            int j[4];
             uint32_t b4 = 0;
+#pragma unroll
+            for (int t = 0; t < 4; t++) {  // (all loads before their first use)
+                const size_t e = base + (size_t)min(m0 + t, w - 1) * 32;
+                v[t] = A.val[e];
+                j[t] = A.col[e];
+            }
 #pragma unroll
             for (int t = 0; t < 4; t++) {
                 const int m = m0 + t;
-                const size_t e = base + (size_t)m * 32;
-                const double v = m < w ? A.val[e] : 0.0;
-                v4[t] = m < w ? f32(v) : 0.f;
+                v4[t] = m < w ? f32(v[t]) : 0.f;
                 if (m < cnt) {
-                    const int j = A.col[e];
-                    fp += entry_term(k, j, v);
+                    fp += entry_term(k, j[t], v[t]);
                     if (mf.enabled) {
                         int r = 2;
-                        while (r > 0 && j < st[r]) r--;
-                        const int off = j - st[r];
+                        while (r > 0 && j[t] < st[r]) r--;
+                        const int off = j[t] - st[r];
                         if (off >= 0 && off < 64)
                             b4 |= (uint32_t)((r << 6) | off) << (8 * t);
                         else
@@ -2246,7 +2251,7 @@ void launch_mixed_setup(const Consts& c, const SortScratch& sc, const Ppe& A, Ma
     mf.cs = sc.cell_start;
     mf.numY = c.numY;
     mf.nkeys = c.nkeys;
-    k_mixed_setup<<<(c.n + 255) / 256, 256, 0, st>>>(c, A, mf, k, ids, warm ? 1 : 0, &ds->sym_fp);
+    k_mixed_setup<<<block_count(c.n), block_threads(c.n), 0, st>>>(c, A, mf, k, ids, warm ? 1 : 0, &ds->sym_fp);
     ++g_launches;
 }
 

@@ -14,9 +14,9 @@ namespace mpsg {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kBatchedList = 80000;  // most particles of the batched list build (k_build_list)
 constexpr int kCollBlocks = 304;  // blocks of the parallel collision pass (two per SM)
 
-inline int blocks_for(int n, int t = kThreads) { return (n + t - 1) / t; }
 
 __device__ __forceinline__ void raise_status(DevStats* ds, int32_t bit) { atomicOr(&ds->status, bit); }
 
@@ -30,27 +30,29 @@ __device__ __forceinline__ bool outside_domain(const Consts& c, double x, double
 // pre-filter at `bound`: pass 1 collects them in a local list, pass 2 calls
 // f(j), where f runs the exact FP64 test and the work.  Splitting the sweep
 // keeps the FP64 work on compact lists, with nearly all lanes of a warp busy.
-// A full list (3-D particles have ~120 neighbours) is worked off and filled
-// again, which keeps the order; running f on every candidate instead took
-// 0.75 ms on a 9,000-particle 3-D tank.
-constexpr int kNear = 64;
+// More survivors than the list holds: f(j) for every candidate (f's exact
+// test then selects the same neighbours in the same order).
 template <bool PLANAR, class F>
 __device__ __forceinline__ void for_each_near(const Consts& c, const StateBuf& s,
                                               const int32_t* __restrict__ cs, int32_t key, int k,
                                               float bound, F&& f) {
+    constexpr int kNear = PLANAR ? 64 : 256;  // ~28 and ~120 neighbours at 3.1 particle distances
     const float2 fk = s.xyf[k];
     const float fx = fk.x, fy = fk.y, fz = PLANAR ? 0.f : s.zf[k];
     int cand[kNear];
     int ns = 0;
     for_each_candidate<PLANAR>(c, cs, key, [&](int j) {
         if (j == k || far32<PLANAR>(s, j, fx, fy, fz, bound)) return;
-        if (ns == kNear) {
-            for (int q = 0; q < kNear; q++) f(cand[q]);
-            ns = 0;
-        }
-        cand[ns++] = j;
+        if (ns < kNear) cand[ns] = j;
+        ns++;
     });
-    for (int q = 0; q < ns; q++) f(cand[q]);
+    if (ns <= kNear) {
+        for (int q = 0; q < ns; q++) f(cand[q]);
+    } else {
+        for_each_candidate<PLANAR>(c, cs, key, [&](int j) {
+            if (j != k) f(j);
+        });
+    }
 }
 
 // Number density at re_p over a particle's current neighbours (d < re_max),
@@ -227,11 +229,15 @@ template <bool PLANAR>
 __global__ void __launch_bounds__(kThreads) k_coll_count(Consts c, StateBuf s,
                                                          const int32_t* __restrict__ skey,
                                                          const int32_t* __restrict__ cs,
-                                                         int32_t* __restrict__ cnt_by_id) {
+                                                         int32_t* __restrict__ cnt_by_id, CollWork cw) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= c.n || s.type[k] != T_FLUID) return;
-    int m = for_each_collision<PLANAR>(c, s, cs, skey[k], k, nullptr);
-    if (m) cnt_by_id[s.id[k]] = m;
+    if (k >= c.n) return;
+    // also resets the parallel pass's counters (every id once)
+    const int id = s.id[k];
+    cw.jn[id] = 0;
+    cw.ver[id] = 0;
+    if (k < 3) cw.ctl[k] = 0;
+    cnt_by_id[id] = s.type[k] == T_FLUID ? for_each_collision<PLANAR>(c, s, cs, skey[k], k, nullptr) : 0;
 }
 
 template <bool PLANAR>
@@ -422,7 +428,13 @@ __global__ void __launch_bounds__(kThreads) k_coll_wave(Consts c, StateBuf s, co
 // and the classic setSourceTerm (src/mps.cpp:262-320): the surface number
 // density summed over the list entries within re_s, in list order (the
 // order in which the reference's getNumberDensity reads the stored list).
-template <bool PLANAR, bool BC>
+//
+// Batches of B candidates in pass 2: their loads, square roots and divisions
+// are independent, only the append and the sums go in order.  With few warps
+// per SM quarter the kernel is bound by the latency of one particle's chain
+// (2,000 particles: 47 -> 27 us with B = 4); at 1M it is bound by issue, where
+// the batch's registers cost more than they give, and B = 1 stays.
+template <bool PLANAR, bool BC, int B>
 __global__ void __launch_bounds__(kThreads) k_build_list(Consts c, StateBuf s,
                                                          const int32_t* __restrict__ skey,
                                                          const int32_t* __restrict__ cs, NbList nb,
@@ -448,19 +460,32 @@ __global__ void __launch_bounds__(kThreads) k_build_list(Consts c, StateBuf s,
         });
         if (ns <= c.K) {
             // exact test, compacting in place (order kept): src/mps.cpp:585-619
-            for (int q = 0; q < ns; q++) {
-                const int j = nb.slot[(size_t)q * np + k];
-                const double d2 = dist2<PLANAR>(s, k, j, xi, yi, zi);
-                if (!lt_cut(d2, c.t_max)) continue;
-                const double dist = dsqrt(d2);
-                const double w = weight(dist, c.re_p);
-                if (lt_cut(dist, c.re_p)) nd = dadd(nd, w);  // src/mps.cpp:573-583
-                if (BC && lt_cut(dist, c.re_s)) nsurf = dadd(nsurf, weight(dist, c.re_s));
-                const size_t e = (size_t)m * np + k;
-                nb.slot[e] = j;
-                nb.dist[e] = dist;
-                nb.wp[e] = w;
-                m++;
+            for (int q0 = 0; q0 < ns; q0 += B) {
+                int j[B];
+                double dist[B], w[B], ws[B];
+                bool in[B];
+#pragma unroll
+                for (int t = 0; t < B; t++) j[t] = nb.slot[(size_t)min(q0 + t, ns - 1) * np + k];
+#pragma unroll
+                for (int t = 0; t < B; t++) {
+                    const double d2 = dist2<PLANAR>(s, k, j[t], xi, yi, zi);
+                    in[t] = q0 + t < ns && lt_cut(d2, c.t_max);
+                    if (B == 1 && !in[t]) continue;
+                    dist[t] = dsqrt(d2);
+                    w[t] = weight(dist[t], c.re_p);
+                    ws[t] = BC ? weight(dist[t], c.re_s) : 0.0;
+                }
+#pragma unroll
+                for (int t = 0; t < B; t++) {
+                    if (!in[t]) continue;
+                    if (lt_cut(dist[t], c.re_p)) nd = dadd(nd, w[t]);  // src/mps.cpp:573-583
+                    if (BC && lt_cut(dist[t], c.re_s)) nsurf = dadd(nsurf, ws[t]);
+                    const size_t e = (size_t)m * np + k;
+                    nb.slot[e] = j[t];
+                    nb.dist[e] = dist[t];
+                    nb.wp[e] = w[t];
+                    m++;
+                }
             }
         } else {
             // more survivors than the list holds: the exact one-pass sweep
@@ -531,31 +556,53 @@ __global__ void __launch_bounds__(kThreads) k_source_ho(Consts c, StateBuf s, Nb
     A.src[k] = b;
 }
 
-// MPS::setMatrix (src/mps.cpp:322-360): one SELL-32 row per Inner slot.
+// MPS::setMatrix (src/mps.cpp:322-360): one SELL-32 row per Inner slot.  With
+// FP also the matrix's symmetry fingerprint, from the entries as they are made
+// (a pass of its own read them all again: 22 us at 2,000 particles).
+template <bool FP>
 __global__ void __launch_bounds__(kThreads) k_assemble(Consts c, StateBuf s, NbList nb, Ppe A,
-                                                       DevStats* ds) {
+                                                       int32_t* __restrict__ parent,
+                                                       int8_t* __restrict__ has_surface, DevStats* ds) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     int off = 0;
+    unsigned long long fp = 0;
     if (k < c.n) {
+        parent[k] = k;  // the union-find's start (ensureDirichletBoundaryConnection)
+        has_surface[k] = 0;
         double diag = 0.0;
         double rsum = 0.0;  // diag + the off-diagonals: the terms of neighbours without an unknown
         if (s.bc[k] == BC_INNER) {
             const int np = nb.n_pad, m = nb.cnt[k];
             const size_t sbase = (size_t)(k >> 5) * c.K * 32 + (k & 31);
-            for (int q = 0; q < m; q++) {
-                int j = nb.slot[(size_t)q * np + k];
-                int8_t bj = s.bc[j];
-                if (bj == BC_IGNORED) continue;
-                double dist = nb.dist[(size_t)q * np + k];
-                if (!lt_cut(dist, c.re_p)) continue;
-                double a = ddiv(dmul(c.mat_c, nb.wp[(size_t)q * np + k]), c.rho);
-                diag = dadd(diag, a);
-                if (bj == BC_INNER) {
-                    A.col[sbase + (size_t)off * 32] = j;
-                    A.val[sbase + (size_t)off * 32] = -a;
-                    off++;
-                } else {
-                    rsum = dadd(rsum, a);
+            // four neighbours' loads and divisions at a time, sums in order
+            for (int q0 = 0; q0 < m; q0 += 4) {
+                int j[4];
+                int8_t bj[4];
+                double a[4];
+                bool in[4];
+#pragma unroll
+                for (int t = 0; t < 4; t++) {
+                    const size_t e = (size_t)min(q0 + t, m - 1) * np + k;
+                    j[t] = nb.slot[e];
+                    a[t] = nb.wp[e];
+                    in[t] = q0 + t < m && lt_cut(nb.dist[e], c.re_p);
+                }
+#pragma unroll
+                for (int t = 0; t < 4; t++) bj[t] = s.bc[j[t]];
+#pragma unroll
+                for (int t = 0; t < 4; t++) a[t] = ddiv(dmul(c.mat_c, a[t]), c.rho);
+#pragma unroll
+                for (int t = 0; t < 4; t++) {
+                    if (!in[t] || bj[t] == BC_IGNORED) continue;
+                    diag = dadd(diag, a[t]);
+                    if (bj[t] == BC_INNER) {
+                        A.col[sbase + (size_t)off * 32] = j[t];
+                        A.val[sbase + (size_t)off * 32] = -a[t];
+                        if (FP) fp += entry_term(k, j[t], -a[t]);
+                        off++;
+                    } else {
+                        rsum = dadd(rsum, a[t]);
+                    }
                 }
             }
             if (c.qc_on) {
@@ -580,6 +627,12 @@ __global__ void __launch_bounds__(kThreads) k_assemble(Consts c, StateBuf s, NbL
     }
     if ((threadIdx.x & 31) == 0 && (k >> 5) < (c.n + 31) / 32) {
         A.slice_w[k >> 5] = w;
+    }
+    if (FP) {
+        fp = warp_sum64(fp);
+        if ((threadIdx.x & 31) == 0 && fp) atomicAdd(&ds->sym_fp, fp);
+    }
+    if ((threadIdx.x & 31) == 0 && (k >> 5) < (c.n + 31) / 32) {
         if (tot) atomicAdd(&ds->nnz_off, (unsigned long long)tot);
     }
 }
@@ -619,11 +672,6 @@ __device__ void uf_union(int* par, int a, int b, DevStats* ds) {
     raise_status(ds, ST_TIMEOUT);
 }
 
-__global__ void k_cc_init(int n, int* par) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) par[k] = k;
-}
-
 // Sampled linking (the Afforest scheme of Sutton et al., 2018): almost every
 // particle of a scene belongs to one large component, and its edges need not
 // all be processed.  Pass 1 joins each particle to the components of its first
@@ -635,7 +683,7 @@ __global__ void k_cc_init(int n, int* par) {
 // the components, and every flag derived from them, are those of processing
 // all edges.
 constexpr int kCcLinks = 2;
-constexpr int kCcSamples = 1024;
+constexpr int kCcSamples = 256;  // (a wrong guess costs time only; 1,024 took 18 us to count)
 
 __global__ void __launch_bounds__(kThreads) k_cc_link(Consts c, StateBuf s, NbList nb, int* par,
                                                       DevStats* ds) {
@@ -741,14 +789,27 @@ __global__ void __launch_bounds__(kThreads) k_gradient(Consts c, StateBuf s, NbL
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= c.n || s.bc[k] == BC_IGNORED) return;
     const int np = nb.n_pad, m = nb.cnt[k];
+    // four neighbours' loads at a time (the columns of the list are one trip to
+    // memory, the neighbours' fields a second), minima and sums in list order
     double pmin = s.p[k];
-    for (int q = 0; q < m; q++) {
-        int j = nb.slot[(size_t)q * np + k];
-        if (s.type[j] == T_DUMMY) continue;
-        if (lt_cut(nb.dist[(size_t)q * np + k], c.re_p)) {
-            double pj = s.p[j];
-            if (pmin > pj) pmin = pj;
+    for (int q0 = 0; q0 < m; q0 += 4) {
+        int j[4];
+        bool in[4];
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            const size_t e = (size_t)min(q0 + t, m - 1) * np + k;
+            j[t] = nb.slot[e];
+            in[t] = q0 + t < m && lt_cut(nb.dist[e], c.re_p);
         }
+        double pj[4];
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            pj[t] = s.p[j[t]];
+            in[t] = in[t] && s.type[j[t]] != T_DUMMY;
+        }
+#pragma unroll
+        for (int t = 0; t < 4; t++)
+            if (in[t] && pmin > pj[t]) pmin = pj[t];
     }
     s.minp[k] = pmin;
     // a fluid particle is never Ignored (only dummies and ghosts are)
@@ -756,17 +817,40 @@ __global__ void __launch_bounds__(kThreads) k_gradient(Consts c, StateBuf s, NbL
     const double xi = s.x[k], yi = s.y[k], zi = PLANAR ? 0.0 : s.z[k];
     if (!MIXED) {
         double gx = 0.0, gy = 0.0, gz = 0.0;
-        for (int q = 0; q < m; q++) {
-            int j = nb.slot[(size_t)q * np + k];
-            if (s.type[j] == T_DUMMY) continue;
-            double dist = nb.dist[(size_t)q * np + k];
-            if (!lt_cut(dist, c.re_p)) continue;
-            double dp = dsub(s.p[j], pmin);
-            double w = nb.wp[(size_t)q * np + k];
-            double d2 = dmul(dist, dist);
-            gx = dadd(gx, ddiv(dmul(dmul(dsub(s.x[j], xi), dp), w), d2));
-            gy = dadd(gy, ddiv(dmul(dmul(dsub(s.y[j], yi), dp), w), d2));
-            if (!PLANAR) gz = dadd(gz, ddiv(dmul(dmul(dsub(s.z[j], zi), dp), w), d2));
+        for (int q0 = 0; q0 < m; q0 += 4) {
+            int j[4];
+            double dist[4], w[4], dp[4], tx[4], ty[4], tz[4];
+            bool in[4];
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                const size_t e = (size_t)min(q0 + t, m - 1) * np + k;
+                j[t] = nb.slot[e];
+                dist[t] = nb.dist[e];
+                w[t] = nb.wp[e];
+            }
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                in[t] = q0 + t < m && lt_cut(dist[t], c.re_p) && s.type[j[t]] != T_DUMMY;
+                dp[t] = s.p[j[t]];
+                tx[t] = s.x[j[t]];
+                ty[t] = s.y[j[t]];
+                tz[t] = PLANAR ? 0.0 : s.z[j[t]];
+            }
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                dp[t] = dsub(dp[t], pmin);
+                const double d2 = dmul(dist[t], dist[t]);
+                tx[t] = ddiv(dmul(dmul(dsub(tx[t], xi), dp[t]), w[t]), d2);
+                ty[t] = ddiv(dmul(dmul(dsub(ty[t], yi), dp[t]), w[t]), d2);
+                if (!PLANAR) tz[t] = ddiv(dmul(dmul(dsub(tz[t], zi), dp[t]), w[t]), d2);
+            }
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                if (!in[t]) continue;
+                gx = dadd(gx, tx[t]);
+                gy = dadd(gy, ty[t]);
+                if (!PLANAR) gz = dadd(gz, tz[t]);
+            }
         }
         gx = dmul(gx, c.grad_scale);
         gy = dmul(gy, c.grad_scale);
@@ -781,17 +865,33 @@ __global__ void __launch_bounds__(kThreads) k_gradient(Consts c, StateBuf s, NbL
         float gx = 0.f, gy = 0.f;
         const float2 hk = s.xyf[k], lk = s.xylo[k];
         const float pmh = f32(pmin), pml = f32(pmin - (double)pmh);
-        for (int q = 0; q < m; q++) {
-            int j = nb.slot[(size_t)q * np + k];
-            if (s.type[j] == T_DUMMY) continue;
-            double dist = nb.dist[(size_t)q * np + k];
-            if (!lt_cut(dist, c.re_p)) continue;
-            const float2 hj = s.xyf[j], lj = s.xylo[j], pj = s.pf[j];
-            const float fd = f32(dist);
-            const float dp = (pj.x - pmh) + (pj.y - pml);
-            const float coef = dp * (c.fre_p / fd - 1.f) / (fd * fd);
-            gx = fmaf((hj.x - hk.x) + (lj.x - lk.x), coef, gx);
-            gy = fmaf((hj.y - hk.y) + (lj.y - lk.y), coef, gy);
+        for (int q0 = 0; q0 < m; q0 += 4) {
+            int j[4];
+            double dist[4];
+            float2 hj[4], lj[4], pj[4];
+            bool in[4];
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                const size_t e = (size_t)min(q0 + t, m - 1) * np + k;
+                j[t] = nb.slot[e];
+                dist[t] = nb.dist[e];
+            }
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                in[t] = q0 + t < m && lt_cut(dist[t], c.re_p) && s.type[j[t]] != T_DUMMY;
+                hj[t] = s.xyf[j[t]];
+                lj[t] = s.xylo[j[t]];
+                pj[t] = s.pf[j[t]];
+            }
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                if (!in[t]) continue;
+                const float fd = f32(dist[t]);
+                const float dp = (pj[t].x - pmh) + (pj[t].y - pml);
+                const float coef = dp * (c.fre_p / fd - 1.f) / (fd * fd);
+                gx = fmaf((hj[t].x - hk.x) + (lj[t].x - lk.x), coef, gx);
+                gy = fmaf((hj[t].y - hk.y) + (lj[t].y - lk.y), coef, gy);
+            }
         }
         const float sc = -c.fgrad_scale / f32(c.rho);
         ax[k] = (double)(gx * sc);
@@ -869,21 +969,21 @@ __global__ void k_number_density(Consts c, StateBuf s) {
 
 void launch_explicit(const Consts& c, const StateBuf& in, const StateBuf& out,
                      const SortScratch& sc, int mixed, DevStats* ds, cudaStream_t st) {
-    int nb = blocks_for(c.n);
+    int nb = block_count(c.n);
     if (c.planar) {
         if (mixed) {
-            k_explicit<true, true><<<nb, kThreads, 0, st>>>(c, in, out, sc.skey, sc.cell_start, ds);
+            k_explicit<true, true><<<nb, block_threads(c.n), 0, st>>>(c, in, out, sc.skey, sc.cell_start, ds);
             ++g_launches;
         } else {
-            k_explicit<true, false><<<nb, kThreads, 0, st>>>(c, in, out, sc.skey, sc.cell_start, ds);
+            k_explicit<true, false><<<nb, block_threads(c.n), 0, st>>>(c, in, out, sc.skey, sc.cell_start, ds);
             ++g_launches;
         }
     } else {
         if (mixed) {
-            k_explicit<false, true><<<nb, kThreads, 0, st>>>(c, in, out, sc.skey, sc.cell_start, ds);
+            k_explicit<false, true><<<nb, block_threads(c.n), 0, st>>>(c, in, out, sc.skey, sc.cell_start, ds);
             ++g_launches;
         } else {
-            k_explicit<false, false><<<nb, kThreads, 0, st>>>(c, in, out, sc.skey, sc.cell_start, ds);
+            k_explicit<false, false><<<nb, block_threads(c.n), 0, st>>>(c, in, out, sc.skey, sc.cell_start, ds);
             ++g_launches;
         }
     }
@@ -892,29 +992,25 @@ void launch_explicit(const Consts& c, const StateBuf& in, const StateBuf& out,
 void launch_collision(const Consts& c, const StateBuf& s, const SortScratch& sc,
                       int32_t* cand_cnt, int32_t* cand_base, const CollWork& cw, CollPair* pairs,
                       int32_t pair_cap, int32_t* scan_tmp, DevStats* ds, cudaStream_t st) {
-    int nb = blocks_for(c.n);
-    cudaMemsetAsync(cand_cnt, 0, sizeof(int32_t) * (c.n + 1), st);
+    int nb = block_count(c.n);
     if (c.planar) {
-        k_coll_count<true><<<nb, kThreads, 0, st>>>(c, s, sc.skey, sc.cell_start, cand_cnt);
+        k_coll_count<true><<<nb, block_threads(c.n), 0, st>>>(c, s, sc.skey, sc.cell_start, cand_cnt, cw);
         ++g_launches;
     } else {
-        k_coll_count<false><<<nb, kThreads, 0, st>>>(c, s, sc.skey, sc.cell_start, cand_cnt);
+        k_coll_count<false><<<nb, block_threads(c.n), 0, st>>>(c, s, sc.skey, sc.cell_start, cand_cnt, cw);
         ++g_launches;
     }
     launch_exclusive_scan(cand_cnt, cand_base, c.n, scan_tmp, st);
     const int32_t* total = cand_base + c.n;
     if (c.planar) {
-        k_coll_write<true><<<nb, kThreads, 0, st>>>(c, s, sc.skey, sc.cell_start, cand_cnt,
+        k_coll_write<true><<<nb, block_threads(c.n), 0, st>>>(c, s, sc.skey, sc.cell_start, cand_cnt,
                                                     cand_base, pairs, pair_cap, ds);
     } else {
-        k_coll_write<false><<<nb, kThreads, 0, st>>>(c, s, sc.skey, sc.cell_start, cand_cnt,
+        k_coll_write<false><<<nb, block_threads(c.n), 0, st>>>(c, s, sc.skey, sc.cell_start, cand_cnt,
                                                      cand_base, pairs, pair_cap, ds);
     }
     ++g_launches;
     if (!cw.serial) {
-        cudaMemsetAsync(cw.jn, 0, sizeof(int32_t) * c.n, st);
-        cudaMemsetAsync(cw.ver, 0, sizeof(int32_t) * c.n, st);
-        cudaMemsetAsync(cw.ctl, 0, sizeof(int32_t) * 4, st);
         k_coll_jlists<<<kCollBlocks, kThreads, 0, st>>>(s, pairs, total, pair_cap, cw);
         if (c.planar)
             k_coll_wave<true><<<kCollBlocks, kThreads, 0, st>>>(c, s, pairs, total, pair_cap, cand_cnt,
@@ -931,99 +1027,103 @@ void launch_collision(const Consts& c, const StateBuf& s, const SortScratch& sc,
     ++g_launches;
 }
 
+template <bool PLANAR, bool BC>
+static void build_list(const Consts& c, const StateBuf& s, const SortScratch& sc, const NbList& nb, const Ppe& A,
+                       DevStats* ds, cudaStream_t st) {
+    if (c.n <= kBatchedList)
+        k_build_list<PLANAR, BC, 4><<<block_count(c.n), block_threads(c.n), 0, st>>>(c, s, sc.skey, sc.cell_start, nb,
+                                                                                    A, ds);
+    else
+        k_build_list<PLANAR, BC, 1><<<block_count(c.n), block_threads(c.n), 0, st>>>(c, s, sc.skey, sc.cell_start, nb,
+                                                                                    A, ds);
+    ++g_launches;
+}
+
 void launch_build_list(const Consts& c, const StateBuf& s, const SortScratch& sc,
                        const NbList& nb, DevStats* ds, cudaStream_t st) {
-    int g = blocks_for(c.n);
     const Ppe none{};
-    if (c.planar) {
-        k_build_list<true, false><<<g, kThreads, 0, st>>>(c, s, sc.skey, sc.cell_start, nb, none, ds);
-        ++g_launches;
-    } else {
-        k_build_list<false, false><<<g, kThreads, 0, st>>>(c, s, sc.skey, sc.cell_start, nb, none, ds);
-        ++g_launches;
-    }
+    if (c.planar)
+        build_list<true, false>(c, s, sc, nb, none, ds, st);
+    else
+        build_list<false, false>(c, s, sc, nb, none, ds, st);
 }
 
 void launch_build_list_bc_source(const Consts& c, const StateBuf& s, const SortScratch& sc,
                                  const NbList& nb, const Ppe& A, DevStats* ds, cudaStream_t st) {
-    int g = blocks_for(c.n);
-    if (c.planar) {
-        k_build_list<true, true><<<g, kThreads, 0, st>>>(c, s, sc.skey, sc.cell_start, nb, A, ds);
-        ++g_launches;
-    } else {
-        k_build_list<false, true><<<g, kThreads, 0, st>>>(c, s, sc.skey, sc.cell_start, nb, A, ds);
-        ++g_launches;
-    }
+    if (c.planar)
+        build_list<true, true>(c, s, sc, nb, A, ds, st);
+    else
+        build_list<false, true>(c, s, sc, nb, A, ds, st);
     if (c.ho_on) {
-        if (c.planar) {
-            k_source_ho<true><<<g, kThreads, 0, st>>>(c, s, nb, A);
-            ++g_launches;
-        } else {
-            k_source_ho<false><<<g, kThreads, 0, st>>>(c, s, nb, A);
-            ++g_launches;
-        }
+        const int g = block_count(c.n), T = block_threads(c.n);
+        if (c.planar)
+            k_source_ho<true><<<g, T, 0, st>>>(c, s, nb, A);
+        else
+            k_source_ho<false><<<g, T, 0, st>>>(c, s, nb, A);
+        ++g_launches;
     }
 }
 
-void launch_assemble(const Consts& c, const StateBuf& s, const NbList& nb, const Ppe& A,
-                     DevStats* ds, cudaStream_t st) {
-    k_assemble<<<blocks_for(c.n), kThreads, 0, st>>>(c, s, nb, A, ds);
+void launch_assemble(const Consts& c, const StateBuf& s, const NbList& nb, const Ppe& A, int32_t* parent,
+                     int8_t* has_surface, bool fingerprint, DevStats* ds, cudaStream_t st) {
+    const int g = block_count(c.n), T = block_threads(c.n);
+    if (fingerprint)
+        k_assemble<true><<<g, T, 0, st>>>(c, s, nb, A, parent, has_surface, ds);
+    else
+        k_assemble<false><<<g, T, 0, st>>>(c, s, nb, A, parent, has_surface, ds);
     ++g_launches;
 }
 
 void launch_dirichlet(const Consts& c, const StateBuf& s, const NbList& nb, const Ppe& A,
                       int32_t* parent, int8_t* has_surface, DevStats* ds, cudaStream_t st) {
-    int g = blocks_for(c.n);
-    cudaMemsetAsync(has_surface, 0, c.n, st);
+    int g = block_count(c.n);
     int* giant = parent + c.n;  // the parent array has one spare element
-    k_cc_init<<<g, kThreads, 0, st>>>(c.n, parent);
+    k_cc_link<<<g, block_threads(c.n), 0, st>>>(c, s, nb, parent, ds);
     ++g_launches;
-    k_cc_link<<<g, kThreads, 0, st>>>(c, s, nb, parent, ds);
+    k_cc_compress<<<g, block_threads(c.n), 0, st>>>(c.n, parent, ds);
     ++g_launches;
-    k_cc_compress<<<g, kThreads, 0, st>>>(c.n, parent, ds);
+    k_cc_giant<<<1, kCcSamples, 0, st>>>(c.n, parent, giant);
     ++g_launches;
-    k_cc_giant<<<1, 1024, 0, st>>>(c.n, parent, giant);
+    k_cc_hook<<<g, block_threads(c.n), 0, st>>>(c, s, nb, parent, giant, ds);
     ++g_launches;
-    k_cc_hook<<<g, kThreads, 0, st>>>(c, s, nb, parent, giant, ds);
+    k_cc_mark<<<g, block_threads(c.n), 0, st>>>(c, s, parent, has_surface, ds);
     ++g_launches;
-    k_cc_mark<<<g, kThreads, 0, st>>>(c, s, parent, has_surface, ds);
-    ++g_launches;
-    k_cc_apply<<<g, kThreads, 0, st>>>(c, s, parent, has_surface, A, ds);
+    k_cc_apply<<<g, block_threads(c.n), 0, st>>>(c, s, parent, has_surface, A, ds);
     ++g_launches;
 }
 
 void launch_pressure_post(const Consts& c, const StateBuf& s, const NbList& nb, const double* x,
                           double* x_prev, double* ax, double* ay, double* az, int mixed,
                           DevStats* ds, cudaStream_t st) {
-    int g = blocks_for(c.n);
-    k_pressure_out<<<g, kThreads, 0, st>>>(c.n, x, s.p, s.pf, s.id, x_prev, ds);
+    int g = block_count(c.n);
+    k_pressure_out<<<g, block_threads(c.n), 0, st>>>(c.n, x, s.p, s.pf, s.id, x_prev, ds);
     ++g_launches;
     if (c.planar) {
         if (mixed) {
-            k_gradient<true, true><<<g, kThreads, 0, st>>>(c, s, nb, ax, ay, az);
+            k_gradient<true, true><<<g, block_threads(c.n), 0, st>>>(c, s, nb, ax, ay, az);
             ++g_launches;
         } else {
-            k_gradient<true, false><<<g, kThreads, 0, st>>>(c, s, nb, ax, ay, az);
+            k_gradient<true, false><<<g, block_threads(c.n), 0, st>>>(c, s, nb, ax, ay, az);
             ++g_launches;
         }
-        k_move2<true><<<g, kThreads, 0, st>>>(c, s, ax, ay, az, ds);
+        k_move2<true><<<g, block_threads(c.n), 0, st>>>(c, s, ax, ay, az, ds);
         ++g_launches;
     } else {
         if (mixed) {
-            k_gradient<false, true><<<g, kThreads, 0, st>>>(c, s, nb, ax, ay, az);
+            k_gradient<false, true><<<g, block_threads(c.n), 0, st>>>(c, s, nb, ax, ay, az);
             ++g_launches;
         } else {
-            k_gradient<false, false><<<g, kThreads, 0, st>>>(c, s, nb, ax, ay, az);
+            k_gradient<false, false><<<g, block_threads(c.n), 0, st>>>(c, s, nb, ax, ay, az);
             ++g_launches;
         }
-        k_move2<false><<<g, kThreads, 0, st>>>(c, s, ax, ay, az, ds);
+        k_move2<false><<<g, block_threads(c.n), 0, st>>>(c, s, ax, ay, az, ds);
         ++g_launches;
     }
 }
 
 void launch_number_density(const Consts& c, const StateBuf& s, const NbList& /*nb*/,
                            cudaStream_t st) {
-    k_number_density<<<blocks_for(c.n), kThreads, 0, st>>>(c, s);
+    k_number_density<<<block_count(c.n), block_threads(c.n), 0, st>>>(c, s);
     ++g_launches;
 }
 

@@ -127,18 +127,10 @@ int grid_for(int n) { return (n + kSymThreads - 1) / kSymThreads; }
 
 }  // namespace
 
-void launch_symmetry_check(const Consts& c, const StateBuf& s, const Ppe& A, DevStats* ds,
-                           cudaStream_t st) {
-    SellRows rows{A.offcnt, A.col, A.val, s.id, c.K, c.n};
-    k_sym_fingerprint<<<grid_for(c.n), kSymThreads, 0, st>>>(rows, &ds->sym_fp);
-    ++g_launches;
-    launch_symmetry_locate(c, s, A, ds, st);
-}
-
 void launch_symmetry_locate(const Consts& c, const StateBuf& s, const Ppe& A, DevStats* ds,
                             cudaStream_t st) {
     SellRows rows{A.offcnt, A.col, A.val, s.id, c.K, c.n};
-    k_sym_locate<<<grid_for(c.n), kSymThreads, 0, st>>>(rows, &ds->sym_fp, &ds->asym_big, &ds->asym_any,
+    k_sym_locate<<<block_count(c.n), block_threads(c.n), 0, st>>>(rows, &ds->sym_fp, &ds->asym_big, &ds->asym_any,
                                                         &ds->status);
     ++g_launches;
 }
