@@ -57,6 +57,12 @@ static __device__ __noinline__ float f32_fp64(double x) { return __double2float_
 __device__ __forceinline__ double ddiv(double a, double b) {
     double q;
     if (x64::div_rn<Fp32Approx>(a, b, q)) return q;
+    // +-0 over a normal number is +-0 (clamped pressures make most of a resting
+    // scene's gradient terms 0, and one such lane would send its warp through
+    // the FP64 instructions)
+    const uint64_t A = x64::bits_of(a), B = x64::bits_of(b);
+    if ((A << 1) == 0 && ((uint32_t)(B >> 52) & 0x7ffu) - 1u < 2046u)
+        return x64::double_of((A ^ B) & (1ull << 63));
     return ddiv_fp64(a, b);
 }
 __device__ __forceinline__ double dsqrt(double a) {
@@ -166,6 +172,49 @@ __device__ __forceinline__ bool far32(const StateBuf& s, int j, float fx, float 
         r += dz * dz;
     }
     return r > bound;
+}
+
+// The candidates of slot k (itself left out) that survive the FP32 pre-filter,
+// in sweep order: four candidates' positions are loaded and tested at a time.
+template <bool PLANAR, class F>
+__device__ __forceinline__ void for_each_survivor(const Consts& c, const StateBuf& s,
+                                                  const int32_t* __restrict__ cs, int32_t key, int k, float bound,
+                                                  F&& f) {
+    const float2 fk = s.xyf[k];
+    const float fx = fk.x, fy = fk.y, fz = PLANAR ? 0.f : s.zf[k];
+    auto range = [&](int b, int e) {
+#pragma unroll 1
+        for (int j0 = b; j0 < e; j0 += 4) {
+            bool near[4];
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                const int j = min(j0 + t, e - 1);
+                near[t] = !far32<PLANAR>(s, j, fx, fy, fz, bound) && j0 + t < e && j != k;
+            }
+#pragma unroll
+            for (int t = 0; t < 4; t++)
+                if (near[t]) f(j0 + t);
+        }
+    };
+    if (PLANAR) {
+        const int kk = key - 1;
+        int b[3], e[3];
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            b[r] = __ldg(cs + kk + (r - 1) * c.numY);
+            e[r] = __ldg(cs + kk + (r - 1) * c.numY + 3);
+        }
+#pragma unroll 1
+        for (int r = 0; r < 3; r++) range(r == 0 ? b[0] : (r == 1 ? b[1] : b[2]), r == 0 ? e[0] : (r == 1 ? e[1] : e[2]));
+    } else {
+#pragma unroll 1
+        for (int jx = -1; jx <= 1; jx++)
+#pragma unroll 1
+            for (int jy = -1; jy <= 1; jy++) {
+                const int kk = key + (jx * c.numY + jy) * c.numZ - 1;
+                range(__ldg(cs + kk), __ldg(cs + kk + 3));
+            }
+    }
 }
 
 // Symmetry fingerprint of a matrix (the test of solvePoissonEquation,

@@ -217,18 +217,18 @@ __global__ void k_mg_dense(MgLevel L, float* out) {
         M[i][j] = v;
     }
     __syncthreads();
-    // 32 x 32 threads, each with up to 3 x 3 entries: per pivot the row and the
+    // 32 x W threads (W >= n / 3), each with up to 3 x 3 entries: per pivot the row and the
     // column of the pivot are read, then every entry is updated (two block
     // barriers and no index division; strided loops with four barriers took
     // 20 us at 40 cells and 72 us at 90)
     static_assert(kMgMaxCoarsest <= 96, "three rows and columns per thread");
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, W = blockDim.x >> 5;
     for (int k = 0; k < n; k++) {
         const float piv = 1.f / M[k][k];
         float row[3], col[3];
 #pragma unroll
         for (int q = 0; q < 3; q++) {
-            const int j = tx + 32 * q, i = ty + 32 * q;
+            const int j = tx + 32 * q, i = ty + W * q;
             row[q] = j < n ? (j == k ? 1.f : M[k][j]) * piv : 0.f;
             col[q] = i < n ? M[i][k] : 0.f;
         }
@@ -237,7 +237,7 @@ __global__ void k_mg_dense(MgLevel L, float* out) {
         for (int a = 0; a < 3; a++)
 #pragma unroll
             for (int b = 0; b < 3; b++) {
-                const int i = ty + 32 * a, j = tx + 32 * b;
+                const int i = ty + W * a, j = tx + 32 * b;
                 if (i >= n || j >= n) continue;
                 if (i == k)
                     M[i][j] = row[b];
@@ -269,7 +269,8 @@ void launch_mg_setup(const Consts& c, const Ppe& A, const MatFree& mf, const Mg&
         k_mg_coarsen<<<block_count(C.nx * C.ny), block_threads(C.nx * C.ny), 0, st>>>(mg.lev[l], C, mg.omega, mg.nact + l + 1);
         ++g_launches;
     }
-    k_mg_dense<<<1, 1024, 0, st>>>(mg.lev[mg.nlev], mg.dense);
+    const int nd = mg.lev[mg.nlev].nx * mg.lev[mg.nlev].ny;
+    k_mg_dense<<<1, 32 * ((nd + 2) / 3), 0, st>>>(mg.lev[mg.nlev], mg.dense);
     ++g_launches;
 }
 

@@ -383,7 +383,7 @@ __device__ __forceinline__ bool solve_reduce_f2(GridBar& gb, const F2 (&v)[3], f
 
 // ------------------------------------------------------------------ SpMV
 // y_i = sum over the SELL-32 row (padding entries are (i, 0)) + diag_i x_i,
-// loads batched four at a time so that gathers overlap.
+// loads batched eight and four at a time so that gathers overlap.
 __device__ __forceinline__ double spmv64_row(const Ppe& A, int K, int sl, int lane, int row,
                                              const double* __restrict__ x, double xi) {
     const int w = __ldg(A.slice_w + sl);
@@ -391,16 +391,37 @@ __device__ __forceinline__ double spmv64_row(const Ppe& A, int K, int sl, int la
     const double* vp = A.val + (size_t)sl * K * 32 + lane;
     double s0 = 0.0, s1 = 0.0;
     int m = 0;
-    for (; m + 4 <= w; m += 4) {
-        int c0 = __ldg(cp + (m + 0) * 32), c1 = __ldg(cp + (m + 1) * 32);
-        int c2 = __ldg(cp + (m + 2) * 32), c3 = __ldg(cp + (m + 3) * 32);
-        double v0 = __ldg(vp + (m + 0) * 32), v1 = __ldg(vp + (m + 1) * 32);
-        double v2 = __ldg(vp + (m + 2) * 32), v3 = __ldg(vp + (m + 3) * 32);
-        double x0 = __ldcg(x + c0), x1 = __ldcg(x + c1), x2 = __ldcg(x + c2), x3 = __ldcg(x + c3);
-        s0 = fma(v0, x0, s0);
-        s1 = fma(v1, x1, s1);
-        s0 = fma(v2, x2, s0);
-        s1 = fma(v3, x3, s1);
+    for (; m + 8 <= w; m += 8) {
+        int c[8];
+        double v[8], g[8];
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+            c[t] = __ldg(cp + (m + t) * 32);
+            v[t] = __ldg(vp + (m + t) * 32);
+        }
+#pragma unroll
+        for (int t = 0; t < 8; t++) g[t] = __ldcg(x + c[t]);
+#pragma unroll
+        for (int t = 0; t < 8; t += 2) {
+            s0 = fma(v[t], g[t], s0);
+            s1 = fma(v[t + 1], g[t + 1], s1);
+        }
+    }
+    if (m + 4 <= w) {
+        int c[4];
+        double v[4], g[4];
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            c[t] = __ldg(cp + (m + t) * 32);
+            v[t] = __ldg(vp + (m + t) * 32);
+        }
+#pragma unroll
+        for (int t = 0; t < 4; t++) g[t] = __ldcg(x + c[t]);
+        s0 = fma(v[0], g[0], s0);
+        s1 = fma(v[1], g[1], s1);
+        s0 = fma(v[2], g[2], s0);
+        s1 = fma(v[3], g[3], s1);
+        m += 4;
     }
     for (; m < w; m++) s0 = fma(__ldg(vp + m * 32), __ldcg(x + __ldg(cp + m * 32)), s0);
     return fma(A.diag[row], xi, s0 + s1);
@@ -484,14 +505,14 @@ __device__ __forceinline__ float compact_row_sum(const Ppe& A, const MatFree& mf
     };
     float a0 = 0.f, a1 = 0.f;
     const int groups = (w + 3) >> 2;
-    int g = 0;
-    for (; g + kGroups <= groups; g += kGroups) {
+    for (int g = 0; g < groups; g += kGroups) {
         float4 v[kGroups];
         uint32_t b4[kGroups];
 #pragma unroll
         for (int q = 0; q < kGroups; q++) {
-            v[q] = __ldg(vp + (g + q) * 32);
-            b4[q] = __ldg(ip + (g + q) * 32);
+            const int h = min(g + q, groups - 1);
+            v[q] = __ldg(vp + h * 32);
+            b4[q] = __ldg(ip + h * 32);
         }
         float x[kGroups][4];
 #pragma unroll
@@ -500,22 +521,12 @@ __device__ __forceinline__ float compact_row_sum(const Ppe& A, const MatFree& mf
             for (int t = 0; t < 4; t++) x[q][t] = __ldcg(u + col(b4[q], t)) - ui;
 #pragma unroll
         for (int q = 0; q < kGroups; q++) {
+            if (g + q >= groups) break;
             a0 = fmaf(v[q].x, x[q][0], a0);
             a1 = fmaf(v[q].y, x[q][1], a1);
             a0 = fmaf(v[q].z, x[q][2], a0);
             a1 = fmaf(v[q].w, x[q][3], a1);
         }
-    }
-    for (; g < groups; g++) {
-        const float4 v = __ldg(vp + g * 32);
-        const uint32_t b4 = __ldg(ip + g * 32);
-        float x[4];
-#pragma unroll
-        for (int t = 0; t < 4; t++) x[t] = __ldcg(u + col(b4, t)) - ui;
-        a0 = fmaf(v.x, x[0], a0);
-        a1 = fmaf(v.y, x[1], a1);
-        a0 = fmaf(v.z, x[2], a0);
-        a1 = fmaf(v.w, x[3], a1);
     }
     return a0 + a1;
 }
@@ -594,16 +605,15 @@ __device__ __forceinline__ void off_rows(const Ppe& A, const MatFree& mf, int K,
         o2 = i2 >= 0 ? spmv32_sell_row(A, K, i2, v, vi2) : 0.f;
         return;
     }
-    const int j2 = i2 >= 0 ? i2 : i;  // a lone row is paired with itself
+    const int j2 = i2 >= 0 ? i2 : i;
     const int8_t fa = mf.sell_row[i], fb = mf.sell_row[j2];
     const int wa = __ldg(A.slice_w + (i >> 5)), wb = __ldg(A.slice_w + (j2 >> 5));
     const int sa[3] = {__ldg(mf.rs + i), __ldg(mf.rs + mf.rs_stride + i), __ldg(mf.rs + 2 * mf.rs_stride + i)};
     const int sb[3] = {__ldg(mf.rs + j2), __ldg(mf.rs + mf.rs_stride + j2), __ldg(mf.rs + 2 * mf.rs_stride + j2)};
     // pairs need a group in each row (a slice of rows without off-diagonals
     // has width 0 and no stored groups at all)
-    if (!fa && !fb && wa > 0 && wb > 0) {
-        compact_pair(A, mf, K, i, j2, wa, wb, sa, sb, v, vi, i2 >= 0 ? vi2 : vi, o, o2);
-        if (i2 < 0) o2 = 0.f;
+    if (i2 >= 0 && !fa && !fb && wa > 0 && wb > 0) {
+        compact_pair(A, mf, K, i, j2, wa, wb, sa, sb, v, vi, vi2, o, o2);
         return;
     }
     o = fa ? spmv32_sell_row(A, K, i, v, vi) : compact_row_sum(A, mf, K, i, v, vi);
@@ -1853,8 +1863,11 @@ __device__ __forceinline__ void solve_mixed_overlap(const Ppe& A, const MatFree&
                 const bool ok = mg_split_cycle<NV>(mg, gb, ds, ((warp * G + b) << 5) + lane, G * NV, sm, floats, s_cp);
                 if (tid == 0) s_cycle_ok = ok;
             } else {
-                for (int sla = sl0 + warp - kVW; sla < sl1; sla += 2 * kZW) {
-                    const int slb = sla + kZW;
+                // two slices per warp at a time (off_rows pairs their rows) once
+                // every warp has one: pairing sooner would only idle the others
+                const int step = sl1 - sl0 > kZW ? 2 : 1;
+                for (int sla = sl0 + warp - kVW; sla < sl1; sla += step * kZW) {
+                    const int slb = step == 2 ? sla + kZW : sl1;
                     const int i = sla * 32 + lane;
                     int i2 = slb < sl1 ? slb * 32 + lane : -1;
                     if (i2 >= n) i2 = -1;

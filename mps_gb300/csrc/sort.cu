@@ -63,41 +63,42 @@ __global__ void k_gather(int n, int nkeys, const int32_t* __restrict__ perm, con
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     const int o = perm[p];
-    const int32_t kk = key[o];
+    const int32_t kk = key[o], me = pid[p];
+    // the particle's fields, in flight while its place is found
+    const double x = in.x[o], y = in.y[o], vx = in.vx[o], vy = in.vy[o];
+    const double z = planar ? 0.0 : in.z[o], vz = planar ? 0.0 : in.vz[o];
+    const double pr = in.p[o], minp = in.minp[o], ndr = in.ndr[o], nd_last = in.nd_last[o];
+    const int8_t type = in.type[o], bc = in.bc[o], dir = in.dir[o];
     int k = p;
     if (kk < nkeys) {
         const int b = start[kk], e = start[kk + 1];
-        const int32_t me = pid[p];
         k = b;
 #pragma unroll 4
         for (int t = b; t < e; t++) k += pid[t] < me;
     }
     skey[k] = kk;
-    const double x = in.x[o], y = in.y[o];
     out.x[k] = x;
     out.y[k] = y;
     const float xh = f32(x), yh = f32(y);
     out.xyf[k] = make_float2(xh, yh);
     // x - xh is exact in FP64 (xh is x rounded to 24 bits)
     out.xylo[k] = make_float2(f32(x - (double)xh), f32(y - (double)yh));
-    const double vx = in.vx[o], vy = in.vy[o];
     out.vx[k] = vx;
     out.vy[k] = vy;
     out.vf[k] = make_float2(f32(vx), f32(vy));
     if (!planar) {
-        const double z = in.z[o];
         out.z[k] = z;
         out.zf[k] = f32(z);
-        out.vz[k] = in.vz[o];
+        out.vz[k] = vz;
     }
-    out.p[k] = in.p[o];
-    out.minp[k] = in.minp[o];
-    out.ndr[k] = in.ndr[o];
-    out.nd_last[k] = in.nd_last[o];
-    out.id[k] = in.id[o];
-    out.type[k] = in.type[o];
-    out.bc[k] = in.bc[o];
-    out.dir[k] = in.dir[o];
+    out.p[k] = pr;
+    out.minp[k] = minp;
+    out.ndr[k] = ndr;
+    out.nd_last[k] = nd_last;
+    out.id[k] = me;
+    out.type[k] = type;
+    out.bc[k] = bc;
+    out.dir[k] = dir;
 }
 
 // ---- exclusive scan (one block, or three passes: tile sums, scan of sums, tile scan) ----

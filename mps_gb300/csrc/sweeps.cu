@@ -37,12 +37,9 @@ __device__ __forceinline__ void for_each_near(const Consts& c, const StateBuf& s
                                               const int32_t* __restrict__ cs, int32_t key, int k,
                                               float bound, F&& f) {
     constexpr int kNear = PLANAR ? 64 : 256;  // ~28 and ~120 neighbours at 3.1 particle distances
-    const float2 fk = s.xyf[k];
-    const float fx = fk.x, fy = fk.y, fz = PLANAR ? 0.f : s.zf[k];
     int cand[kNear];
     int ns = 0;
-    for_each_candidate<PLANAR>(c, cs, key, [&](int j) {
-        if (j == k || far32<PLANAR>(s, j, fx, fy, fz, bound)) return;
+    for_each_survivor<PLANAR>(c, s, cs, key, k, bound, [&](int j) {
         if (ns < kNear) cand[ns] = j;
         ns++;
     });
@@ -62,11 +59,8 @@ template <bool PLANAR>
 __device__ double sweep_number_density_p(const Consts& c, const StateBuf& s, const int32_t* cs,
                                          int32_t key, int k) {
     double xi = s.x[k], yi = s.y[k], zi = PLANAR ? 0.0 : s.z[k];
-    const float2 fk = s.xyf[k];
-    const float fx = fk.x, fy = fk.y, fz = PLANAR ? 0.f : s.zf[k];
     double nd = 0.0;
-    for_each_candidate<PLANAR>(c, cs, key, [&](int j) {
-        if (j == k || far32<PLANAR>(s, j, fx, fy, fz, c.ft_max)) return;
+    for_each_survivor<PLANAR>(c, s, cs, key, k, c.ft_max, [&](int j) {
         double d2 = dist2<PLANAR>(s, k, j, xi, yi, zi);
         if (lt_cut(d2, c.t_max) && lt_cut(d2, c.t_p)) nd = dadd(nd, weight(dsqrt(d2), c.re_p));
     });
@@ -210,12 +204,9 @@ __device__ __forceinline__ int for_each_collision(const Consts& c, const StateBu
                                                   const int32_t* cs, int32_t key, int k,
                                                   CollPair* out) {
     double xi = s.x[k], yi = s.y[k], zi = PLANAR ? 0.0 : s.z[k];
-    const float2 fk = s.xyf[k];
-    const float fx = fk.x, fy = fk.y, fz = PLANAR ? 0.f : s.zf[k];
     int32_t idi = s.id[k];
     int m = 0;
-    for_each_candidate<PLANAR>(c, cs, key, [&](int j) {
-        if (j == k || far32<PLANAR>(s, j, fx, fy, fz, c.ft_cd)) return;
+    for_each_survivor<PLANAR>(c, s, cs, key, k, c.ft_cd, [&](int j) {
         double d2 = dist2<PLANAR>(s, k, j, xi, yi, zi);
         if (!(lt_cut(d2, c.t_max) && lt_cut(d2, c.t_cd))) return;
         if (s.type[j] == T_FLUID && s.id[j] >= idi) return;
@@ -446,15 +437,12 @@ __global__ void __launch_bounds__(kThreads) k_build_list(Consts c, StateBuf s,
     double nd = 0.0, nsurf = 0.0;  // number densities at re_p and (BC) re_s
     if (valid) {
         const double xi = s.x[k], yi = s.y[k], zi = PLANAR ? 0.0 : s.z[k];
-        const float2 fk = s.xyf[k];
-        const float fx = fk.x, fy = fk.y, fz = PLANAR ? 0.f : s.zf[k];
         // Pass 1: the candidates that survive the FP32 pre-filter, in sweep
         // order.  Pass 2 then runs the exact FP64 test, square root and
         // division on these compact per-particle lists, with nearly all lanes
         // of a warp busy (a candidate survives for only part of a warp).
         int ns = 0;
-        for_each_candidate<PLANAR>(c, cs, skey[k], [&](int j) {
-            if (j == k || far32<PLANAR>(s, j, fx, fy, fz, c.ft_max)) return;
+        for_each_survivor<PLANAR>(c, s, cs, skey[k], k, c.ft_max, [&](int j) {
             if (ns < c.K) nb.slot[(size_t)ns * np + k] = j;
             ns++;
         });
