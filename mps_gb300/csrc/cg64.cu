@@ -24,6 +24,8 @@
 //  * an exchange is one tagged store per block and value and one polling warp
 //    per value in every block (no counter, no second trip for the sums);
 //    divisions run once per block, in that warp, on the integer pipe.
+// Scenes of up to 4,000 rows run on one cluster of 16 blocks, whose exchange is a
+// hardware barrier and stores into the other blocks' shared memory.
 // A window that does not fit shared memory (very wide scenes) makes the whole
 // grid gather p from global memory, with a third exchange per iteration.
 #include <algorithm>
@@ -95,7 +97,21 @@ __device__ __forceinline__ double warp_add2(double a, double b, int lane) {
     return v;
 }
 
-template <int M, bool RELEASE, int BS, class Post>
+// In a cluster (CL) the sums go straight into the other blocks' shared memory
+// and its hardware barrier is both the wait and the release; the blocks of a
+// cluster are always co-resident, so it needs no limit.
+constexpr int kCluster64 = 16;
+
+__device__ __forceinline__ void st_remote64(const double* local, int rank, double v) {
+    unsigned a = (unsigned)__cvta_generic_to_shared(local), r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(r), "d"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_barrier64() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+template <int M, bool RELEASE, int BS, bool CL, class Post>
 __device__ __forceinline__ bool exchange(Exchange& ex, const double (&v)[M], bool warp_has_rows,
                                          double (&tot)[M], double (&aux)[M], DevStats* ds, Post&& post) {
     constexpr int kW = BS / 32;
@@ -103,6 +119,7 @@ __device__ __forceinline__ bool exchange(Exchange& ex, const double (&v)[M], boo
     __shared__ double sh[M][kW];
     __shared__ double s_tot[M], s_aux[M];
     __shared__ int s_bad[M];
+    __shared__ double slots[CL ? 2 : 1][M][kCluster64];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if constexpr (M == 2) {
         double s = 0.0;
@@ -118,6 +135,34 @@ __device__ __forceinline__ bool exchange(Exchange& ex, const double (&v)[M], boo
     }
     __syncthreads();
     ex.number++;
+    if constexpr (CL) {
+        const int par = ex.number & 1;
+        if (warp < M) {
+            double s = lane < kW ? sh[warp][lane] : 0.0;
+#pragma unroll
+            for (int o = kW / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            // kW lanes hold the sum, at least as many as the cluster has blocks
+            if (lane < ex.size) st_remote64(&slots[par][warp][ex.rank], lane, s);
+        }
+        cluster_barrier64();
+        if (warp < M) {
+            double t = lane < ex.size ? slots[par][warp][lane] : 0.0;
+#pragma unroll
+            for (int o = kCluster64 / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            const double x = post((int)warp, t);
+            if (lane == 0) {
+                s_tot[warp] = t;
+                s_aux[warp] = x;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < M; m++) {
+            tot[m] = s_tot[m];
+            aux[m] = s_aux[m];
+        }
+        return true;
+    }
     if (warp < M) {
         double s = lane < kW ? sh[warp][lane] : 0.0;
 #pragma unroll
@@ -244,7 +289,7 @@ __device__ __forceinline__ double row_gather(const double* __restrict__ vp, cons
     return s0 + s1;
 }
 
-template <int BS>
+template <int BS, bool CL>
 __global__ void __launch_bounds__(BS, 1) k_cg64(Ppe A, Krylov kv, Cg64Args a, DevStats* ds) {
     extern __shared__ __align__(16) unsigned char smem[];
     if (*(volatile int32_t*)&ds->status & ST_ASYMMETRIC) {  // the reference exits here
@@ -255,6 +300,7 @@ __global__ void __launch_bounds__(BS, 1) k_cg64(Ppe A, Krylov kv, Cg64Args a, De
         }
         return;
     }
+    if (CL) cluster_barrier64();  // every block runs before any stores into its shared memory
     constexpr int kW = BS / 32;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     Exchange ex{reinterpret_cast<unsigned long long*>(kv.partials), 0u, (int)blockIdx.x, (int)gridDim.x};
@@ -386,7 +432,7 @@ __global__ void __launch_bounds__(BS, 1) k_cg64(Ppe A, Krylov kv, Cg64Args a, De
     }
     // no rows: the block still tells whether its (empty) window fits
     auto none = [](int, double) { return 0.0; };
-    if (!exchange<3, true, BS>(ex, acc, has_rows, tot, aux, ds, none)) return;
+    if (!exchange<3, true, BS, CL>(ex, acc, has_rows, tot, aux, ds, none)) return;
     const double rhs2 = tot[0];
     const bool gather = tot[2] > 0.0;
     double rn2 = rhs2, rz = tot[1], beta = 0.0;
@@ -453,7 +499,7 @@ __global__ void __launch_bounds__(BS, 1) k_cg64(Ppe A, Krylov kv, Cg64Args a, De
                 if (i < a.n) __stcg(kv.p + i, fma(beta, __ldcg(kv.p + i), __ldcg(kv.z + i)));
             }
             double none1[1] = {0.0};
-            if (!exchange<1, true, BS>(ex, none1, false, t1, x1, ds, none)) return;
+            if (!exchange<1, true, BS, CL>(ex, none1, false, t1, x1, ds, none)) return;
             for (int s = warp; s < S; s += kW) {
                 const int i = row_of(s);
                 if (i >= a.n) continue;
@@ -465,7 +511,7 @@ __global__ void __launch_bounds__(BS, 1) k_cg64(Ppe A, Krylov kv, Cg64Args a, De
                 pq[0] = fma(p, q, pq[0]);
             }
         }
-        if (!exchange<1, false, BS>(ex, pq, has_rows, t1, x1, ds,
+        if (!exchange<1, false, BS, CL>(ex, pq, has_rows, t1, x1, ds,
                                     [&](int, double t) { return ddiv(rz, t); }))
             return;
         const double alpha = x1[0];
@@ -497,7 +543,7 @@ __global__ void __launch_bounds__(BS, 1) k_cg64(Ppe A, Krylov kv, Cg64Args a, De
                 a2[1] = fma(r, z, a2[1]);
             }
         }
-        if (!exchange<2, true, BS>(ex, a2, has_rows, t2, x2, ds, [&](int m, double t) {
+        if (!exchange<2, true, BS, CL>(ex, a2, has_rows, t2, x2, ds, [&](int m, double t) {
                 return m == 0 ? (t < thr ? 1.0 : 0.0) : ddiv(t, rz);
             }))
             return;
@@ -513,6 +559,7 @@ __global__ void __launch_bounds__(BS, 1) k_cg64(Ppe A, Krylov kv, Cg64Args a, De
     if (resident && !gather)  // (where the grid gathers, every block works on the global arrays)
         for (int s = warp; s < S; s += kW)
             if (row_of(s) < a.n) kv.x[row_of(s)] = sx[s * 32 + lane];
+    if (CL) cluster_barrier64();  // no block leaves while another may still store into its slots
     if (blockIdx.x == 0 && tid == 0) {
         ds->cg_iterations = it;
         ds->refinements = 0;
@@ -527,9 +574,14 @@ constexpr int kSmem64 = 224 * 1024;
 // together); fewer: 512 (cheaper block barriers).
 constexpr int kWideSlices = 32;
 
+// Largest scene of the one-cluster form: per iteration 6.6 us up to 2,000 rows,
+// 7.6 at 3,400 and 9.0 at 4,500 (16 SMs issue all the FP64 work) against 8.2 to
+// 8.4 us for one block per SM at any of these sizes.
+constexpr int kClusterRows64 = 4000;
+
 template <int BS>
 int grid64(int device) {
-    const void* fn = (const void*)k_cg64<BS>;
+    const void* fn = (const void*)k_cg64<BS, false>;
     int sms = 0, per = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem64) != cudaSuccess ||
@@ -544,6 +596,37 @@ int grid64(int device) {
 
 int cg64_grid(int device) { return std::min(grid64<512>(device), grid64<1024>(device)); }
 
+namespace {
+void cluster_launch64(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& at, int blocks, cudaStream_t st) {
+    cfg = cudaLaunchConfig_t{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(512);
+    cfg.dynamicSmemBytes = kSmem64;
+    cfg.stream = st;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = blocks;
+    at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+}
+}  // namespace
+
+int cg64_cluster() {
+    const void* fn = (const void*)k_cg64<512, true>;
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem64);
+    cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    for (int blocks = kCluster64; blocks >= 8; blocks /= 2) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at[1];
+        cluster_launch64(cfg, at[0], blocks, nullptr);
+        int fit = 0;
+        if (cudaOccupancyMaxActiveClusters(&fit, fn, &cfg) == cudaSuccess && fit > 0) return blocks;
+        cudaGetLastError();
+    }
+    return 0;
+}
+
 void launch_solve_fp64(const Consts& c, const Ppe& A, const Krylov& k, double tol, int64_t max_iter,
                        DevStats* ds, cudaStream_t st) {
     Cg64Args a;
@@ -554,15 +637,24 @@ void launch_solve_fp64(const Consts& c, const Ppe& A, const Krylov& k, double to
     a.tol = tol;
     a.max_iter = max_iter;
     a.lidx = reinterpret_cast<uint16_t*>(A.val32);  // the mixed solver's values: not used by this one
-    const int grid = std::min(k.grid, a.nslices);
     Ppe AA = A;
     Krylov kk = k;
     void* args[] = {&AA, &kk, &a, &ds};
+    ++g_launches;
+    if (k.cluster64 > 0 && c.n <= kClusterRows64) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at[1];
+        int blocks = k.cluster64;  // a power of two, no more than there are slices
+        while (blocks > a.nslices) blocks /= 2;
+        cluster_launch64(cfg, at[0], blocks, st);
+        cudaLaunchKernelExC(&cfg, (const void*)k_cg64<512, true>, args);
+        return;
+    }
+    const int grid = std::min(k.grid, a.nslices);
     cudaMemsetAsync(k.partials, 0, sizeof(unsigned long long) * 16 * grid, st);
     const bool wide = a.nslices > kWideSlices * grid;
-    const void* fn = wide ? (const void*)k_cg64<1024> : (const void*)k_cg64<512>;
+    const void* fn = wide ? (const void*)k_cg64<1024, false> : (const void*)k_cg64<512, false>;
     cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(wide ? 1024 : 512), args, kSmem64, st);
-    ++g_launches;
 }
 
 }  // namespace mpsg

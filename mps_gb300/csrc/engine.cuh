@@ -313,7 +313,8 @@ struct Krylov {
     unsigned int* barrier;  // monotonically increasing arrival counter
     double* totals;         // unused scratch (8 doubles)
     int32_t grid;           // cooperative grid size
-    int32_t cluster;        // blocks of a one-cluster solve (0: the device runs none)
+    int32_t cluster;        // blocks of a one-cluster mixed solve (0: the device runs none)
+    int32_t cluster64;      // the same for the FP64 solve
     int32_t block;
 };
 void solver_setup(Krylov& k, int32_t n_pad, int device);
@@ -323,6 +324,8 @@ int selftest_wait_limit(int blocks, int* gave_up, int* status, float* ms);
 // ----------------------------------------------------------------- cg64.cu
 // Blocks the FP64 solve may use on the device (0: it does not fit).
 int cg64_grid(int device);
+// Blocks of its one-cluster form (0: the device runs none).
+int cg64_cluster();
 // Solves A x = b; returns through DevStats (iterations, residual, status).
 // A.val32 is scratch of this solve.
 void launch_solve_fp64(const Consts& c, const Ppe& A, const Krylov& k, double tol,

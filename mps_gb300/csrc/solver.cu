@@ -2256,6 +2256,7 @@ void solver_setup(Krylov& k, int32_t /*n_pad*/, int device) {
     k.grid = std::min({g1, g2, g3});
     k.block = kBlock;
     k.cluster = cluster_blocks();
+    k.cluster64 = cg64_cluster();
 }
 
 void launch_mixed_setup(const Consts& c, const SortScratch& sc, const Ppe& A, MatFree& mf,
