@@ -256,7 +256,7 @@ void enqueue_pre_solve(mps_engine* e) {
     launch_explicit(c, e->S(), e->buf[e->cur ^ 1], e->sc, mixed, e->ds, st);
     e->swap();
     if (taping) tape_phase(e, TAPE_EXPLICIT);
-    launch_rebuild(c, e->S(), e->buf[e->cur ^ 1], e->sc, e->ds, st);
+    launch_rebuild(c, e->S(), e->buf[e->cur ^ 1], e->sc, e->ds, st, true);
     e->swap();
     launch_collision(c, e->S(), e->sc, e->cand_cnt, e->cand_base, e->cw, e->pairs, e->pair_cap,
                      e->sc.scan_tmp, e->ds, st);
@@ -714,6 +714,7 @@ int mps_create(const mps_params* prm, int32_t n, const double* pos, const double
         cudaMemsetAsync(t.z, 0, np * 8, e->st);
         cudaMemsetAsync(t.vz, 0, np * 8, e->st);
     }
+    cudaMemsetAsync(e->sc.cell_count, 0, sizeof(int32_t) * ((size_t)c.nkeys + 2), e->st);
     cudaMemsetAsync(e->kv.x, 0, np * 8, e->st);
     cudaMemsetAsync(e->kv.x_prev, 0, np * 8, e->st);
     cudaMemsetAsync(e->nb.cnt, 0, np * 4, e->st);

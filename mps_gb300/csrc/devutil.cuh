@@ -112,6 +112,26 @@ __device__ __forceinline__ int32_t cell_key(const Consts& c, double x, double y,
     return (ix * c.numY + iy) * c.numZ + iz;
 }
 
+// Counts slot k into its cell: the cell key (nkeys for ghosts) and the slot's
+// rank among the cell's arrivals.  A particle whose position is not finite
+// becomes a ghost: the reference has no defined behaviour here; it is taken out
+// of the neighbour search and the step reports an error.
+__device__ __forceinline__ void count_cell(const Consts& c, int k, double x, double y, double z, int8_t& type,
+                                           int32_t* __restrict__ key, int32_t* __restrict__ rank,
+                                           int32_t* __restrict__ count, DevStats* ds) {
+    int32_t kk = c.nkeys;
+    if (type != T_GHOST) {
+        if (isfinite(x) && isfinite(y) && isfinite(z)) {
+            kk = cell_key(c, x, y, z);
+        } else {
+            type = T_GHOST;
+            atomicOr(&ds->status, ST_NONFINITE);
+        }
+    }
+    key[k] = kk;
+    rank[k] = atomicAdd(count + kk, 1);
+}
+
 // Visits the candidate slots of the 3x3(x3) cells around `key` in the
 // reference's order: jx outer, jy, jz inner (src/mps.cpp:599-601), and
 // ascending id inside a cell.  Keys are x-major, so the cells of one jx

@@ -129,13 +129,15 @@ struct CollPair {
 struct SortScratch {
     int32_t *key, *rank, *perm, *skey;  // per slot
     int32_t* pid;                       // ids in perm's order
-    int32_t *cell_count, *cell_start;   // nkeys + 2
+    int32_t *cell_count, *cell_start;   // nkeys + 2; the counts are 0 between builds
     int32_t *scan_tmp;                  // block sums
 };
+// counted: the slots' keys and ranks are there (launch_explicit made them).
 void launch_rebuild(const Consts& c, const StateBuf& in, const StateBuf& out, SortScratch& s,
-                    DevStats* ds, cudaStream_t st);
-// exclusive scan of n int32 (in-place allowed); out has n+1 entries (total last)
-void launch_exclusive_scan(const int32_t* in, int32_t* out, int32_t n, int32_t* tmp,
+                    DevStats* ds, cudaStream_t st, bool counted = false);
+// exclusive scan of n int32 (in-place allowed unless clear); out has n+1 entries
+// (total last); clear: `in` is 0 afterwards
+void launch_exclusive_scan(int32_t* in, int32_t* out, int32_t n, int32_t* tmp, bool clear,
                            cudaStream_t st);
 size_t scan_tmp_ints(int32_t n);
 
@@ -195,6 +197,7 @@ struct MatFree {
 
 void launch_initial_number_density(const Consts& c, const StateBuf& s, const SortScratch& sc,
                                    const NbList& nb, DevStats* ds, cudaStream_t st);
+// Also counts the moved particles into their cells for the next build.
 void launch_explicit(const Consts& c, const StateBuf& in, const StateBuf& out,
                      const SortScratch& sc, int mixed, DevStats* ds, cudaStream_t st);
 // Buffers of the collision pass's parallel application (sweeps.cu).

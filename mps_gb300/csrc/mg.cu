@@ -42,22 +42,6 @@ __device__ __forceinline__ int list_active(bool act, int I, int32_t* list, int32
     return act ? pos : -1;
 }
 
-// Every cell's r, e and t to 0 on the levels the grid-wide phases visit by
-// list (levels 1 .. ngrid + 1), and the list lengths to 0.
-__global__ void k_mg_clear(Mg mg) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
-    if (t < kMgMaxLevels) mg.nact[t] = 0;
-    for (int l = 1; l <= mg.ngrid + 1 && l <= mg.nlev; l++) {
-        const MgLevel& L = mg.lev[l];
-        const int n = L.nx * L.ny;
-        for (int I = t; I < n; I += nt) {
-            L.r[I] = 0.f;
-            L.e[I] = 0.f;
-            L.t[I] = 0.f;
-        }
-    }
-}
-
 // Level 1's 9-point stencil of cell I: the sum over the cell's rows of
 // their row-to-cell sums B (k_mg_rowcell), which is P1^T A P1 (rows that are
 // not unknowns have B = 0).  Nine coalesced loads per row instead of a walk
@@ -85,8 +69,22 @@ __global__ void k_mg_level1(Consts c, MgLevel L, const float* __restrict__ B, si
 // Smoothed transfer: B = A P1 per slot (the row's sums over the 3x3 cells
 // around its own, diagonal included), in the entry order of k_mg_level1.
 // Slots that are not unknowns get 0.
-__global__ void k_mg_rowcell(Consts c, Ppe A, MatFree mf, size_t np, float* __restrict__ B) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+//
+// Also, for the cycle: every cell's r, e and t to 0 on the levels the grid-wide
+// phases visit by list (levels 1 .. ngrid + 1), and the list lengths to 0.
+__global__ void k_mg_rowcell(Consts c, Ppe A, MatFree mf, Mg mg) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+    const size_t np = (size_t)mg.n_pad;
+    float* __restrict__ B = mg.rowcell;
+    if (i < kMgMaxLevels) mg.nact[i] = 0;
+    for (int l = 1; l <= mg.ngrid + 1 && l <= mg.nlev; l++) {
+        const MgLevel& L = mg.lev[l];
+        for (int I = i; I < L.nx * L.ny; I += nt) {
+            L.r[I] = 0.f;
+            L.e[I] = 0.f;
+            L.t[I] = 0.f;
+        }
+    }
     if (i >= c.n) return;
     float st[9];
 #pragma unroll
@@ -152,10 +150,8 @@ __global__ void k_mg_rowcell(Consts c, Ppe A, MatFree mf, size_t np, float* __re
 // omega invd_j r_j (one Jacobi step from zero on F, then its residual);
 // summed over the 2x2 children it is a fixed 4x4 stencil on r_F, whose
 // weights depend only on the operator and omega.
-__global__ void k_mg_coarsen(MgLevel F, MgLevel C, float omega, int32_t* nact_c) {
-    const int I = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void coarsen_cell(const MgLevel& F, const MgLevel& C, float omega, int32_t* nact_c, int I) {
     const int nc = C.nx * C.ny;
-    if (I >= nc) return;
     const int X = I / C.ny, Y = I - X * C.ny;
     const int nf = F.nx * F.ny;
     float st[9], w[16];
@@ -198,9 +194,14 @@ __global__ void k_mg_coarsen(MgLevel F, MgLevel C, float omega, int32_t* nact_c)
     for (int k = 0; k < 16; k++) C.rw[(size_t)k * nc + I] = w[k];
 }
 
+__global__ void k_mg_coarsen(MgLevel F, MgLevel C, float omega, int32_t* nact_c) {
+    const int I = blockIdx.x * blockDim.x + threadIdx.x;
+    if (I < C.nx * C.ny) coarsen_cell(F, C, omega, nact_c, I);
+}
+
 // Dense inverse of the coarsest operator; cells without unknowns get an
 // identity row so that the matrix stays invertible (their residual is 0).
-__global__ void k_mg_dense(MgLevel L, float* out) {
+__device__ __forceinline__ void dense_inverse(const MgLevel& L, float* out) {
     __shared__ float M[kMgMaxCoarsest][kMgMaxCoarsest];
     const int n = L.nx * L.ny;
     for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
@@ -217,10 +218,9 @@ __global__ void k_mg_dense(MgLevel L, float* out) {
         M[i][j] = v;
     }
     __syncthreads();
-    // 32 x W threads (W >= n / 3), each with up to 3 x 3 entries: per pivot the row and the
+    // 32 x 32 threads, each with up to 3 x 3 entries: per pivot the row and the
     // column of the pivot are read, then every entry is updated (two block
-    // barriers and no index division; strided loops with four barriers took
-    // 20 us at 40 cells and 72 us at 90)
+    // barriers per pivot and no index division)
     static_assert(kMgMaxCoarsest <= 96, "three rows and columns per thread");
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, W = blockDim.x >> 5;
     for (int k = 0; k < n; k++) {
@@ -251,27 +251,41 @@ __global__ void k_mg_dense(MgLevel L, float* out) {
     for (int t = threadIdx.x; t < n * n; t += blockDim.x) out[t] = M[t / n][t % n];
 }
 
+// The levels after `first`, one after another, and the coarsest one's inverse: a
+// few thousand cells, for which a launch each costs more than one block's time
+// (and a batch makes all of them once per scene).
+constexpr int kTailThreads = 1024;
+constexpr int kTailCells = 2048;
+__global__ void __launch_bounds__(kTailThreads) k_mg_tail(__grid_constant__ const Mg mg, int first) {
+    for (int l = first; l < mg.nlev; l++) {
+        const MgLevel &F = mg.lev[l], &C = mg.lev[l + 1];
+        for (int I = threadIdx.x; I < C.nx * C.ny; I += kTailThreads)
+            coarsen_cell(F, C, mg.omega, mg.nact + l + 1, I);
+        __syncthreads();
+    }
+    dense_inverse(mg.lev[mg.nlev], mg.dense);
+}
+
 }  // namespace
 
 void launch_mg_setup(const Consts& c, const Ppe& A, const MatFree& mf, const Mg& mg,
                      cudaStream_t st) {
     if (!mg.enabled) return;
     // the rows' 3x3-cell sums: the operator of modes 1 and 3, and level 1's stencil
-    k_mg_rowcell<<<block_count(c.n), block_threads(c.n), 0, st>>>(c, A, mf, (size_t)mg.n_pad, mg.rowcell);
-    ++g_launches;
+    k_mg_rowcell<<<block_count(c.n), block_threads(c.n), 0, st>>>(c, A, mf, mg);
     const MgLevel& L1 = mg.lev[1];
-    k_mg_clear<<<block_count(L1.nx * L1.ny), block_threads(L1.nx * L1.ny), 0, st>>>(mg);
-    k_mg_level1<<<block_count(L1.nx * L1.ny), block_threads(L1.nx * L1.ny), 0, st>>>(c, L1, mg.rowcell, (size_t)mg.n_pad, mf.cs, mg.nact,
-                                                             mg.act1_rng);
-    g_launches += 2;
-    for (int l = 1; l < mg.nlev; l++) {
+    k_mg_level1<<<block_count(L1.nx * L1.ny), block_threads(L1.nx * L1.ny), 0, st>>>(
+        c, L1, mg.rowcell, (size_t)mg.n_pad, mf.cs, mg.nact, mg.act1_rng);
+    int l = 1;
+    for (; l < mg.nlev; l++) {
         const MgLevel& C = mg.lev[l + 1];
-        k_mg_coarsen<<<block_count(C.nx * C.ny), block_threads(C.nx * C.ny), 0, st>>>(mg.lev[l], C, mg.omega, mg.nact + l + 1);
+        const int nc = C.nx * C.ny;
+        if (nc <= kTailCells) break;
+        k_mg_coarsen<<<block_count(nc), block_threads(nc), 0, st>>>(mg.lev[l], C, mg.omega, mg.nact + l + 1);
         ++g_launches;
     }
-    const int nd = mg.lev[mg.nlev].nx * mg.lev[mg.nlev].ny;
-    k_mg_dense<<<1, 32 * ((nd + 2) / 3), 0, st>>>(mg.lev[mg.nlev], mg.dense);
-    ++g_launches;
+    k_mg_tail<<<1, kTailThreads, 0, st>>>(mg, l);
+    g_launches += 3;
 }
 
 }  // namespace mpsg

@@ -230,7 +230,7 @@ extern "C" int mps_number_density_static(const mps_params* prm, int32_t n, const
     ce = cudaMemsetAsync(v.count, 0, sizeof(int32_t) * (c.nkeys + 1), st);
     if (ce != cudaSuccess) return na_fail(MPS_ERR_CUDA, cudaGetErrorString(ce));
     k_na_keys<<<G, T, 0, st>>>(c, n, d_pos, d_type, v);
-    launch_exclusive_scan(v.count, v.start, c.nkeys + 1, v.scan, st);
+    launch_exclusive_scan(v.count, v.start, c.nkeys + 1, v.scan, false, st);
     k_na_scatter<<<G, T, 0, st>>>(n, v);
     k_na_cellsort<<<(c.nkeys + T - 1) / T, T, 0, st>>>(c.nkeys, v);
     k_na_gather<<<G, T, 0, st>>>(n, d_pos, v);

@@ -25,20 +25,10 @@ __global__ void k_keys(Consts c, StateBuf s, int32_t* __restrict__ key, int32_t*
                        int32_t* __restrict__ count, DevStats* ds) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= c.n) return;
-    int32_t kk = c.nkeys;
-    if (s.type[k] != T_GHOST) {
-        const double x = s.x[k], y = s.y[k], z = c.planar ? 0.0 : s.z[k];
-        if (isfinite(x) && isfinite(y) && isfinite(z)) {
-            kk = cell_key(c, x, y, z);
-        } else {
-            // the reference has no defined behaviour here; the particle is
-            // taken out of the neighbour search and the step reports an error
-            s.type[k] = T_GHOST;
-            atomicOr(&ds->status, ST_NONFINITE);
-        }
-    }
-    key[k] = kk;
-    rank[k] = atomicAdd(count + kk, 1);
+    int8_t t = s.type[k];
+    const int8_t t0 = t;
+    count_cell(c, k, s.x[k], s.y[k], c.planar ? 0.0 : s.z[k], t, key, rank, count, ds);
+    if (t != t0) s.type[k] = t;
 }
 
 __global__ void k_scatter(int n, const int32_t* __restrict__ key, const int32_t* __restrict__ rank,
@@ -157,8 +147,8 @@ __global__ void k_scan_top(int32_t* sums, int nb) {
     }
 }
 
-__global__ void k_scan_apply(const int32_t* in, int n, const int32_t* __restrict__ sums,
-                             int32_t* out) {
+__global__ void k_scan_apply(int32_t* in, int n, const int32_t* __restrict__ sums, int32_t* out,
+                             bool clear) {
     __shared__ int sh[32];
     int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     int v[kScanItems];
@@ -174,7 +164,10 @@ __global__ void k_scan_apply(const int32_t* in, int n, const int32_t* __restrict
 #pragma unroll
     for (int t = 0; t < kScanItems; t++) {
         int i = base + t;
-        if (i < n) out[i] = pre;
+        if (i < n) {
+            if (clear) in[i] = 0;
+            out[i] = pre;
+        }
         pre += v[t];
     }
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == blockDim.x - 1) out[n] = pre;
@@ -182,7 +175,7 @@ __global__ void k_scan_apply(const int32_t* in, int n, const int32_t* __restrict
 
 // One block, tiles of four items per thread in turn.
 constexpr int kScanOne = 1024;
-__global__ void __launch_bounds__(kScanOne) k_scan_one(const int32_t* in, int n, int32_t* out) {
+__global__ void __launch_bounds__(kScanOne) k_scan_one(int32_t* in, int n, int32_t* out, bool clear) {
     __shared__ int sh[32];
     int carry = 0;
     for (int base = 0; base < n; base += 4 * kScanOne) {
@@ -197,7 +190,10 @@ __global__ void __launch_bounds__(kScanOne) k_scan_one(const int32_t* in, int n,
         int pre = carry + block_exclusive_scan(s, sh, &tot);
 #pragma unroll
         for (int t = 0; t < 4; t++) {
-            if (i0 + t < n) out[i0 + t] = pre;
+            if (i0 + t < n) {
+                if (clear) in[i0 + t] = 0;
+                out[i0 + t] = pre;
+            }
             pre += v[t];
         }
         carry += tot;
@@ -209,11 +205,11 @@ __global__ void __launch_bounds__(kScanOne) k_scan_one(const int32_t* in, int n,
 
 size_t scan_tmp_ints(int32_t n) { return (size_t)(n + kScanTile - 1) / kScanTile + 32; }
 
-void launch_exclusive_scan(const int32_t* in, int32_t* out, int32_t n, int32_t* tmp,
+void launch_exclusive_scan(int32_t* in, int32_t* out, int32_t n, int32_t* tmp, bool clear,
                            cudaStream_t st) {
     // up to four tiles one block is faster than three dependent launches (9 us)
     if (n <= 16 * kScanOne) {
-        k_scan_one<<<1, kScanOne, 0, st>>>(in, n, out);
+        k_scan_one<<<1, kScanOne, 0, st>>>(in, n, out, clear);
         ++g_launches;
         return;
     }
@@ -222,17 +218,19 @@ void launch_exclusive_scan(const int32_t* in, int32_t* out, int32_t n, int32_t* 
     ++g_launches;
     k_scan_top<<<1, 1024, 0, st>>>(tmp, nb);
     ++g_launches;
-    k_scan_apply<<<nb, kScanThreads, 0, st>>>(in, n, tmp, out);
+    k_scan_apply<<<nb, kScanThreads, 0, st>>>(in, n, tmp, out, clear);
     ++g_launches;
 }
 
 void launch_rebuild(const Consts& c, const StateBuf& in, const StateBuf& out, SortScratch& s,
-                    DevStats* ds, cudaStream_t st) {
+                    DevStats* ds, cudaStream_t st, bool counted) {
     const int T = block_threads(c.n), nb = block_count(c.n);
-    cudaMemsetAsync(s.cell_count, 0, sizeof(int32_t) * (c.nkeys + 1), st);
-    k_keys<<<nb, T, 0, st>>>(c, in, s.key, s.rank, s.cell_count, ds);
-    ++g_launches;
-    launch_exclusive_scan(s.cell_count, s.cell_start, c.nkeys + 1, s.scan_tmp, st);
+    if (!counted) {
+        k_keys<<<nb, T, 0, st>>>(c, in, s.key, s.rank, s.cell_count, ds);
+        ++g_launches;
+    }
+    // (the scan clears the counts for the next build)
+    launch_exclusive_scan(s.cell_count, s.cell_start, c.nkeys + 1, s.scan_tmp, true, st);
     k_scatter<<<nb, T, 0, st>>>(c.n, s.key, s.rank, s.cell_start, in.id, s.perm, s.pid);
     ++g_launches;
     k_gather<<<nb, T, 0, st>>>(c.n, c.nkeys, s.perm, s.pid, s.cell_start, s.key, s.skey, in, out, c.planar);

@@ -75,7 +75,8 @@ template <bool PLANAR, bool MIXED>
 __global__ void __launch_bounds__(kThreads) k_explicit(Consts c, StateBuf in, StateBuf out,
                                                        const int32_t* __restrict__ skey,
                                                        const int32_t* __restrict__ cs,
-                                                       DevStats* ds) {
+                                                       int32_t* __restrict__ nkey, int32_t* __restrict__ nrank,
+                                                       int32_t* __restrict__ ncount, DevStats* ds) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= c.n) return;
     int8_t t = in.type[k];
@@ -171,6 +172,7 @@ __global__ void __launch_bounds__(kThreads) k_explicit(Consts c, StateBuf in, St
         out.z[k] = z;
         out.vz[k] = vz;
     }
+    count_cell(c, k, x, y, PLANAR ? 0.0 : z, t, nkey, nrank, ncount, ds);  // for the next build
     out.type[k] = t;
     out.nd_last[k] = nd_last;
     out.p[k] = in.p[k];
@@ -237,7 +239,7 @@ __global__ void __launch_bounds__(kThreads) k_coll_write(Consts c, StateBuf s,
                                                          const int32_t* __restrict__ cs,
                                                          const int32_t* __restrict__ cnt_by_id,
                                                          const int32_t* __restrict__ base_by_id,
-                                                         CollPair* pairs, int32_t cap,
+                                                         CollPair* pairs, int32_t cap, CollWork cw,
                                                          DevStats* ds) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= c.n || s.type[k] != T_FLUID) return;
@@ -248,7 +250,18 @@ __global__ void __launch_bounds__(kThreads) k_coll_write(Consts c, StateBuf s,
         raise_status(ds, ST_CAPACITY);
         return;
     }
-    for_each_collision<PLANAR>(c, s, cs, skey[k], k, pairs + b);
+    const int m = for_each_collision<PLANAR>(c, s, cs, skey[k], k, pairs + b);
+    if (cw.serial) return;
+    // each pair with a fluid partner j: its index in j's short list
+    for (int t = b; t < b + m; t++) {
+        const CollPair q = pairs[t];
+        if (s.type[q.sj] != T_FLUID) continue;
+        const int p = atomicAdd(cw.jn + q.ij, 1);
+        if (p < kCollJList)
+            cw.jl[(size_t)q.ij * kCollJList + p] = t;
+        else
+            atomicOr(cw.ctl + 1, 1);
+    }
 }
 
 // One pair of the collision loop (the body of src/mps.cpp:222-247), with
@@ -320,35 +333,6 @@ __device__ __forceinline__ void coll_apply_pair(const Consts& c, const StateBuf&
     }
 }
 
-// The serial pass: every pair in order by one thread (verification mode, or
-// when a particle is the partner of more than kCollJList pairs).  Also
-// reports the candidate count.
-template <bool PLANAR>
-__global__ void k_coll_apply(Consts c, StateBuf s, const CollPair* __restrict__ pairs,
-                             const int32_t* __restrict__ total_p, int32_t cap, CollWork cw, DevStats* ds) {
-    int32_t total = *total_p;
-    ds->n_cand = total;
-    if (total > cap) total = cap;
-    if (!cw.serial && !cw.ctl[1]) return;  // the parallel pass applied them
-    const double inv_rho = ddiv(1.0, c.rho);
-    for (int32_t t = 0; t < total; t++) coll_apply_pair<PLANAR, true>(c, s, pairs[t], inv_rho);
-}
-
-// Per pair with a fluid partner j: its index in j's short list.
-__global__ void k_coll_jlists(StateBuf s, const CollPair* __restrict__ pairs, const int32_t* __restrict__ total_p,
-                              int32_t cap, CollWork cw) {
-    const int32_t total = min(*total_p, cap);
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-        const CollPair q = pairs[t];
-        if (s.type[q.sj] != T_FLUID) continue;
-        const int p = atomicAdd(cw.jn + q.ij, 1);
-        if (p < kCollJList)
-            cw.jl[(size_t)q.ij * kCollJList + p] = t;
-        else
-            atomicOr(cw.ctl + 1, 1);
-    }
-}
-
 __device__ __forceinline__ int ld_acquire_i32(const int32_t* p) {
     int v;
     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -367,8 +351,16 @@ __global__ void __launch_bounds__(kThreads) k_coll_wave(Consts c, StateBuf s, co
                                                         const int32_t* __restrict__ base_by_id, CollWork cw,
                                                         DevStats* ds) {
     const int32_t total = min(*total_p, cap);
-    if (total == 0 || cw.serial || *(volatile int32_t*)(cw.ctl + 1)) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) ds->n_cand = *total_p;
+    if (total == 0) return;
     const double inv_rho = ddiv(1.0, c.rho);
+    if (cw.serial || *(volatile int32_t*)(cw.ctl + 1)) {
+        // the serial pass: every pair in order by one thread (verification mode, or
+        // when a particle is the partner of more than kCollJList pairs)
+        if (blockIdx.x == 0 && threadIdx.x == 0)
+            for (int32_t t = 0; t < total; t++) coll_apply_pair<PLANAR, true>(c, s, pairs[t], inv_rho);
+        return;
+    }
     __shared__ int s_chunk;
     for (;;) {
         __syncthreads();
@@ -960,18 +952,18 @@ void launch_explicit(const Consts& c, const StateBuf& in, const StateBuf& out,
     int nb = block_count(c.n);
     if (c.planar) {
         if (mixed) {
-            k_explicit<true, true><<<nb, block_threads(c.n), 0, st>>>(c, in, out, sc.skey, sc.cell_start, ds);
+            k_explicit<true, true><<<nb, block_threads(c.n), 0, st>>>(c, in, out, sc.skey, sc.cell_start, sc.key, sc.rank, sc.cell_count, ds);
             ++g_launches;
         } else {
-            k_explicit<true, false><<<nb, block_threads(c.n), 0, st>>>(c, in, out, sc.skey, sc.cell_start, ds);
+            k_explicit<true, false><<<nb, block_threads(c.n), 0, st>>>(c, in, out, sc.skey, sc.cell_start, sc.key, sc.rank, sc.cell_count, ds);
             ++g_launches;
         }
     } else {
         if (mixed) {
-            k_explicit<false, true><<<nb, block_threads(c.n), 0, st>>>(c, in, out, sc.skey, sc.cell_start, ds);
+            k_explicit<false, true><<<nb, block_threads(c.n), 0, st>>>(c, in, out, sc.skey, sc.cell_start, sc.key, sc.rank, sc.cell_count, ds);
             ++g_launches;
         } else {
-            k_explicit<false, false><<<nb, block_threads(c.n), 0, st>>>(c, in, out, sc.skey, sc.cell_start, ds);
+            k_explicit<false, false><<<nb, block_threads(c.n), 0, st>>>(c, in, out, sc.skey, sc.cell_start, sc.key, sc.rank, sc.cell_count, ds);
             ++g_launches;
         }
     }
@@ -988,31 +980,18 @@ void launch_collision(const Consts& c, const StateBuf& s, const SortScratch& sc,
         k_coll_count<false><<<nb, block_threads(c.n), 0, st>>>(c, s, sc.skey, sc.cell_start, cand_cnt, cw);
         ++g_launches;
     }
-    launch_exclusive_scan(cand_cnt, cand_base, c.n, scan_tmp, st);
+    launch_exclusive_scan(cand_cnt, cand_base, c.n, scan_tmp, false, st);
     const int32_t* total = cand_base + c.n;
+    const int T = block_threads(c.n);
     if (c.planar) {
-        k_coll_write<true><<<nb, block_threads(c.n), 0, st>>>(c, s, sc.skey, sc.cell_start, cand_cnt,
-                                                    cand_base, pairs, pair_cap, ds);
+        k_coll_write<true><<<nb, T, 0, st>>>(c, s, sc.skey, sc.cell_start, cand_cnt, cand_base, pairs, pair_cap, cw, ds);
+        k_coll_wave<true><<<kCollBlocks, kThreads, 0, st>>>(c, s, pairs, total, pair_cap, cand_cnt, cand_base, cw, ds);
     } else {
-        k_coll_write<false><<<nb, block_threads(c.n), 0, st>>>(c, s, sc.skey, sc.cell_start, cand_cnt,
-                                                     cand_base, pairs, pair_cap, ds);
+        k_coll_write<false><<<nb, T, 0, st>>>(c, s, sc.skey, sc.cell_start, cand_cnt, cand_base, pairs, pair_cap, cw,
+                                              ds);
+        k_coll_wave<false><<<kCollBlocks, kThreads, 0, st>>>(c, s, pairs, total, pair_cap, cand_cnt, cand_base, cw, ds);
     }
-    ++g_launches;
-    if (!cw.serial) {
-        k_coll_jlists<<<kCollBlocks, kThreads, 0, st>>>(s, pairs, total, pair_cap, cw);
-        if (c.planar)
-            k_coll_wave<true><<<kCollBlocks, kThreads, 0, st>>>(c, s, pairs, total, pair_cap, cand_cnt,
-                                                                cand_base, cw, ds);
-        else
-            k_coll_wave<false><<<kCollBlocks, kThreads, 0, st>>>(c, s, pairs, total, pair_cap, cand_cnt,
-                                                                 cand_base, cw, ds);
-        g_launches += 2;
-    }
-    if (c.planar)
-        k_coll_apply<true><<<1, 1, 0, st>>>(c, s, pairs, total, pair_cap, cw, ds);
-    else
-        k_coll_apply<false><<<1, 1, 0, st>>>(c, s, pairs, total, pair_cap, cw, ds);
-    ++g_launches;
+    g_launches += 2;
 }
 
 template <bool PLANAR, bool BC>
