@@ -43,7 +43,7 @@ constexpr int kMaxBlocks = 160;   // blocks of an exchange: 5 slots per polling 
 constexpr int kPolls = kMaxBlocks / 32;
 constexpr int kWinSlices = 1024;  // slices of a window at most (16-bit indices reach 2048)
 constexpr int kListBytes = kWinSlices * 4;
-constexpr int kStateWords = 6;    // FP64 words of a resident row: diagonal, its inverse, x, r, two sums
+constexpr int kStateWords = 9;    // FP64 words of a resident row: diagonal, its inverse, x, r, four sums, z
 // Polls before an exchange gives up (~0.3 us each: ~2.4 s, far above any
 // legitimate wait).
 constexpr long long kSpinLimit64 = 1ll << 23;
@@ -107,6 +107,13 @@ __device__ __forceinline__ void st_remote64(const double* local, int rank, doubl
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
     asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(r), "d"(v) : "memory");
 }
+__device__ __forceinline__ double ld_remote64(const double* local, int rank) {
+    unsigned a = (unsigned)__cvta_generic_to_shared(local), r;
+    double v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(r) : "memory");
+    return v;
+}
 __device__ __forceinline__ void cluster_barrier64() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
@@ -149,6 +156,9 @@ __device__ __forceinline__ bool exchange(Exchange& ex, const double (&v)[M], boo
             double t = lane < ex.size ? slots[par][warp][lane] : 0.0;
 #pragma unroll
             for (int o = kCluster64 / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            // the same total in every lane: one that divided by a partial 0 would send
+            // the warp through the FP64 division (1.3 us)
+            t = __shfl_sync(0xffffffffu, t, 0);
             const double x = post((int)warp, t);
             if (lane == 0) {
                 s_tot[warp] = t;
@@ -370,8 +380,25 @@ __global__ void __launch_bounds__(BS, 1) k_cg64(Ppe A, Krylov kv, Cg64Args a, De
     uint16_t* ridx = reinterpret_cast<uint16_t*>(rval + (size_t)S * 32 * wq);
     const bool resident = !over && (size_t)kListBytes + (size_t)cnt * 256 + (size_t)S * 32 * (kStateWords * 8 + wq * 10) +
                                            (size_t)nwords * 8 <= (size_t)a.smem;
-    double *sd = state, *si = sd + S * 32, *sx = si + S * 32, *sr = sx + S * 32, *s_even = sr + S * 32,
-           *s_odd = s_even + S * 32;
+    double *sd = state, *si = sd + S * 32, *sx = si + S * 32, *sr = sx + S * 32, *s_sum = sr + S * 32,
+           *sz = s_sum + 4 * S * 32;
+    // A cluster whose blocks are all resident publishes z in its blocks' shared
+    // memory: the window reads the owner's copy, and the exchange's barrier has no
+    // global stores to wait for.  src = where a block's z array lies (its offset
+    // depends on the block's window), one word per block.
+    __shared__ int s_src[kCluster64];
+    bool zshared = false;
+    if constexpr (CL) {
+        const int mine = resident ? (int)(reinterpret_cast<unsigned char*>(sz) - smem) : -1;
+        if (warp == 0 && lane < ex.size) {
+            unsigned d = (unsigned)__cvta_generic_to_shared(&s_src[ex.rank]), r;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(d), "r"(lane));
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(r), "r"(mine) : "memory");
+        }
+        cluster_barrier64();
+        zshared = true;
+        for (int q = 0; q < ex.size; q++) zshared = zshared && s_src[q] >= 0;
+    }
     int own = 0;  // window index of this block's first row (its slices follow one another)
     if (!over) {
         own = slot_of(sl0) * 32;
@@ -398,12 +425,23 @@ __global__ void __launch_bounds__(BS, 1) k_cg64(Ppe A, Krylov kv, Cg64Args a, De
         }
         for (int k = tid; k < nwords; k += BS) {
             unsigned b = bits[k];
-            for (int pos = before[k]; b; b &= b - 1) wl[pos++] = k * 32 + __ffs(b) - 1;
+            for (int pos = before[k]; b; b &= b - 1, pos++) {
+                const int slice = k * 32 + __ffs(b) - 1;
+                if (CL && zshared) {  // owner and first byte of the slice's z there
+                    const int q = (int)(((int64_t)(slice + 1) * gridDim.x - 1) / a.nslices);
+                    const int first = (int)((int64_t)a.nslices * q / gridDim.x);
+                    wl[pos] = q << 20 | (s_src[q] + (slice - first) * 256);
+                } else {
+                    wl[pos] = slice;
+                }
+            }
         }
     }
     __syncthreads();  // bits and before are free: a streamed block's window may cover them
     if (!over)
         for (int k = tid; k < cnt * 32; k += BS) pwin[k] = 0.0;
+
+    const int parts = 4 * S <= kW ? 4 : 2;  // warps per slice of a resident block's products
 
     // ---- x = 0, r = b, z = D^-1 r (published, rows past n as 0)
     double acc[3] = {0.0, 0.0, over ? 1.0 : 0.0}, tot[3], aux[3];
@@ -416,7 +454,10 @@ __global__ void __launch_bounds__(BS, 1) k_cg64(Ppe A, Krylov kv, Cg64Args a, De
         }
         const double inv = d != 0.0 ? ddiv(1.0, d) : 1.0;
         const double z = inv * b;
-        __stcg(kv.z + i, z);
+        if (CL && zshared)
+            sz[l] = z;
+        else
+            __stcg(kv.z + i, z);
         kv.inv_diag[i] = inv;
         kv.x[i] = 0.0;
         kv.r[i] = b;
@@ -443,39 +484,43 @@ __global__ void __launch_bounds__(BS, 1) k_cg64(Ppe A, Krylov kv, Cg64Args a, De
         // ---- p = z + beta p on the window, q = A p and p.q on the own rows
         double pq[1] = {0.0}, t1[1], x1[1];
         if (!gather) {
-            for (int k = tid; k < cnt * 32; k += BS)
-                pwin[k] = fma(beta, pwin[k], __ldcg(kv.z + wl[k >> 5] * 32 + (k & 31)));
+            if (CL && zshared) {
+                for (int k = tid; k < cnt * 32; k += BS) {
+                    const int w = wl[k >> 5];
+                    const double* z = reinterpret_cast<const double*>(smem + (w & 0xfffff)) + (k & 31);
+                    pwin[k] = fma(beta, pwin[k], ld_remote64(z, w >> 20));
+                }
+            } else {
+                for (int k = tid; k < cnt * 32; k += BS)
+                    pwin[k] = fma(beta, pwin[k], __ldcg(kv.z + wl[k >> 5] * 32 + (k & 31)));
+            }
             __syncthreads();
             if (resident) {
-                // two warps per slice: the even and the odd entries of the
-                // groups of four (row_window's two sums)
-                for (int t = warp; t < 2 * S; t += kW) {
-                    const int s = t >> 1, half = t & 1;
+                // two or four warps per slice, each every second or fourth entry: a
+                // shorter chain of dependent multiply-adds (~120 cycles each), as long
+                // as every part has a warp of its own (22,000 rows, 5 slices per block:
+                // 8.4 us per iteration in halves, 8.8 in quarters; 6,000 rows: 8.3, 8.0)
+                for (int t = warp; t < parts * S; t += kW) {
+                    const int s = t / parts, part = t & (parts - 1);
                     const int w = __ldg(A.slice_w + sl0 + s), i = row_of(s);
                     const double* vp = rval + (size_t)s * wq * 32 + lane;
                     const uint16_t* ip = ridx + ((size_t)s * wq * 32 + lane * 4);
                     double sum = 0.0;
                     if (i < a.n) {
-                        const int main = w & ~3;
-                        int m = 0;
-#pragma unroll 2
-                        for (; m < main; m += 4) {
-                            const ushort2 q = half ? make_ushort2(ip[m * 32 + 1], ip[m * 32 + 3])
-                                                   : make_ushort2(ip[m * 32], ip[m * 32 + 2]);
-                            sum = fma(vp[(m + half) * 32], pwin[q.x], sum);
-                            sum = fma(vp[(m + half + 2) * 32], pwin[q.y], sum);
-                        }
-                        if (!half)
-                            for (; m < w; m++) sum = fma(vp[m * 32], pwin[ip[main * 32 + (m - main)]], sum);
+#pragma unroll 4
+                        for (int m = part; m < w; m += parts)
+                            sum = fma(vp[m * 32], pwin[ip[(m & ~3) * 32 + (m & 3)]], sum);
                     }
-                    (half ? s_odd : s_even)[s * 32 + lane] = sum;
+                    s_sum[(part * S + s) * 32 + lane] = sum;
                 }
                 __syncthreads();
                 for (int s = warp; s < S; s += kW) {
                     const int l = s * 32 + lane;
                     const double p = pwin[own + l];
-                    const double q = fma(sd[l], p, s_even[l] + s_odd[l]);
-                    s_even[l] = q;
+                    double o = s_sum[l] + s_sum[S * 32 + l];
+                    if (parts == 4) o += s_sum[2 * S * 32 + l] + s_sum[3 * S * 32 + l];
+                    const double q = fma(sd[l], p, o);
+                    s_sum[l] = q;
                     pq[0] = fma(p, q, pq[0]);
                 }
             } else {
@@ -520,11 +565,14 @@ __global__ void __launch_bounds__(BS, 1) k_cg64(Ppe A, Krylov kv, Cg64Args a, De
         if (!gather && resident) {
             for (int s = warp; s < S; s += kW) {
                 const int l = s * 32 + lane;
-                sx[l] = fma(alpha, pwin[own + l], sx[l]);
-                const double r = fma(-alpha, s_even[l], sr[l]);
-                sr[l] = r;
+                const double r = fma(-alpha, s_sum[l], sr[l]);
                 const double z = si[l] * r;
-                __stcg(kv.z + row_of(s), z);
+                if (CL && zshared)
+                    sz[l] = z;
+                else
+                    __stcg(kv.z + row_of(s), z);
+                sr[l] = r;
+                sx[l] = fma(alpha, pwin[own + l], sx[l]);
                 a2[0] = fma(r, r, a2[0]);
                 a2[1] = fma(r, z, a2[1]);
             }
@@ -574,9 +622,9 @@ constexpr int kSmem64 = 224 * 1024;
 // together); fewer: 512 (cheaper block barriers).
 constexpr int kWideSlices = 32;
 
-// Largest scene of the one-cluster form: per iteration 6.6 us up to 2,000 rows,
-// 7.6 at 3,400 and 9.0 at 4,500 (16 SMs issue all the FP64 work) against 8.2 to
-// 8.4 us for one block per SM at any of these sizes.
+// Largest scene of the one-cluster form: per iteration 5.2 to 5.5 us up to 2,000
+// rows and 6.5 at 3,400 (16 SMs issue all the FP64 work) against 7.5 to 8.2 us
+// for one block per SM at 4,500 to 11,000.
 constexpr int kClusterRows64 = 4000;
 
 template <int BS>
