@@ -215,8 +215,23 @@ __device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
     return F2{hi, lo - (hi - s)};
 }
 
-__device__ __forceinline__ F2 f2_shfl_down(F2 v, int o) {
-    return F2{__shfl_down_sync(0xffffffffu, v.hi, o), __shfl_down_sync(0xffffffffu, v.lo, o)};
+// Sums of three pairs over the warp, in lanes 0, 8 and 16: the first two steps
+// also deal the values to groups of lanes, so that six additions (of ~10
+// instructions and two shuffles) do the work of fifteen.  Each value is summed in
+// the order of a plain shuffle tree.
+__device__ __forceinline__ F2 f2_shfl_xor(F2 v, int o) {
+    return F2{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
+}
+__device__ __forceinline__ F2 f2_warp_add3(const F2 (&v)[3], int lane) {
+    const F2 zero = {0.f, 0.f};
+    const bool low = lane < 16, even = (lane & 8) == 0;
+    const F2 a = f2_add(low ? v[0] : v[2], f2_shfl_xor(low ? v[2] : v[0], 16));
+    const F2 b0 = f2_shfl_xor(low ? zero : v[1], 16);
+    const F2 b = low ? f2_add(v[1], b0) : zero;
+    F2 r = f2_add(even ? a : b, f2_shfl_xor(even ? b : a, 8));
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) r = f2_add(r, f2_shfl_xor(r, o));
+    return r;
 }
 
 // As publish_partials / sum_partials, on pairs: every warp reduces its lanes
@@ -224,36 +239,29 @@ __device__ __forceinline__ F2 f2_shfl_down(F2 v, int o) {
 // to the partials buffer; after the barrier every block sums the partials in
 // the same order (bitwise the same totals everywhere) and rounds each total
 // to FP32.
-template <int M, int BS>
-__device__ __forceinline__ const F2* publish_partials_f2(GridBar& gb, const F2 (&v)[M]) {
+template <int BS>
+__device__ __forceinline__ const F2* publish_partials_f2(GridBar& gb, const F2 (&v)[3]) {
     constexpr int kW = BS / 32;
-    static_assert(kW <= 32 && M <= 8, "one warp reduces the warps' pairs");
-    __shared__ F2 sh[M][kW];
+    static_assert(kW <= 32, "one warp reduces the warps' pairs");
+    __shared__ F2 sh[3][kW];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     F2* part = reinterpret_cast<F2*>(gb.partials + (size_t)gb.parity * gb.size * 8);
     gb.parity ^= 1;
-#pragma unroll
-    for (int m = 0; m < M; m++) {
-        F2 a = v[m];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a = f2_add(a, f2_shfl_down(a, o));
-        if (lane == 0) sh[m][warp] = a;
-    }
+    const F2 s = f2_warp_add3(v, lane);
+    if ((lane & 7) == 0 && lane < 24) sh[lane >> 3][warp] = s;
     __syncthreads();
     if (warp == 0) {
+        F2 w[3];
 #pragma unroll
-        for (int m = 0; m < M; m++) {
-            F2 a = lane < kW ? sh[m][lane] : F2{0.f, 0.f};
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) a = f2_add(a, f2_shfl_down(a, o));
-            if (lane == 0) part[gb.rank * 8 + m] = a;
-        }
+        for (int m = 0; m < 3; m++) w[m] = lane < kW ? sh[m][lane] : F2{0.f, 0.f};
+        const F2 t = f2_warp_add3(w, lane);
+        if ((lane & 7) == 0 && lane < 24) part[gb.rank * 8 + (lane >> 3)] = t;
     }
     return part;
 }
 
-template <int M>
-__device__ __forceinline__ void sum_partials_f2(const GridBar& gb, const F2* part, float (&tot)[M]) {
+__device__ __forceinline__ void sum_partials_f2(const GridBar& gb, const F2* part, float (&tot)[3]) {
+    constexpr int M = 3;
     __shared__ float s_tot[M];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp == 0) {
@@ -278,24 +286,19 @@ __device__ __forceinline__ void sum_partials_f2(const GridBar& gb, const F2* par
                 for (int m = 0; m < M; m++)
                     if (b0 + 32 * u < gb.size) a[m] = f2_add(a[m], F2{q[m][u].x, q[m][u].y});
         }
-#pragma unroll
-        for (int m = 0; m < M; m++) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) a[m] = f2_add(a[m], f2_shfl_down(a[m], o));
-            if (lane == 0) s_tot[m] = a[m].hi + a[m].lo;
-        }
+        const F2 t = f2_warp_add3(a, lane);
+        if ((lane & 7) == 0 && lane < 24) s_tot[lane >> 3] = t.hi + t.lo;
     }
     __syncthreads();
 #pragma unroll
     for (int m = 0; m < M; m++) tot[m] = s_tot[m];
 }
 
-template <int M, int BS>
-__device__ __forceinline__ bool reduce_sync_f2(GridBar& gb, const F2 (&v)[M], float (&tot)[M],
-                                               DevStats* ds) {
-    const F2* part = publish_partials_f2<M, BS>(gb, v);
+template <int BS>
+__device__ __forceinline__ bool reduce_sync_f2(GridBar& gb, const F2 (&v)[3], float (&tot)[3], DevStats* ds) {
+    const F2* part = publish_partials_f2<BS>(gb, v);
     if (!grid_sync(gb, ds)) return false;
-    sum_partials_f2<M>(gb, part, tot);
+    sum_partials_f2(gb, part, tot);
     return true;
 }
 
@@ -319,39 +322,33 @@ __device__ __forceinline__ void st_remote(const F2* local, int rank, F2 v) {
 // reduce_sync_f2 within a cluster: every block stores its M pairs into its
 // slot of every block, and after the barrier each block adds the slots in
 // rank order.  Two slot sets in turn, as with the partials in global memory.
-template <int M, int BS>
-__device__ __forceinline__ void cluster_reduce_f2(GridBar& gb, const F2 (&v)[M], float (&tot)[M]) {
+template <int BS>
+__device__ __forceinline__ void cluster_reduce_f2(GridBar& gb, const F2 (&v)[3], float (&tot)[3]) {
     constexpr int kW = BS / 32;
-    __shared__ F2 sh[M][kW];
-    __shared__ F2 slots[2][M][kClusterMax];
-    __shared__ float s_tot[M];
+    __shared__ F2 sh[3][kW];
+    __shared__ F2 slots[2][3][kClusterMax];
+    __shared__ float s_tot[3];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, par = gb.parity;
     gb.parity ^= 1;
-#pragma unroll
-    for (int m = 0; m < M; m++) {
-        F2 a = v[m];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a = f2_add(a, f2_shfl_down(a, o));
-        if (lane == 0) sh[m][warp] = a;
-    }
+    const F2 s = f2_warp_add3(v, lane);
+    if ((lane & 7) == 0 && lane < 24) sh[lane >> 3][warp] = s;
     __syncthreads();
-    if (warp < M) {
+    if (warp < 3) {
         F2 a = lane < kW ? sh[warp][lane] : F2{0.f, 0.f};
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a = f2_add(a, f2_shfl_down(a, o));
-        a = F2{__shfl_sync(0xffffffffu, a.hi, 0), __shfl_sync(0xffffffffu, a.lo, 0)};
+        for (int o = 16; o > 0; o >>= 1) a = f2_add(a, f2_shfl_xor(a, o));
         if (lane < gb.size) st_remote(&slots[par][warp][gb.rank], lane, a);
     }
     cluster_barrier();
-    if (warp < M) {
+    if (warp < 3) {
         F2 a = lane < gb.size ? slots[par][warp][lane] : F2{0.f, 0.f};
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a = f2_add(a, f2_shfl_down(a, o));
+        for (int o = kClusterMax / 2; o > 0; o >>= 1) a = f2_add(a, f2_shfl_xor(a, o));
         if (lane == 0) s_tot[warp] = a.hi + a.lo;
     }
     __syncthreads();
 #pragma unroll
-    for (int m = 0; m < M; m++) tot[m] = s_tot[m];
+    for (int m = 0; m < 3; m++) tot[m] = s_tot[m];
 }
 
 // The barrier and the sums of a solve's blocks: a grid's (CL false) or a cluster's.
@@ -374,10 +371,10 @@ __device__ __forceinline__ bool solve_reduce(GridBar& gb, const double (&v)[1], 
 template <bool CL, int BS>
 __device__ __forceinline__ bool solve_reduce_f2(GridBar& gb, const F2 (&v)[3], float (&tot)[3], DevStats* ds) {
     if constexpr (CL) {
-        cluster_reduce_f2<3, BS>(gb, v, tot);
+        cluster_reduce_f2<BS>(gb, v, tot);
         return true;
     } else {
-        return reduce_sync_f2<3, BS>(gb, v, tot, ds);
+        return reduce_sync_f2<BS>(gb, v, tot, ds);
     }
 }
 
@@ -1624,7 +1621,7 @@ __device__ __forceinline__ void solve_mixed(const Ppe& A, const MatFree& mf, con
             }
             const F2 v3[3] = {g, dl, rr};
             float t3[3];
-            if (!reduce_sync_f2<3, BS>(gb, v3, t3, ds)) return;
+            if (!reduce_sync_f2<BS>(gb, v3, t3, ds)) return;
             if (t3[2] < ithr || inner_total + k >= a.max_iter) break;
             const float gamma = t3[0], delta = t3[1];
             if (k == 0) {
