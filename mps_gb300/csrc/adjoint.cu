@@ -139,131 +139,143 @@ __global__ void k_pick(int m, const int32_t* __restrict__ sid, const double* __r
 }
 
 // ------------------------------------------------------------ adjoint kernels
-__device__ __forceinline__ double d2_of(const double* const* x, int i, int j) {
-    // exact FP64 squared distance in the forward's order, (dx^2 + dy^2) + dz^2
-    const double dx = dsub(x[0][j], x[0][i]), dy = dsub(x[1][j], x[1][i]),
-                 dz = dsub(x[2][j], x[2][i]);
-    return dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
+// The gather kernels walk a particle's list with kLanes lanes: their time is FP64
+// issue (a warp's FP64 instruction holds an SM quarter for 64 cycles) and the
+// latency of a serial walk, and a scene of a few thousand particles has fewer warps
+// than the chip has quarters with one lane each.  One division and one square root
+// per pair (on the integer pipe).  The reverse step's five gathers at 2,144
+// particles: 394 us with one lane, up to five FP64 divisions and the z terms of a
+// planar scene; 84 us so (243 us at 27,676 particles).
+constexpr int kLanes = 8;
+
+__device__ __forceinline__ double lane_sum(double v) {
+#pragma unroll
+    for (int o = kLanes / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
 }
 
-// move: a_bar = dt v_bar + dt^2 x_bar for particles the move displaced
-__global__ void k_adj_move(int n, double dt, int planar, const int8_t* __restrict__ type1,
-                           Arr3 xb, Arr3 vb, Arr3 ab) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const bool f = type1[i] == T_FLUID;
-    for (int d = 0; d < 3; d++)
-        ab.p[d][i] = (f && !(planar && d == 2)) ? dt * vb.p[d][i] + dt * dt * xb.p[d][i] : 0.0;
+// r = x_j - x_i and the exact FP64 squared distance in the forward's order; a planar
+// scene's z differences are zeros
+template <bool PLANAR>
+__device__ __forceinline__ double d2_r(const double* const* x, int j, const double (&xi)[3], double (&r)[3]) {
+    r[0] = dsub(x[0][j], xi[0]);
+    r[1] = dsub(x[1][j], xi[1]);
+    const double s = dadd(dmul(r[0], r[0]), dmul(r[1], r[1]));
+    if (PLANAR) return s;
+    r[2] = dsub(x[2][j], xi[2]);
+    return dadd(s, dmul(r[2], r[2]));
 }
 
-__global__ void k_adj_pplus(int n, const double* __restrict__ praw, double* __restrict__ pplus) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) pplus[i] = praw[i] < 0.0 ? 0.0 : praw[i];
-}
+__device__ __forceinline__ double clamp_p(double p) { return p < 0.0 ? 0.0 : p; }
 
-// setMinimumPressure replayed: value and the particle attaining it
-__global__ void k_adj_minp(int n, Consts c, TapeStep t, const double* __restrict__ pplus,
-                           double* __restrict__ phat, int32_t* __restrict__ amin) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (t.bc[i] == BC_IGNORED) {
-        phat[i] = 0.0;
-        amin[i] = -1;
-        return;
+// move: a_bar = dt v_bar + dt^2 x_bar for particles the move displaced;
+// setMinimumPressure replayed: value and the particle attaining it (the first of the
+// list on equal values); phat_bar_i = -Kg sum_j (a_bar_i . r_ij) w(d)/d^2
+template <bool PLANAR>
+__global__ void k_adj_own(int n, Consts c, TapeStep t, Arr3 xb, Arr3 vb, Arr3 ab, double* __restrict__ phat,
+                          int32_t* __restrict__ amin, double* __restrict__ phatbar) {
+    constexpr int D = PLANAR ? 2 : 3;
+    const int gid = blockIdx.x * blockDim.x + threadIdx.x, g = gid % kLanes;
+    const bool on = gid / kLanes < n;
+    const int i = on ? gid / kLanes : n - 1;
+    const bool f = t.type1[i] == T_FLUID, used = t.bc[i] != BC_IGNORED;
+    double a[3] = {0.0, 0.0, 0.0}, xi[3];
+    for (int d = 0; d < D; d++) {
+        xi[d] = t.st2[d][i];
+        if (f) a[d] = c.dt * vb.p[d][i] + c.dt * c.dt * xb.p[d][i];
     }
-    double mn = pplus[i];
-    int arg = i;
-    const int m = t.l2cnt[i];
-    for (int q = 0; q < m; q++) {
+    double mn = clamp_p(t.praw[i]), s = 0.0;
+    int arg = i, at = -1;
+    const int m = f || used ? t.l2cnt[i] : 0;
+    for (int q = g; q < m; q += kLanes) {
         const int j = t.l2id[(size_t)q * n + i];
         if (t.type1[j] == T_DUMMY) continue;
-        if (d2_of(t.st2, i, j) < c.t_p && mn > pplus[j]) {
-            mn = pplus[j];
+        double r[3];
+        const double d2 = d2_r<PLANAR>(t.st2, j, xi, r);
+        if (!(d2 < c.t_p)) continue;
+        const double pj = clamp_p(t.praw[j]);
+        if (mn > pj) {
+            mn = pj;
             arg = j;
+            at = q;
+        }
+        if (!f) continue;
+        const double inv = ddiv(1.0, dsqrt(d2));
+        double ar = a[0] * r[0] + a[1] * r[1];
+        if (!PLANAR) ar += a[2] * r[2];
+        s += ar * ((c.re_p * inv - 1.0) * (inv * inv));
+    }
+#pragma unroll
+    for (int o = kLanes / 2; o > 0; o >>= 1) {
+        const double om = __shfl_xor_sync(0xffffffffu, mn, o);
+        const int oarg = __shfl_xor_sync(0xffffffffu, arg, o), oat = __shfl_xor_sync(0xffffffffu, at, o);
+        if (mn > om || (mn == om && oat < at)) {
+            mn = om;
+            arg = oarg;
+            at = oat;
         }
     }
-    phat[i] = mn;
-    amin[i] = arg;
-}
-
-// phat_bar_i = -Kg sum_j (a_bar_i . r_ij) w(d)/d^2
-__global__ void k_adj_grad_local(int n, Consts c, TapeStep t, Arr3 ab, double* __restrict__ phatbar) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (t.type1[i] != T_FLUID) {
-        phatbar[i] = 0.0;
-        return;
-    }
-    const double Kg = -c.grad_scale / c.rho;
-    const double a0 = ab.p[0][i], a1 = ab.p[1][i], a2 = ab.p[2][i];
-    double s = 0.0;
-    const int m = t.l2cnt[i];
-    for (int q = 0; q < m; q++) {
-        const int j = t.l2id[(size_t)q * n + i];
-        if (t.type1[j] == T_DUMMY) continue;
-        const double d2 = d2_of(t.st2, i, j);
-        if (!(d2 < c.t_p)) continue;
-        const double d = sqrt(d2);
-        const double phi = (c.re_p / d - 1.0) / d2;
-        const double r0 = t.st2[0][j] - t.st2[0][i], r1 = t.st2[1][j] - t.st2[1][i],
-                     r2 = t.st2[2][j] - t.st2[2][i];
-        s += (a0 * r0 + a1 * r1 + a2 * r2) * phi;
-    }
-    phatbar[i] = -Kg * s;
+    s = lane_sum(s);
+    if (!on || g != 0) return;
+    for (int d = 0; d < 3; d++) ab.p[d][i] = a[d];
+    phat[i] = used ? mn : 0.0;
+    amin[i] = used ? arg : -1;
+    phatbar[i] = f ? c.grad_scale / c.rho * s : 0.0;
 }
 
 // x_bar += gradient-term adjoints (both sides of every pair); p+_bar from
 // the gradient sums of the neighbours and from the minima this particle set.
-__global__ void k_adj_grad_gather(int n, Consts c, TapeStep t, const double* __restrict__ pplus,
-                                  const double* __restrict__ phat, Arr3 ab,
+// a_bar is zero for every particle that the move left alone.  a_i's term for j
+// carries x_i through r_ij, a_j's term for i through r_ji = -r_ij: with
+// b = (p+_i - phat_j) a_j - (p+_j - phat_i) a_i the pair gives
+// Kg (phi b + phi'/d (r . b) r).
+template <bool PLANAR>
+__global__ void k_adj_grad_gather(int n, Consts c, TapeStep t, const double* __restrict__ phat, Arr3 ab,
                                   const double* __restrict__ phatbar, const int32_t* __restrict__ amin,
                                   Arr3 xb, double* __restrict__ pbar) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double accp = amin[i] == i ? phatbar[i] : 0.0;
-    if (t.type1[i] == T_GHOST) {
-        pbar[i] = accp;
-        return;
+    constexpr int D = PLANAR ? 2 : 3;
+    const int gid = blockIdx.x * blockDim.x + threadIdx.x, g = gid % kLanes;
+    const bool on = gid / kLanes < n;
+    const int i = on ? gid / kLanes : n - 1;
+    const int8_t ti = t.type1[i];
+    const bool fi = ti == T_FLUID, di = ti == T_DUMMY;
+    const double Kg = -c.grad_scale / c.rho, pi = clamp_p(t.praw[i]), phi_ = phat[i];
+    double ai[3], xi[3], gr[3] = {0.0, 0.0, 0.0}, accm = 0.0, accp = 0.0;
+    for (int d = 0; d < D; d++) {
+        ai[d] = ab.p[d][i];
+        xi[d] = t.st2[d][i];
     }
-    const double Kg = -c.grad_scale / c.rho;
-    const bool fi = t.type1[i] == T_FLUID, di = t.type1[i] == T_DUMMY;
-    const double ai0 = ab.p[0][i], ai1 = ab.p[1][i], ai2 = ab.p[2][i];
-    double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-    const int m = t.l2cnt[i];
-    for (int q = 0; q < m; q++) {
+    const int m = ti == T_GHOST ? 0 : t.l2cnt[i];
+    for (int q = g; q < m; q += kLanes) {
         const int j = t.l2id[(size_t)q * n + i];
-        const double d2 = d2_of(t.st2, i, j);
+        double r[3];
+        const double d2 = d2_r<PLANAR>(t.st2, j, xi, r);
         if (!(d2 < c.t_p)) continue;
-        if (amin[j] == i) accp += phatbar[j];
-        const bool fj = t.type1[j] == T_FLUID, dj = t.type1[j] == T_DUMMY;
-        const double d = sqrt(d2);
-        const double phi = (c.re_p / d - 1.0) / d2;
-        const double dphi_over_d = (-3.0 * c.re_p / (d2 * d2) + 2.0 / (d2 * d)) / d;
-        const double r0 = t.st2[0][j] - t.st2[0][i], r1 = t.st2[1][j] - t.st2[1][i],
-                     r2 = t.st2[2][j] - t.st2[2][i];
-        if (fi && !dj) {  // a_i's term for j: x_i enters through r_ij = x_j - x_i
-            const double qv = pplus[j] - phat[i];
-            const double rv = r0 * ai0 + r1 * ai1 + r2 * ai2;
-            const double s = Kg * qv;
-            g0 -= s * (phi * ai0 + dphi_over_d * rv * r0);
-            g1 -= s * (phi * ai1 + dphi_over_d * rv * r1);
-            g2 -= s * (phi * ai2 + dphi_over_d * rv * r2);
+        if (amin[j] == i) accm += phatbar[j];
+        const int8_t tj = t.type1[j];
+        const bool own = fi && tj != T_DUMMY, other = tj == T_FLUID && !di;
+        if (!own && !other) continue;
+        const double inv = ddiv(1.0, dsqrt(d2)), inv2 = inv * inv, rei = c.re_p * inv;
+        const double phi = (rei - 1.0) * inv2;
+        const double si = own ? clamp_p(t.praw[j]) - phi_ : 0.0, sj = other ? pi - phat[j] : 0.0;
+        double b[3], rb = 0.0, ra = 0.0;
+        for (int d = 0; d < D; d++) {
+            const double aj = ab.p[d][j];
+            b[d] = sj * aj - si * ai[d];
+            rb += r[d] * b[d];
+            ra += r[d] * aj;
         }
-        if (fj && !di) {  // a_j's term for i: r_ji = -r_ij, and p+_i enters through q_ji
-            const double aj0 = ab.p[0][j], aj1 = ab.p[1][j], aj2 = ab.p[2][j];
-            const double qv = pplus[i] - phat[j];
-            const double rv = r0 * aj0 + r1 * aj1 + r2 * aj2;
-            const double s = Kg * qv;
-            g0 += s * (phi * aj0 + dphi_over_d * rv * r0);
-            g1 += s * (phi * aj1 + dphi_over_d * rv * r1);
-            g2 += s * (phi * aj2 + dphi_over_d * rv * r2);
-            accp -= Kg * rv * phi;
-        }
+        const double h = (2.0 - 3.0 * rei) * (inv2 * inv2) * rb;
+        for (int d = 0; d < D; d++) gr[d] += phi * b[d] + h * r[d];
+        if (other) accp += ra * phi;
     }
-    xb.p[0][i] += g0;
-    xb.p[1][i] += g1;
-    xb.p[2][i] += g2;
-    pbar[i] = accp;
+    for (int d = 0; d < D; d++) gr[d] = lane_sum(gr[d]);
+    accp = lane_sum(accp);
+    accm = lane_sum(accm);
+    if (!on || g != 0) return;
+    pbar[i] = (amin[i] == i ? phatbar[i] : 0.0) + accm - Kg * accp;
+    if (ti == T_GHOST) return;
+    for (int d = 0; d < D; d++) xb.p[d][i] += Kg * gr[d];
 }
 
 __global__ void k_adj_sensor(int m, const int32_t* __restrict__ sid, const double* __restrict__ ds_,
@@ -274,66 +286,97 @@ __global__ void k_adj_sensor(int m, const int32_t* __restrict__ sid, const doubl
 
 // The PPE of this step in id order (rows = particle ids, SELL-32 like the
 // engine's), right-hand side = the clamp-masked pressure adjoint.
-__global__ void k_adj_assemble(int n, Consts c, TapeStep t, const double* __restrict__ pbar,
-                               Ppe A) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+template <bool PLANAR>
+__global__ void __launch_bounds__(32 * kLanes) k_adj_assemble(int n, Consts c, TapeStep t,
+                                                              const double* __restrict__ pbar, Ppe A) {
+    __shared__ int s_w;
+    if (threadIdx.x == 0) s_w = 0;
+    __syncthreads();
+    // one block per slice of 32 rows; a row's entries keep the order of its list
+    const int lane = threadIdx.x & 31, g = threadIdx.x % kLanes, row = threadIdx.x / kLanes;
+    const int i = blockIdx.x * 32 + row;
+    const size_t sbase = (size_t)blockIdx.x * c.K * 32 + row;
+    const bool inner = i < n && t.bc[i] == BC_INNER;
     int off = 0;
-    if (i < n) {
-        double diag = 0.0;
-        const bool inner = t.bc[i] == BC_INNER;
-        if (inner) {
-            const size_t sbase = (size_t)(i >> 5) * c.K * 32 + (i & 31);
-            const int m = t.l2cnt[i];
-            for (int q = 0; q < m; q++) {
-                const int j = t.l2id[(size_t)q * n + i];
-                const int8_t bj = t.bc[j];
-                if (bj == BC_IGNORED) continue;
-                const double d2 = d2_of(t.st2, i, j);
-                if (!(d2 < c.t_p)) continue;
-                const double a = ddiv(dmul(c.mat_c, weight(dsqrt(d2), c.re_p)), c.rho);
+    double diag = 0.0, xi[3];
+    if (inner)
+        for (int d = 0; d < (PLANAR ? 2 : 3); d++) xi[d] = t.st2[d][i];
+    const int m = inner ? t.l2cnt[i] : 0;
+    for (int q0 = 0; __any_sync(0xffffffffu, q0 < m); q0 += kLanes) {
+        const int q = q0 + g;
+        bool entry = false;
+        int j = 0;
+        double a = 0.0;
+        if (q < m) {
+            j = t.l2id[(size_t)q * n + i];
+            const int8_t bj = t.bc[j];
+            double r[3], d2;
+            if (bj != BC_IGNORED && (d2 = d2_r<PLANAR>(t.st2, j, xi, r)) < c.t_p) {
+                a = ddiv(dmul(c.mat_c, weight(dsqrt(d2), c.re_p)), c.rho);
                 diag = dadd(diag, a);
-                if (bj == BC_INNER && off < c.K) {
-                    A.col[sbase + (size_t)off * 32] = j;
-                    A.val[sbase + (size_t)off * 32] = -a;
-                    off++;
-                }
+                entry = bj == BC_INNER;
             }
-            if (c.qc_on) diag = dadd(diag, c.qc_term);
-            if (!t.dir[i]) diag = dmul(diag, 2.0);
         }
-        A.diag[i] = diag;
-        A.offcnt[i] = off;
-        A.src[i] = (inner && t.praw[i] > 0.0) ? pbar[i] : 0.0;
-    }
-    const int w = __reduce_max_sync(0xffffffffu, off);
-    if (i < n) {
-        const size_t sbase = (size_t)(i >> 5) * c.K * 32 + (i & 31);
-        for (int m = off; m < w; m++) {
-            A.col[sbase + (size_t)m * 32] = i;
-            A.val[sbase + (size_t)m * 32] = 0.0;
+        const unsigned mine = __ballot_sync(0xffffffffu, entry) >> (lane - g) & ((1u << kLanes) - 1u);
+        const int at = off + __popc(mine & ((1u << g) - 1u));
+        if (entry && at < c.K) {
+            A.col[sbase + (size_t)at * 32] = j;
+            A.val[sbase + (size_t)at * 32] = -a;
         }
+        off = min(off + __popc(mine), c.K);
     }
-    if ((threadIdx.x & 31) == 0 && (i >> 5) < (n + 31) / 32) A.slice_w[i >> 5] = w;
+    diag = lane_sum(diag);
+    if (g == 0) atomicMax(&s_w, off);
+    __syncthreads();
+    const int w = s_w;
+    if (threadIdx.x == 0) A.slice_w[blockIdx.x] = w;
+    if (i >= n) return;
+    for (int q = off + g; q < w; q += kLanes) {
+        A.col[sbase + (size_t)q * 32] = i;
+        A.val[sbase + (size_t)q * 32] = 0.0;
+    }
+    if (g != 0) return;
+    if (inner) {
+        if (c.qc_on) diag = dadd(diag, c.qc_term);
+        if (!t.dir[i]) diag = dmul(diag, 2.0);
+    }
+    A.diag[i] = diag;
+    A.offcnt[i] = off;
+    A.src[i] = (inner && t.praw[i] > 0.0) ? pbar[i] : 0.0;
 }
 
-// x_bar from lambda: source term and matrix entries, both sides of a pair.
+// x_bar from lambda: source term and matrix entries, both sides of a pair.  Also
+// the state at the collision pass's start, and zeros for what that pass adds to x_bar.
+template <bool PLANAR>
 __global__ void k_adj_ppe_gather(int n, Consts c, TapeStep t, const double* __restrict__ lam,
-                                 Arr3 xb) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || t.type1[i] == T_GHOST) return;
+                                 Arr3 xb, Arr6 cur, Arr3 xextra) {
+    constexpr int D = PLANAR ? 2 : 3;
+    const int gid = blockIdx.x * blockDim.x + threadIdx.x, g = gid % kLanes;
+    const bool on = gid / kLanes < n;
+    const int i = on ? gid / kLanes : n - 1;
+#pragma unroll
+    for (int d = 0; d < 6; d++)
+        if (on && g == d) {
+            cur.p[d][i] = t.st1[d][i];
+            if (d < 3) xextra.p[d][i] = 0.0;
+        }
+    const bool ghost = t.type1[i] == T_GHOST;
     const double cm = c.mat_c / c.rho, ks = c.src_g1 / c.n0_p;
     const int8_t bi = t.bc[i];
     const bool ii = bi == BC_INNER;
     const double li = ii ? lam[i] : 0.0, pi = t.praw[i];
     const double si = (ii && !t.dir[i]) ? 2.0 : 1.0;
-    double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-    const int m = t.l2cnt[i];
-    for (int q = 0; q < m; q++) {
+    double xi[3], gr[3] = {0.0, 0.0, 0.0};
+    for (int d = 0; d < D; d++) xi[d] = t.st2[d][i];
+    const int m = ghost ? 0 : t.l2cnt[i];
+    for (int q = g; q < m; q += kLanes) {
         const int j = t.l2id[(size_t)q * n + i];
-        const double d2 = d2_of(t.st2, i, j);
-        if (!(d2 < c.t_p)) continue;
         const int8_t bj = t.bc[j];
         const bool jj = bj == BC_INNER;
+        if (!ii && !jj) continue;
+        double r[3];
+        const double d2 = d2_r<PLANAR>(t.st2, j, xi, r);
+        if (!(d2 < c.t_p)) continue;
         double W = 0.0;
         if (ii) {
             W += li * ks;
@@ -348,33 +391,19 @@ __global__ void k_adj_ppe_gather(int n, Consts c, TapeStep t, const double* __re
             if (ii) W += lj * pi * cm;
         }
         if (W == 0.0) continue;
-        const double d = sqrt(d2);
-        const double coef = W * (-c.re_p / d2) / d;  // W w'(d) / d
-        g0 -= coef * (t.st2[0][j] - t.st2[0][i]);
-        g1 -= coef * (t.st2[1][j] - t.st2[1][i]);
-        g2 -= coef * (t.st2[2][j] - t.st2[2][i]);
+        const double inv = ddiv(1.0, dsqrt(d2));
+        const double coef = W * c.re_p * (inv * inv * inv);  // -W w'(d) / d
+        for (int d = 0; d < D; d++) gr[d] += coef * r[d];
     }
-    xb.p[0][i] += g0;
-    xb.p[1][i] += g1;
-    xb.p[2][i] += g2;
-}
-
-__global__ void k_copy6(int n, Arr6 src, Arr6 dst) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    for (int d = 0; d < 6; d++) dst.p[d][i] = src.p[d][i];
+    for (int d = 0; d < D; d++) gr[d] = lane_sum(gr[d]);
+    if (!on || g != 0 || ghost) return;
+    for (int d = 0; d < D; d++) xb.p[d][i] += gr[d];
 }
 
 __global__ void k_zero3(int n, Arr3 a) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n)
         for (int d = 0; d < 3; d++) a.p[d][i] = 0.0;
-}
-
-__global__ void k_add3(int n, Arr3 src, Arr3 dst) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n)
-        for (int d = 0; d < 3; d++) dst.p[d][i] += src.p[d][i];
 }
 
 // MPS::collision replayed on a copy of the pre-collision state (cur), then
@@ -481,26 +510,44 @@ __global__ void k_adj_collision(int n, Consts c, TapeStep t, Arr6 cur, double* _
     }
 }
 
-// explicit part, per particle: total velocity adjoint vt and a_bar = dt vt
+__device__ __forceinline__ double warp_total(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// what the collision pass added to x_bar, then the explicit part per particle: total
+// velocity adjoint vt and a_bar = dt vt; gpart: a_bar's sums over 32 particles (one
+// block summing all of a_bar is FP64 issue of one SM: 36 us at 27,676 particles)
 __global__ void k_adj_explicit_local(int n, double dt, int planar, const int8_t* __restrict__ type0,
-                                     Arr3 xb, Arr3 vb, Arr3 vt, Arr3 ab) {
+                                     Arr3 xextra, Arr3 xb, Arr3 vb, Arr3 vt, Arr3 ab,
+                                     double* __restrict__ gpart) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const bool f = type0[i] == T_FLUID;
+    const bool on = i < n, f = on && type0[i] == T_FLUID;
+#pragma unroll
     for (int d = 0; d < 3; d++) {
         const bool moves = f && !(planar && d == 2);
-        const double v = moves ? vb.p[d][i] + dt * xb.p[d][i] : vb.p[d][i];
-        vt.p[d][i] = v;
-        ab.p[d][i] = moves ? dt * v : 0.0;
+        double a = 0.0;
+        if (on) {
+            const double x = xb.p[d][i] + xextra.p[d][i];
+            const double v = moves ? vb.p[d][i] + dt * x : vb.p[d][i];
+            a = moves ? dt * v : 0.0;
+            xb.p[d][i] = x;
+            vt.p[d][i] = v;
+            ab.p[d][i] = a;
+        }
+        const double s = warp_total(a);
+        if (on && (i & 31) == 0) gpart[(size_t)3 * (i >> 5) + d] = s;
     }
 }
 
 // g_bar += sum of a_bar over all particles (fixed order: deterministic)
-__global__ void k_adj_gsum(int n, Arr3 ab, double* __restrict__ gbar) {
+__global__ void k_adj_gsum(int m, const double* __restrict__ gpart, double* __restrict__ gbar) {
     __shared__ double sh[3][1024];
     double s[3] = {0.0, 0.0, 0.0};
-    for (int i = threadIdx.x; i < n; i += blockDim.x)
-        for (int d = 0; d < 3; d++) s[d] += ab.p[d][i];
+    for (int i = threadIdx.x; i < m; i += blockDim.x)
+#pragma unroll
+        for (int d = 0; d < 3; d++) s[d] += gpart[(size_t)3 * i + d];
     for (int d = 0; d < 3; d++) sh[d][threadIdx.x] = s[d];
     __syncthreads();
     for (int w = blockDim.x / 2; w > 0; w >>= 1) {
@@ -513,44 +560,48 @@ __global__ void k_adj_gsum(int n, Arr3 ab, double* __restrict__ gbar) {
 }
 
 // explicit part, gathered over the step-start neighbour list: viscosity
-// velocity adjoints and weight (position) adjoints, both sides of a pair.
+// velocity adjoints and weight (position) adjoints, both sides of a pair
+// (a_bar is zero for what is not fluid).
+template <bool PLANAR>
 __global__ void k_adj_explicit_gather(int n, Consts c, TapeStep t, Arr3 ab, Arr3 vt, Arr3 xb,
                                       Arr3 vb) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double va[3] = {vt.p[0][i], vt.p[1][i], vt.p[2][i]};
-    if (t.type0[i] == T_GHOST) {
-        for (int d = 0; d < 3; d++) vb.p[d][i] = va[d];
-        return;
+    constexpr int D = PLANAR ? 2 : 3;
+    const int gid = blockIdx.x * blockDim.x + threadIdx.x, g = gid % kLanes;
+    const bool on = gid / kLanes < n;
+    const int i = on ? gid / kLanes : n - 1;
+    const int8_t ti = t.type0[i];
+    const bool fi = ti == T_FLUID, ghost = ti == T_GHOST;
+    double ai[3], xi[3], ui[3], va[3] = {0.0, 0.0, 0.0}, gr[3] = {0.0, 0.0, 0.0};
+    for (int d = 0; d < D; d++) {
+        ai[d] = ab.p[d][i];
+        xi[d] = t.st0[d][i];
+        ui[d] = t.st0[3 + d][i];
     }
-    const bool fi = t.type0[i] == T_FLUID;
-    const double V = c.visc_a;
-    const double ai[3] = {ab.p[0][i], ab.p[1][i], ab.p[2][i]};
-    double g[3] = {0.0, 0.0, 0.0};
-    const int m = t.l0cnt[i];
-    for (int q = 0; q < m; q++) {
+    const int m = ghost ? 0 : t.l0cnt[i];
+    for (int q = g; q < m; q += kLanes) {
         const int j = t.l0id[(size_t)q * n + i];
-        const double d2 = d2_of(t.st0, i, j);
+        if (!fi && t.type0[j] != T_FLUID) continue;
+        double r[3];
+        const double d2 = d2_r<PLANAR>(t.st0, j, xi, r);
         if (!(d2 < c.t_v)) continue;
-        const bool fj = t.type0[j] == T_FLUID;
-        if (!fi && !fj) continue;
-        const double d = sqrt(d2);
-        const double w = c.re_v / d - 1.0;
+        const double inv = ddiv(1.0, dsqrt(d2)), w = c.re_v * inv - 1.0;
         double W = 0.0;
-        for (int dd = 0; dd < 3; dd++) {
-            const double aj = fj ? ab.p[dd][j] : 0.0;
-            const double du = t.st0[3 + dd][j] - t.st0[3 + dd][i];
-            va[dd] += V * w * (aj - (fi ? ai[dd] : 0.0));
-            if (fi) W += V * ai[dd] * du;
-            if (fj) W -= V * aj * du;
+        for (int d = 0; d < D; d++) {
+            const double da = ab.p[d][j] - ai[d];
+            va[d] += w * da;
+            W += da * (t.st0[3 + d][j] - ui[d]);
         }
-        const double coef = W * (-c.re_v / d2) / d;
-        for (int dd = 0; dd < 3; dd++) g[dd] -= coef * (t.st0[dd][j] - t.st0[dd][i]);
+        const double coef = W * (inv * inv * inv);
+        for (int d = 0; d < D; d++) gr[d] -= coef * r[d];
     }
-    for (int d = 0; d < 3; d++) {
-        vb.p[d][i] = va[d];
-        xb.p[d][i] += g[d];
+    for (int d = 0; d < D; d++) {
+        va[d] = lane_sum(va[d]);
+        gr[d] = lane_sum(gr[d]);
     }
+    if (!on || g != 0) return;
+    for (int d = 0; d < 3; d++) vb.p[d][i] = vt.p[d][i] + (d < D ? c.visc_a * va[d] : 0.0);
+    if (ghost) return;
+    for (int d = 0; d < D; d++) xb.p[d][i] += c.visc_a * c.re_v * gr[d];
 }
 
 __global__ void k_interleave3(int n, Arr3 a, double* __restrict__ out) {
@@ -585,7 +636,7 @@ struct mps_trajectory {
     std::vector<TapeStep> tape;
     // adjoint work arrays (id order)
     double *xb[3]{}, *vb[3]{}, *ab[3]{}, *vt[3]{}, *xextra[3]{}, *cur[6]{};
-    double *pplus = nullptr, *phat = nullptr, *phatbar = nullptr, *pbar = nullptr;
+    double *gpart = nullptr, *phat = nullptr, *phatbar = nullptr, *pbar = nullptr;
     int32_t* amin = nullptr;
     double* rec = nullptr;
     double* gbar = nullptr;
@@ -697,37 +748,43 @@ int record_sensors(mps_trajectory* t, int step) {
     return MPS_OK;
 }
 
-// One reverse step on tape record T (the step's forward has just been taped).
-int reverse_step(mps_trajectory* t, const TapeStep& T, int step) {
+template <bool PLANAR>
+void launch_reverse(mps_trajectory* t, const TapeStep& T, int step) {
     mps_engine* e = t->e;
     const Consts& c = e->c;
-    const int n = t->n, G = block_count(n);
+    const int n = t->n, G = block_count(n), BT = block_threads(n);
+    constexpr int W = 32 * kLanes;
+    const int GL = (n + 31) / 32;  // blocks of the kernels with kLanes lanes per particle
     cudaStream_t st = e->st;
     Arr3 xb = a3(t->xb), vb = a3(t->vb), ab = a3(t->ab), vt = a3(t->vt), xx = a3(t->xextra);
     // move and pressure gradient
-    k_adj_move<<<G, block_threads(n), 0, st>>>(n, c.dt, c.planar, T.type1, xb, vb, ab);
-    k_adj_pplus<<<G, block_threads(n), 0, st>>>(n, T.praw, t->pplus);
-    k_adj_minp<<<G, block_threads(n), 0, st>>>(n, c, T, t->pplus, t->phat, t->amin);
-    k_adj_grad_local<<<G, block_threads(n), 0, st>>>(n, c, T, ab, t->phatbar);
-    k_adj_grad_gather<<<G, block_threads(n), 0, st>>>(n, c, T, t->pplus, t->phat, ab, t->phatbar, t->amin, xb,
-                                        t->pbar);
+    k_adj_own<PLANAR><<<GL, W, 0, st>>>(n, c, T, xb, vb, ab, t->phat, t->amin, t->phatbar);
+    k_adj_grad_gather<PLANAR><<<GL, W, 0, st>>>(n, c, T, t->phat, ab, t->phatbar, t->amin, xb, t->pbar);
     if (t->nsens)
         k_adj_sensor<<<block_count(t->nsens), block_threads(t->nsens), 0, st>>>(t->nsens, t->sensor,
                                                     t->sens_bar + (size_t)step * t->nsens, t->pbar);
     // transpose Poisson solve (A is symmetric): A lambda = masked p_bar
-    k_adj_assemble<<<G, block_threads(n), 0, st>>>(n, c, T, t->pbar, e->A);
-    TCU(cudaMemsetAsync(e->ds, 0, sizeof(DevStats), st));
+    k_adj_assemble<PLANAR><<<GL, W, 0, st>>>(n, c, T, t->pbar, e->A);
     launch_solve_fp64(c, e->A, e->kv, 1e-14, 4 * (int64_t)n + 100, e->ds, st);
-    k_adj_ppe_gather<<<G, block_threads(n), 0, st>>>(n, c, T, e->kv.x, xb);
+    k_adj_ppe_gather<PLANAR><<<GL, W, 0, st>>>(n, c, T, e->kv.x, xb, arr6(t->cur), xx);
     // collision pass
-    k_copy6<<<G, block_threads(n), 0, st>>>(n, arr6(T.st1), arr6(t->cur));
-    k_zero3<<<G, block_threads(n), 0, st>>>(n, xx);
     k_adj_collision<<<1, 1, 0, st>>>(n, c, T, arr6(t->cur), t->rec, xb, vb, xx);
-    k_add3<<<G, block_threads(n), 0, st>>>(n, xx, xb);
     // explicit part
-    k_adj_explicit_local<<<G, block_threads(n), 0, st>>>(n, c.dt, c.planar, T.type0, xb, vb, vt, ab);
-    k_adj_gsum<<<1, 1024, 0, st>>>(n, ab, t->gbar);
-    k_adj_explicit_gather<<<G, block_threads(n), 0, st>>>(n, c, T, ab, vt, xb, vb);
+    k_adj_explicit_local<<<G, BT, 0, st>>>(n, c.dt, c.planar, T.type0, xx, xb, vb, vt, ab, t->gpart);
+    k_adj_gsum<<<1, 1024, 0, st>>>((n + 31) / 32, t->gpart, t->gbar);
+    k_adj_explicit_gather<PLANAR><<<GL, W, 0, st>>>(n, c, T, ab, vt, xb, vb);
+}
+
+// One reverse step on tape record T (the step's forward has just been taped).
+int reverse_step(mps_trajectory* t, const TapeStep& T, int step) {
+    mps_engine* e = t->e;
+    const Consts& c = e->c;
+    cudaStream_t st = e->st;
+    TCU(cudaMemsetAsync(e->ds, 0, sizeof(DevStats), st));
+    if (c.planar)
+        launch_reverse<true>(t, T, step);
+    else
+        launch_reverse<false>(t, T, step);
     TCU(cudaMemcpyAsync(e->hs, e->ds, sizeof(DevStats), cudaMemcpyDeviceToHost, st));
     TCU(cudaStreamSynchronize(st));
     TCU(cudaGetLastError());
@@ -792,9 +849,9 @@ int mps_trajectory_create(mps_engine* e, int32_t n_steps, int32_t checkpoint_eve
         if (t->alloc(&t->xb[d], n) || t->alloc(&t->vb[d], n) || t->alloc(&t->ab[d], n) ||
             t->alloc(&t->vt[d], n) || t->alloc(&t->xextra[d], n))
             return bail("adjoint");
-    if (t->alloc(&t->pplus, n) || t->alloc(&t->phat, n) || t->alloc(&t->phatbar, n) ||
+    if (t->alloc(&t->phat, n) || t->alloc(&t->phatbar, n) ||
         t->alloc(&t->pbar, n) || t->alloc(&t->amin, n) || t->alloc(&t->rec, (size_t)pcap * 13) ||
-        t->alloc(&t->gbar, 4))
+        t->alloc(&t->gbar, 4) || t->alloc(&t->gpart, (n + 31) / 32 * 3))
         return bail("adjoint");
     if (cudaMallocHost(&t->hstage, sizeof(double) * 3 * n) != cudaSuccess) {
         t->hstage = nullptr;
