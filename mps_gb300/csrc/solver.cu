@@ -2181,11 +2181,12 @@ SolveArgs make_args(const Consts& c, double tol, int64_t max_iter) {
 }  // namespace
 
 namespace {
-// Largest scene of the one-cluster solve.  Its 16 SMs take, per inner
-// iteration, 18 us at 2,000 rows, 22 at 11,000 and 31 at 21,000 against 24, 28
-// and 31 for the grid of 152 blocks with its barriers: the line lies where the
-// operator pass on 16 SMs has eaten up what the cluster barriers save.
-constexpr int kClusterRows = 24000;
+// Largest scene of the one-cluster solve.  Its 16 SMs take, per inner iteration,
+// 15.0 us at 2,162 rows, 17.5 at 4,400, 16.7 at 7,456, 20.4 at 11,312 and 27.6 at
+// 21,424, against 17.0, 18.4, 16.9, 17.9 and 20.1 for the grid of 152 blocks: the
+// line lies where the operator pass on 16 SMs has eaten up what the cluster's
+// barriers save.
+constexpr int kClusterRows = 8000;
 // Dynamic shared memory of the overlapped solve's blocks (the split cycle's
 // levels, patches and operator data), and the part of it that the levels may
 // take: 136 KB hold all levels of a tank of 11,000 cells.
