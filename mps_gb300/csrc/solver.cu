@@ -432,6 +432,25 @@ __device__ __forceinline__ double spmv64_row(const Ppe& A, int K, int sl, int la
 // entries no longer shifts the row sum (the operator's smooth modes).
 // Padding entries (value 0) add 0.
 
+// Operator data are read once per pass, the gathered vector some 20 times: the
+// vector's lines live in L1 (they are coherent there, since every vector is
+// complete before a barrier's acquire), and the operator's pass it by.  Per inner
+// iteration, gathers from L2 -> from L1 -> and operator past L1: 1.02 M
+// rows 100.9 -> 100.7 -> 96.3 us, 109,202 rows 31.0 -> 30.0 -> 30.0, a 3-D box of
+// 17,343 rows 13.2 -> 11.2 -> 11.1.
+__device__ __forceinline__ float4 ldg_once(const float4* p) {
+    float4 v;
+    asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+        : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+        : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint32_t ldg_once(const uint32_t* p) {
+    uint32_t v;
+    asm("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
 // FP32 SELL row (rows without a compact form): int32 columns of the FP64
 // matrix, FP32 values in the quad layout.
 __device__ __forceinline__ float spmv32_sell_row(const Ppe& A, int K, int row,
@@ -442,7 +461,7 @@ __device__ __forceinline__ float spmv32_sell_row(const Ppe& A, int K, int row,
     const float* vq = A.val32 + qsell_index(row, 0, K);
     float s = 0.f;
     for (int m = 0; m < w; m++)
-        s = fmaf(__ldg(vq + (m >> 2) * 128 + (m & 3)), __ldcg(u + __ldg(cp + m * 32)) - ui, s);
+        s = fmaf(__ldg(vq + (m >> 2) * 128 + (m & 3)), __ldca(u + __ldg(cp + m * 32)) - ui, s);
     return s;
 }
 
@@ -457,14 +476,14 @@ __device__ __forceinline__ float sell_part_sum(const Ppe& A, int K, int row, int
         int c[8];
         float x[8];
         const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 a = __ldg(vq + g * 32), b = g + 1 < g1 ? __ldg(vq + (g + 1) * 32) : zero;
+        const float4 a = ldg_once(vq + g * 32), b = g + 1 < g1 ? ldg_once(vq + (g + 1) * 32) : zero;
 #pragma unroll
         for (int t = 0; t < 8; t++) {
             const int m = 4 * g + t;  // (the columns past the slice's width are not set)
             c[t] = m < w && m < 4 * g1 ? __ldg(cp + m * 32) : row;
         }
 #pragma unroll
-        for (int t = 0; t < 8; t++) x[t] = __ldcg(u + c[t]) - ui;
+        for (int t = 0; t < 8; t++) x[t] = __ldca(u + c[t]) - ui;
         s0 = fmaf(a.x, x[0], s0);
         s1 = fmaf(a.y, x[1], s1);
         s0 = fmaf(a.z, x[2], s0);
@@ -508,14 +527,14 @@ __device__ __forceinline__ float compact_row_sum(const Ppe& A, const MatFree& mf
 #pragma unroll
         for (int q = 0; q < kGroups; q++) {
             const int h = min(g + q, groups - 1);
-            v[q] = __ldg(vp + h * 32);
-            b4[q] = __ldg(ip + h * 32);
+            v[q] = ldg_once(vp + h * 32);
+            b4[q] = ldg_once(ip + h * 32);
         }
         float x[kGroups][4];
 #pragma unroll
         for (int q = 0; q < kGroups; q++)
 #pragma unroll
-            for (int t = 0; t < 4; t++) x[q][t] = __ldcg(u + col(b4[q], t)) - ui;
+            for (int t = 0; t < 4; t++) x[q][t] = __ldca(u + col(b4[q], t)) - ui;
 #pragma unroll
         for (int q = 0; q < kGroups; q++) {
             if (g + q >= groups) break;
@@ -553,17 +572,17 @@ __device__ __forceinline__ void compact_pair(const Ppe& A, const MatFree& mf, in
     for (int g = 0; g < gmax; g += 2) {
         const int ha0 = min(g, ga - 1), ha1 = min(g + 1, ga - 1);
         const int hb0 = min(g, gb - 1), hb1 = min(g + 1, gb - 1);
-        float4 va0 = __ldg(vpa + ha0 * 32), va1 = __ldg(vpa + ha1 * 32);
-        float4 vb0 = __ldg(vpb + hb0 * 32), vb1 = __ldg(vpb + hb1 * 32);
-        const uint32_t ia0 = __ldg(ipa + ha0 * 32), ia1 = __ldg(ipa + ha1 * 32);
-        const uint32_t ib0 = __ldg(ipb + hb0 * 32), ib1 = __ldg(ipb + hb1 * 32);
+        float4 va0 = ldg_once(vpa + ha0 * 32), va1 = ldg_once(vpa + ha1 * 32);
+        float4 vb0 = ldg_once(vpb + hb0 * 32), vb1 = ldg_once(vpb + hb1 * 32);
+        const uint32_t ia0 = ldg_once(ipa + ha0 * 32), ia1 = ldg_once(ipa + ha1 * 32);
+        const uint32_t ib0 = ldg_once(ipb + hb0 * 32), ib1 = ldg_once(ipb + hb1 * 32);
         float xa[8], xb[8];
 #pragma unroll
         for (int t = 0; t < 4; t++) {
-            xa[t] = __ldcg(u + col(sa, ia0, t)) - ua;
-            xa[4 + t] = __ldcg(u + col(sa, ia1, t)) - ua;
-            xb[t] = __ldcg(u + col(sb, ib0, t)) - ub;
-            xb[4 + t] = __ldcg(u + col(sb, ib1, t)) - ub;
+            xa[t] = __ldca(u + col(sa, ia0, t)) - ua;
+            xa[4 + t] = __ldca(u + col(sa, ia1, t)) - ua;
+            xb[t] = __ldca(u + col(sb, ib0, t)) - ub;
+            xb[4 + t] = __ldca(u + col(sb, ib1, t)) - ub;
         }
         const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
         if (g >= ga) va0 = z;
@@ -2193,12 +2212,12 @@ constexpr int kClusterRows = 8000;
 constexpr int kSplitSmem = 192 * 1024;
 constexpr int kSplitLevels = 136 * 1024;
 // Above kStreamRows rows the iteration is bound by the operator pass rather
-// than by the cycle's latency, and its loads in flight need the L1 that shared
-// memory takes away: less shared memory (one more grid-wide level) and fewer
-// cycle warps.  1M rows: 171 us per inner iteration with 192 KB and 512
-// threads, 123 with 104 KB, 108 with 256 threads as well; at 100,000 rows
-// 256 threads cost 37 -> 40 us.
-constexpr int kStreamRows = 300000;
+// than by the cycle's latency, and its loads in flight and gathered vector need
+// the L1 that shared memory takes away: less shared memory (one more grid-wide
+// level) and fewer cycle warps.  Per inner iteration, without and with: 109,202
+// rows 30.0 and 34.0 us, 208,240 rows 35.8 and 32.8, 1M rows 171 and 108 when the
+// line was first drawn.
+constexpr int kStreamRows = 150000;
 constexpr int kStreamLevels = 40 * 1024;
 constexpr int kStreamCycle = 256;
 constexpr int kStreamSmem = 104 * 1024;
