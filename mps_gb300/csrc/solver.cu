@@ -397,7 +397,7 @@ __device__ __forceinline__ double spmv64_row(const Ppe& A, int K, int sl, int la
             v[t] = __ldg(vp + (m + t) * 32);
         }
 #pragma unroll
-        for (int t = 0; t < 8; t++) g[t] = __ldcg(x + c[t]);
+        for (int t = 0; t < 8; t++) g[t] = __ldca(x + c[t]);
 #pragma unroll
         for (int t = 0; t < 8; t += 2) {
             s0 = fma(v[t], g[t], s0);
@@ -413,14 +413,14 @@ __device__ __forceinline__ double spmv64_row(const Ppe& A, int K, int sl, int la
             v[t] = __ldg(vp + (m + t) * 32);
         }
 #pragma unroll
-        for (int t = 0; t < 4; t++) g[t] = __ldcg(x + c[t]);
+        for (int t = 0; t < 4; t++) g[t] = __ldca(x + c[t]);
         s0 = fma(v[0], g[0], s0);
         s1 = fma(v[1], g[1], s1);
         s0 = fma(v[2], g[2], s0);
         s1 = fma(v[3], g[3], s1);
         m += 4;
     }
-    for (; m < w; m++) s0 = fma(__ldg(vp + m * 32), __ldcg(x + __ldg(cp + m * 32)), s0);
+    for (; m < w; m++) s0 = fma(__ldg(vp + m * 32), __ldca(x + __ldg(cp + m * 32)), s0);
     return fma(A.diag[row], xi, s0 + s1);
 }
 
