@@ -194,46 +194,58 @@ __device__ __forceinline__ bool far32(const StateBuf& s, int j, float fx, float 
     return r > bound;
 }
 
-// The candidates of slot k (itself left out) that survive the FP32 pre-filter,
-// in sweep order: four candidates' positions are loaded and tested at a time.
+// The candidates of slot k (itself left out) in slots [b, e) that survive the FP32
+// pre-filter, in order: four candidates' positions are loaded and tested at a time.
+template <bool PLANAR, class F>
+__device__ __forceinline__ void survivors_of_range(const StateBuf& s, int b, int e, int k, float fx, float fy,
+                                                   float fz, float bound, F&& f) {
+#pragma unroll 1
+    for (int j0 = b; j0 < e; j0 += 4) {
+        bool near[4];
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            const int j = min(j0 + t, e - 1);
+            near[t] = !far32<PLANAR>(s, j, fx, fy, fz, bound) && j0 + t < e && j != k;
+        }
+#pragma unroll
+        for (int t = 0; t < 4; t++)
+            if (near[t]) f(j0 + t);
+    }
+}
+
+// The sweep's slot ranges: three columns of cells (planar) or nine rows (3-D),
+// in sweep order.
+template <bool PLANAR>
+__device__ __forceinline__ void row_range(const Consts& c, const int32_t* __restrict__ cs, int32_t key, int row,
+                                          int& b, int& e) {
+    const int kk = PLANAR ? key - 1 + (row - 1) * c.numY
+                          : key - 1 + ((row / 3 - 1) * c.numY + (row % 3 - 1)) * c.numZ;
+    b = __ldg(cs + kk);
+    e = __ldg(cs + kk + 3);
+}
+
+// All of them, in sweep order.
 template <bool PLANAR, class F>
 __device__ __forceinline__ void for_each_survivor(const Consts& c, const StateBuf& s,
                                                   const int32_t* __restrict__ cs, int32_t key, int k, float bound,
                                                   F&& f) {
     const float2 fk = s.xyf[k];
     const float fx = fk.x, fy = fk.y, fz = PLANAR ? 0.f : s.zf[k];
-    auto range = [&](int b, int e) {
-#pragma unroll 1
-        for (int j0 = b; j0 < e; j0 += 4) {
-            bool near[4];
-#pragma unroll
-            for (int t = 0; t < 4; t++) {
-                const int j = min(j0 + t, e - 1);
-                near[t] = !far32<PLANAR>(s, j, fx, fy, fz, bound) && j0 + t < e && j != k;
-            }
-#pragma unroll
-            for (int t = 0; t < 4; t++)
-                if (near[t]) f(j0 + t);
-        }
-    };
     if (PLANAR) {
-        const int kk = key - 1;
         int b[3], e[3];
 #pragma unroll
-        for (int r = 0; r < 3; r++) {
-            b[r] = __ldg(cs + kk + (r - 1) * c.numY);
-            e[r] = __ldg(cs + kk + (r - 1) * c.numY + 3);
-        }
+        for (int r = 0; r < 3; r++) row_range<PLANAR>(c, cs, key, r, b[r], e[r]);
 #pragma unroll 1
-        for (int r = 0; r < 3; r++) range(r == 0 ? b[0] : (r == 1 ? b[1] : b[2]), r == 0 ? e[0] : (r == 1 ? e[1] : e[2]));
+        for (int r = 0; r < 3; r++)
+            survivors_of_range<PLANAR>(s, r == 0 ? b[0] : (r == 1 ? b[1] : b[2]),
+                                       r == 0 ? e[0] : (r == 1 ? e[1] : e[2]), k, fx, fy, fz, bound, f);
     } else {
 #pragma unroll 1
-        for (int jx = -1; jx <= 1; jx++)
-#pragma unroll 1
-            for (int jy = -1; jy <= 1; jy++) {
-                const int kk = key + (jx * c.numY + jy) * c.numZ - 1;
-                range(__ldg(cs + kk), __ldg(cs + kk + 3));
-            }
+        for (int r = 0; r < 9; r++) {
+            int b, e;
+            row_range<PLANAR>(c, cs, key, r, b, e);
+            survivors_of_range<PLANAR>(s, b, e, k, fx, fy, fz, bound, f);
+        }
     }
 }
 

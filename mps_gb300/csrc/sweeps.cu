@@ -15,6 +15,21 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kBatchedList = 80000;  // most particles of the batched list build (k_build_list)
+// Up to kRowSplit particles the sweeps run with one warp per slot range of a
+// particle's 27 (9) cells: one warp for all of them leaves a scene of 17,000
+// particles fewer warps than SM quarters, each bound by one particle's serial
+// chain.  Split and not, the sweeps' kernels and all
+// of a step but the solve: 3-D box of 17,343 particles 0.92 -> 0.48 ms, dam of 2,162
+// 0.19 -> 0.14 (mixed) and 0.23 -> 0.20 (FP64); nothing at 50,469 (0.26 ms both) and
+// a loss at 109,202 (0.44 -> 0.50).
+constexpr int kRowSplit = 20000;
+template <bool PLANAR>
+constexpr int kRows = PLANAR ? 3 : 9;
+// Survivors of one range that a thread keeps: at 3.1 particle distances up to 4 x 4
+// columns of 6 in the middle row of a 3-D box, 4 x 6 planar.
+template <bool PLANAR>
+constexpr int kRowNear = PLANAR ? 64 : 128;
+constexpr int kListWarps = 8;  // warps per 32 particles of the split gradient
 constexpr int kCollBlocks = 304;  // blocks of the parallel collision pass (two per SM)
 
 
@@ -52,6 +67,27 @@ __device__ __forceinline__ void for_each_near(const Consts& c, const StateBuf& s
     }
 }
 
+// As for_each_near, over one of the sweep's slot ranges.
+template <bool PLANAR, class F>
+__device__ __forceinline__ void for_each_near_row(const Consts& c, const StateBuf& s,
+                                                  const int32_t* __restrict__ cs, int32_t key, int k, int row,
+                                                  float bound, F&& f) {
+    const float2 fk = s.xyf[k];
+    int b, e, ns = 0;
+    row_range<PLANAR>(c, cs, key, row, b, e);
+    int cand[kRowNear<PLANAR>];
+    survivors_of_range<PLANAR>(s, b, e, k, fk.x, fk.y, PLANAR ? 0.f : s.zf[k], bound, [&](int j) {
+        if (ns < kRowNear<PLANAR>) cand[ns] = j;
+        ns++;
+    });
+    if (ns <= kRowNear<PLANAR>) {
+        for (int q = 0; q < ns; q++) f(cand[q]);
+    } else {
+        for (int j = b; j < e; j++)
+            if (j != k) f(j);
+    }
+}
+
 // Number density at re_p over a particle's current neighbours (d < re_max),
 // in sweep order: the value a later setNumberDensity reads from the stale
 // list of a particle that has just become a ghost (src/mps.cpp:590-593).
@@ -70,45 +106,51 @@ __device__ double sweep_number_density_p(const Consts& c, const StateBuf& s, con
 // ---------------------------------------------------------------------------
 // calcGravity + calcViscosity + moveParticles (+ checkBoundaryViolation),
 // src/mps.cpp:165-215 and 643-667, fused with the first neighbour sweep.
-// Reads `in`, writes the moved state to `out` (same slot order).
-template <bool PLANAR, bool MIXED>
-__global__ void __launch_bounds__(kThreads) k_explicit(Consts c, StateBuf in, StateBuf out,
+// Reads `in`, writes the moved state to `out` (same slot order).  SPLIT: warp y of
+// a block of 32 particles sums slot range y, the ranges' FP32 sums are added in
+// range order (mixed precision only: the FP64 sum rounds like the reference's,
+// neighbour by neighbour).
+template <bool PLANAR, bool MIXED, bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? 32 * kRows<PLANAR> : kThreads) k_explicit(Consts c, StateBuf in, StateBuf out,
                                                        const int32_t* __restrict__ skey,
                                                        const int32_t* __restrict__ cs,
                                                        int32_t* __restrict__ nkey, int32_t* __restrict__ nrank,
                                                        int32_t* __restrict__ ncount, DevStats* ds) {
+    static_assert(MIXED || !SPLIT, "the FP64 sum is serial");
     int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= c.n) return;
+    if (!SPLIT && k >= c.n) return;
+    __shared__ float part[SPLIT ? kRows<PLANAR> : 1][3][32];
+    const int lane = threadIdx.x & 31;
+    if (SPLIT) k = min(k, c.n - 1);
+    // pairs (j) over this thread's part of the sweep
+    auto sweep = [&](int32_t key, auto&& pair) {
+        if constexpr (SPLIT)
+            for_each_near_row<PLANAR>(c, in, cs, key, k, threadIdx.y, c.ft_v, pair);
+        else
+            for_each_near<PLANAR>(c, in, cs, key, k, c.ft_v, pair);
+    };
+    // the ranges' sums, in range order
+    auto total = [&](int d) {
+        float v = part[0][d][lane];
+        for (int r = 1; r < kRows<PLANAR>; r++) v += part[r][d][lane];
+        return v;
+    };
     int8_t t = in.type[k];
     double x = in.x[k], y = in.y[k], vx = in.vx[k], vy = in.vy[k];
     double z = PLANAR ? c.z0 : in.z[k], vz = PLANAR ? 0.0 : in.vz[k];
     double nd_last = in.nd_last[k];
-    if (t == T_FLUID) {
-        const int32_t key = skey[k];
-        double ax, ay, az;
-        if (!MIXED) {
-            double tx = 0.0, ty = 0.0, tz = 0.0;
-            for_each_near<PLANAR>(c, in, cs, key, k, c.ft_v, [&](int j) {
-                double d2 = dist2<PLANAR>(in, k, j, x, y, z);
-                if (lt_cut(d2, c.t_max) && lt_cut(d2, c.t_v)) {
-                    double w = weight(dsqrt(d2), c.re_v);
-                    tx = dadd(tx, dmul(dsub(in.vx[j], vx), w));
-                    ty = dadd(ty, dmul(dsub(in.vy[j], vy), w));
-                    if (!PLANAR) tz = dadd(tz, dmul(dsub(in.vz[j], vz), w));
-                }
-            });
-            ax = dadd(c.g[0], dmul(tx, c.visc_a));
-            ay = dadd(c.g[1], dmul(ty, c.visc_a));
-            az = PLANAR ? 0.0 : dadd(c.g[2], dmul(tz, c.visc_a));
-        } else if (PLANAR) {
+    const bool fluid = t == T_FLUID;
+    const int32_t key = fluid ? skey[k] : 0;
+    float tx = 0.f, ty = 0.f, tz = 0.f;
+    if (MIXED && fluid) {
+        if (PLANAR) {
             // FP32 weights and FP32 accumulation; the neighbour set is the
             // exact FP64 one: the FP32 squared distance of the coordinate
             // pairs decides outside the band [fv_in, fv_out] around the
             // threshold (its error is far inside the band), the exact FP64
             // test inside it
-            float tx = 0.f, ty = 0.f;
             const float2 hk = in.xyf[k], lk = in.xylo[k], vk = in.vf[k];
-            for_each_near<PLANAR>(c, in, cs, key, k, c.ft_v, [&](int j) {
+            sweep(key, [&](int j) {
                 const float2 hj = in.xyf[j], lj = in.xylo[j];
                 const float dx = (hj.x - hk.x) + (lj.x - lk.x);
                 const float dy = (hj.y - hk.y) + (lj.y - lk.y);
@@ -125,15 +167,11 @@ __global__ void __launch_bounds__(kThreads) k_explicit(Consts c, StateBuf in, St
                     ty = fmaf(vj.y - vk.y, w, ty);
                 }
             });
-            ax = c.g[0] + (double)(tx * c.fvisc_a);
-            ay = c.g[1] + (double)(ty * c.fvisc_a);
-            az = 0.0;
         } else {
             // FP32 weights and FP32 accumulation; the neighbour set is the
             // exact FP64 one.
-            float tx = 0.f, ty = 0.f, tz = 0.f;
             const float fvx = f32(vx), fvy = f32(vy), fvz = f32(vz);
-            for_each_near<PLANAR>(c, in, cs, key, k, c.ft_v, [&](int j) {
+            sweep(key, [&](int j) {
                 double d2 = dist2<PLANAR>(in, k, j, x, y, z);
                 if (lt_cut(d2, c.t_max) && lt_cut(d2, c.t_v)) {
                     float w = c.fre_v * rsqrtf(f32(d2)) - 1.f;
@@ -142,6 +180,35 @@ __global__ void __launch_bounds__(kThreads) k_explicit(Consts c, StateBuf in, St
                     if (!PLANAR) tz = fmaf(f32(in.vz[j]) - fvz, w, tz);
                 }
             });
+        }
+    }
+    if constexpr (SPLIT) {
+        part[threadIdx.y][0][lane] = tx;
+        part[threadIdx.y][1][lane] = ty;
+        part[threadIdx.y][2][lane] = tz;
+        __syncthreads();
+        if (threadIdx.y != 0 || blockIdx.x * blockDim.x + threadIdx.x >= c.n) return;
+        tx = total(0);
+        ty = total(1);
+        tz = PLANAR ? 0.f : total(2);
+    }
+    if (fluid) {
+        double ax, ay, az;
+        if (!MIXED) {
+            double sx = 0.0, sy = 0.0, sz = 0.0;
+            for_each_near<PLANAR>(c, in, cs, key, k, c.ft_v, [&](int j) {
+                double d2 = dist2<PLANAR>(in, k, j, x, y, z);
+                if (lt_cut(d2, c.t_max) && lt_cut(d2, c.t_v)) {
+                    double w = weight(dsqrt(d2), c.re_v);
+                    sx = dadd(sx, dmul(dsub(in.vx[j], vx), w));
+                    sy = dadd(sy, dmul(dsub(in.vy[j], vy), w));
+                    if (!PLANAR) sz = dadd(sz, dmul(dsub(in.vz[j], vz), w));
+                }
+            });
+            ax = dadd(c.g[0], dmul(sx, c.visc_a));
+            ay = dadd(c.g[1], dmul(sy, c.visc_a));
+            az = PLANAR ? 0.0 : dadd(c.g[2], dmul(sz, c.visc_a));
+        } else {
             ax = c.g[0] + (double)(tx * c.fvisc_a);
             ay = c.g[1] + (double)(ty * c.fvisc_a);
             az = PLANAR ? 0.0 : c.g[2] + (double)(tz * c.fvisc_a);
@@ -204,33 +271,53 @@ __global__ void __launch_bounds__(kThreads) k_explicit(Consts c, StateBuf in, St
 template <bool PLANAR>
 __device__ __forceinline__ int for_each_collision(const Consts& c, const StateBuf& s,
                                                   const int32_t* cs, int32_t key, int k,
-                                                  CollPair* out) {
+                                                  CollPair* out, int row = -1) {
     double xi = s.x[k], yi = s.y[k], zi = PLANAR ? 0.0 : s.z[k];
     int32_t idi = s.id[k];
     int m = 0;
-    for_each_survivor<PLANAR>(c, s, cs, key, k, c.ft_cd, [&](int j) {
+    auto pair = [&](int j) {
         double d2 = dist2<PLANAR>(s, k, j, xi, yi, zi);
         if (!(lt_cut(d2, c.t_max) && lt_cut(d2, c.t_cd))) return;
         if (s.type[j] == T_FLUID && s.id[j] >= idi) return;
         if (out) out[m] = CollPair{k, j, idi, s.id[j], dsqrt(d2)};
         m++;
-    });
+    };
+    if (row < 0) {
+        for_each_survivor<PLANAR>(c, s, cs, key, k, c.ft_cd, pair);
+    } else {
+        const float2 fk = s.xyf[k];
+        int b, e;
+        row_range<PLANAR>(c, cs, key, row, b, e);
+        survivors_of_range<PLANAR>(s, b, e, k, fk.x, fk.y, PLANAR ? 0.f : s.zf[k], c.ft_cd, pair);
+    }
     return m;
 }
 
-template <bool PLANAR>
-__global__ void __launch_bounds__(kThreads) k_coll_count(Consts c, StateBuf s,
+template <bool PLANAR, bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? 32 * kRows<PLANAR> : kThreads) k_coll_count(Consts c, StateBuf s,
                                                          const int32_t* __restrict__ skey,
                                                          const int32_t* __restrict__ cs,
                                                          int32_t* __restrict__ cnt_by_id, CollWork cw) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
+    int m = 0;
+    if (SPLIT) {  // one warp per slot range, as k_explicit
+        __shared__ int part[kRows<PLANAR>][32];
+        const int lane = threadIdx.x & 31;
+        if (k < c.n && s.type[k] == T_FLUID)
+            m = for_each_collision<PLANAR>(c, s, cs, skey[k], k, nullptr, threadIdx.y);
+        part[threadIdx.y][lane] = m;
+        __syncthreads();
+        if (threadIdx.y != 0) return;
+        for (int r = 1; r < kRows<PLANAR>; r++) m += part[r][lane];
+    }
     if (k >= c.n) return;
+    if (!SPLIT && s.type[k] == T_FLUID) m = for_each_collision<PLANAR>(c, s, cs, skey[k], k, nullptr);
     // also resets the parallel pass's counters (every id once)
     const int id = s.id[k];
     cw.jn[id] = 0;
     cw.ver[id] = 0;
     if (k < 3) cw.ctl[k] = 0;
-    cnt_by_id[id] = s.type[k] == T_FLUID ? for_each_collision<PLANAR>(c, s, cs, skey[k], k, nullptr) : 0;
+    cnt_by_id[id] = m;
 }
 
 template <bool PLANAR>
@@ -418,76 +505,75 @@ __global__ void __launch_bounds__(kThreads) k_coll_wave(Consts c, StateBuf s, co
 // (2,000 particles: 47 -> 27 us with B = 4); at 1M it is bound by issue, where
 // the batch's registers cost more than they give, and B = 1 stays.
 template <bool PLANAR, bool BC, int B>
-__global__ void __launch_bounds__(kThreads) k_build_list(Consts c, StateBuf s,
-                                                         const int32_t* __restrict__ skey,
-                                                         const int32_t* __restrict__ cs, NbList nb,
-                                                         Ppe A, DevStats* ds) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = k < c.n && s.type[k] != T_GHOST;
+__device__ __forceinline__ void list_serial(const Consts& c, const StateBuf& s, const int32_t* __restrict__ skey,
+                                            const int32_t* __restrict__ cs, const NbList& nb, int k, int& m,
+                                            double& nd, double& nsurf) {
     const int np = nb.n_pad;
-    int m = 0;
-    double nd = 0.0, nsurf = 0.0;  // number densities at re_p and (BC) re_s
-    if (valid) {
-        const double xi = s.x[k], yi = s.y[k], zi = PLANAR ? 0.0 : s.z[k];
-        // Pass 1: the candidates that survive the FP32 pre-filter, in sweep
-        // order.  Pass 2 then runs the exact FP64 test, square root and
-        // division on these compact per-particle lists, with nearly all lanes
-        // of a warp busy (a candidate survives for only part of a warp).
-        int ns = 0;
-        for_each_survivor<PLANAR>(c, s, cs, skey[k], k, c.ft_max, [&](int j) {
-            if (ns < c.K) nb.slot[(size_t)ns * np + k] = j;
-            ns++;
-        });
-        if (ns <= c.K) {
-            // exact test, compacting in place (order kept): src/mps.cpp:585-619
-            for (int q0 = 0; q0 < ns; q0 += B) {
-                int j[B];
-                double dist[B], w[B], ws[B];
-                bool in[B];
+    const double xi = s.x[k], yi = s.y[k], zi = PLANAR ? 0.0 : s.z[k];
+    // Pass 1: the candidates that survive the FP32 pre-filter, in sweep
+    // order.  Pass 2 then runs the exact FP64 test, square root and
+    // division on these compact per-particle lists, with nearly all lanes
+    // of a warp busy (a candidate survives for only part of a warp).
+    int ns = 0;
+    for_each_survivor<PLANAR>(c, s, cs, skey[k], k, c.ft_max, [&](int j) {
+        if (ns < c.K) nb.slot[(size_t)ns * np + k] = j;
+        ns++;
+    });
+    if (ns <= c.K) {
+        // exact test, compacting in place (order kept): src/mps.cpp:585-619
+        for (int q0 = 0; q0 < ns; q0 += B) {
+            int j[B];
+            double dist[B], w[B], ws[B];
+            bool in[B];
 #pragma unroll
-                for (int t = 0; t < B; t++) j[t] = nb.slot[(size_t)min(q0 + t, ns - 1) * np + k];
+            for (int t = 0; t < B; t++) j[t] = nb.slot[(size_t)min(q0 + t, ns - 1) * np + k];
 #pragma unroll
-                for (int t = 0; t < B; t++) {
-                    const double d2 = dist2<PLANAR>(s, k, j[t], xi, yi, zi);
-                    in[t] = q0 + t < ns && lt_cut(d2, c.t_max);
-                    if (B == 1 && !in[t]) continue;
-                    dist[t] = dsqrt(d2);
-                    w[t] = weight(dist[t], c.re_p);
-                    ws[t] = BC ? weight(dist[t], c.re_s) : 0.0;
-                }
-#pragma unroll
-                for (int t = 0; t < B; t++) {
-                    if (!in[t]) continue;
-                    if (lt_cut(dist[t], c.re_p)) nd = dadd(nd, w[t]);  // src/mps.cpp:573-583
-                    if (BC && lt_cut(dist[t], c.re_s)) nsurf = dadd(nsurf, ws[t]);
-                    const size_t e = (size_t)m * np + k;
-                    nb.slot[e] = j[t];
-                    nb.dist[e] = dist[t];
-                    nb.wp[e] = w[t];
-                    m++;
-                }
+            for (int t = 0; t < B; t++) {
+                const double d2 = dist2<PLANAR>(s, k, j[t], xi, yi, zi);
+                in[t] = q0 + t < ns && lt_cut(d2, c.t_max);
+                if (B == 1 && !in[t]) continue;
+                dist[t] = dsqrt(d2);
+                w[t] = weight(dist[t], c.re_p);
+                ws[t] = BC ? weight(dist[t], c.re_s) : 0.0;
             }
-        } else {
-            // more survivors than the list holds: the exact one-pass sweep
-            for_each_candidate<PLANAR>(c, cs, skey[k], [&](int j) {
-                if (j == k) return;
-                const double d2 = dist2<PLANAR>(s, k, j, xi, yi, zi);
-                if (!lt_cut(d2, c.t_max)) return;
-                const double dist = dsqrt(d2);
-                const double w = weight(dist, c.re_p);
-                if (lt_cut(dist, c.re_p)) nd = dadd(nd, w);
-                if (m < c.K) {
-                    if (BC && lt_cut(dist, c.re_s)) nsurf = dadd(nsurf, weight(dist, c.re_s));
-                    const size_t e = (size_t)m * np + k;
-                    nb.slot[e] = j;
-                    nb.dist[e] = dist;
-                    nb.wp[e] = w;
-                }
+#pragma unroll
+            for (int t = 0; t < B; t++) {
+                if (!in[t]) continue;
+                if (lt_cut(dist[t], c.re_p)) nd = dadd(nd, w[t]);  // src/mps.cpp:573-583
+                if (BC && lt_cut(dist[t], c.re_s)) nsurf = dadd(nsurf, ws[t]);
+                const size_t e = (size_t)m * np + k;
+                nb.slot[e] = j[t];
+                nb.dist[e] = dist[t];
+                nb.wp[e] = w[t];
                 m++;
-            });
+            }
         }
-        s.nd_last[k] = nd;
+    } else {
+        // more survivors than the list holds: the exact one-pass sweep
+        for_each_candidate<PLANAR>(c, cs, skey[k], [&](int j) {
+            if (j == k) return;
+            const double d2 = dist2<PLANAR>(s, k, j, xi, yi, zi);
+            if (!lt_cut(d2, c.t_max)) return;
+            const double dist = dsqrt(d2);
+            const double w = weight(dist, c.re_p);
+            if (lt_cut(dist, c.re_p)) nd = dadd(nd, w);
+            if (m < c.K) {
+                if (BC && lt_cut(dist, c.re_s)) nsurf = dadd(nsurf, weight(dist, c.re_s));
+                const size_t e = (size_t)m * np + k;
+                nb.slot[e] = j;
+                nb.dist[e] = dist;
+                nb.wp[e] = w;
+            }
+            m++;
+        });
     }
+}
+
+// What follows a particle's list and sums: called by whole warps, one particle per lane.
+template <bool BC>
+__device__ __forceinline__ void list_finish(const Consts& c, const StateBuf& s, const NbList& nb, const Ppe& A,
+                                            DevStats* ds, int k, bool valid, int m, double nd, double nsurf) {
+    if (valid) s.nd_last[k] = nd;
     if (k < c.n) nb.cnt[k] = m < c.K ? m : c.K;
     if (m > c.K) raise_status(ds, ST_CAPACITY);
     if (BC) {
@@ -510,6 +596,134 @@ __global__ void __launch_bounds__(kThreads) k_build_list(Consts c, StateBuf s,
     // one atomic per warp for the largest neighbour count
     const int wmax = __reduce_max_sync(0xffffffffu, m);
     if ((threadIdx.x & 31) == 0 && wmax > 0) atomicMax(&ds->max_neighbors, wmax);
+}
+
+template <bool PLANAR, bool BC, int B>
+__global__ void __launch_bounds__(kThreads) k_build_list(Consts c, StateBuf s,
+                                                         const int32_t* __restrict__ skey,
+                                                         const int32_t* __restrict__ cs, NbList nb,
+                                                         Ppe A, DevStats* ds) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool valid = k < c.n && s.type[k] != T_GHOST;
+    int m = 0;
+    double nd = 0.0, nsurf = 0.0;  // number densities at re_p and (BC) re_s
+    if (valid) list_serial<PLANAR, BC, B>(c, s, skey, cs, nb, k, m, nd, nsurf);
+    list_finish<BC>(c, s, nb, A, ds, k, valid, m, nd, nsurf);
+}
+
+// The same list with one warp per slot range (32 particles per block) for the
+// pre-filter; then the block's warps share the survivors, each entry at the place
+// that counts the survivors before it.  The few particles with a survivor that the
+// exact test rejects close the gap afterwards.  A range with more survivors than a
+// thread keeps, or a list longer than the table, sends the block through the serial
+// form.
+template <bool PLANAR, bool BC>
+__global__ void __launch_bounds__(32 * kRows<PLANAR>) k_build_rows(Consts c, StateBuf s,
+                                                                   const int32_t* __restrict__ skey,
+                                                                   const int32_t* __restrict__ cs, NbList nb,
+                                                                   Ppe A, DevStats* ds) {
+    constexpr int R = kRows<PLANAR>;
+    __shared__ int s_cnt[R][32], s_gap[32];
+    __shared__ double s_term[2][1 + BC][32][32], s_surf[32];
+    const int lane = threadIdx.x, row = threadIdx.y;
+    const int k = blockIdx.x * 32 + lane;
+    const bool valid = k < c.n && s.type[k] != T_GHOST;
+    const int np = nb.n_pad;
+    int cand[kRowNear<PLANAR>];
+    int ns = 0;
+    if (valid) {
+        const float2 fk = s.xyf[k];
+        int b, e;
+        row_range<PLANAR>(c, cs, skey[k], row, b, e);
+        survivors_of_range<PLANAR>(s, b, e, k, fk.x, fk.y, PLANAR ? 0.f : s.zf[k], c.ft_max, [&](int j) {
+            if (ns < kRowNear<PLANAR>) cand[ns] = j;
+            ns++;
+        });
+    }
+    s_cnt[row][lane] = ns;
+    if (row == 0) s_gap[lane] = 0;
+    __syncthreads();
+    int at = 0, m = 0;
+    for (int r = 0; r < R; r++) {
+        if (r == row) at = m;
+        m += s_cnt[r][lane];
+    }
+    double nd = 0.0, nsurf = 0.0;
+    if (__syncthreads_or(ns > kRowNear<PLANAR> || m > c.K)) {
+        if (row != 0) return;
+        m = 0;
+        if (valid) list_serial<PLANAR, BC, 1>(c, s, skey, cs, nb, k, m, nd, nsurf);
+        list_finish<BC>(c, s, nb, A, ds, k, valid, m, nd, nsurf);
+        return;
+    }
+    for (int q = 0; q < ns; q++) nb.slot[(size_t)(at + q) * np + k] = cand[q];
+    __syncthreads();
+    // 32 entries at a time: the warps share them, four per pass and warp, then one
+    // warp per sum adds the terms in list order (src/mps.cpp:573-583; 0 outside the
+    // radius, which adds nothing) while the others go on
+    const int wmax = __reduce_max_sync(0xffffffffu, m);  // (the same in every warp)
+    const double xi = valid ? s.x[k] : 0.0, yi = valid ? s.y[k] : 0.0, zi = PLANAR || !valid ? 0.0 : s.z[k];
+    double sum = 0.0;
+    bool gap = false;
+    for (int q0 = 0, par = 0; q0 < wmax; q0 += 32, par ^= 1) {
+        for (int b = row; b < 32; b += 4 * R) {
+            int j[4];
+            double dist[4], w[4], ws[4];
+            bool in[4];
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                const int q = q0 + b + t * R;
+                in[t] = b + t * R < 32 && q < m;
+                j[t] = in[t] ? nb.slot[(size_t)q * np + k] : min(k, c.n - 1);
+            }
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                const double d2 = in[t] ? dist2<PLANAR>(s, k, j[t], xi, yi, zi) : 1.0;
+                if (in[t] && !lt_cut(d2, c.t_max)) j[t] = -1;
+                dist[t] = dsqrt(d2);
+                w[t] = weight(dist[t], c.re_p);
+                ws[t] = !BC ? 0.0 : (c.re_s == c.re_p ? w[t] : weight(dist[t], c.re_s));
+            }
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                const int q = b + t * R;
+                if (q >= 32) break;
+                const bool used = in[t] && j[t] >= 0;
+                s_term[par][0][q][lane] = used && lt_cut(dist[t], c.re_p) ? w[t] : 0.0;
+                if (BC) s_term[par][BC][q][lane] = used && lt_cut(dist[t], c.re_s) ? ws[t] : 0.0;
+                if (!in[t]) continue;
+                const size_t e = (size_t)(q0 + q) * np + k;
+                if (!used) nb.slot[e] = -1;
+                gap = gap || !used;
+                nb.dist[e] = dist[t];
+                nb.wp[e] = w[t];
+            }
+        }
+        __syncthreads();
+        if (row < 1 + BC) {
+#pragma unroll 8
+            for (int q = 0; q < 32; q++) sum = dadd(sum, s_term[par][row][q][lane]);
+        }
+    }
+    if (gap) s_gap[lane] = 1;
+    if (BC && row == 1) s_surf[lane] = sum;
+    __syncthreads();
+    if (row != 0) return;
+    if (s_gap[lane]) {
+        const int all = m;
+        m = 0;
+        for (int q = 0; q < all; q++) {
+            const size_t e = (size_t)q * np + k, o = (size_t)m * np + k;
+            if (nb.slot[e] < 0) continue;
+            if (o != e) {
+                nb.slot[o] = nb.slot[e];
+                nb.dist[o] = nb.dist[e];
+                nb.wp[o] = nb.wp[e];
+            }
+            m++;
+        }
+    }
+    list_finish<BC>(c, s, nb, A, ds, k, valid, m, sum, BC ? s_surf[lane] : 0.0);
 }
 
 // Higher-order source term (src/mps.cpp:288-306), needs every neighbour's BC.
@@ -763,16 +977,25 @@ __global__ void k_pressure_out(int n, const double* __restrict__ x, double* __re
 // not Ignored, then MPS::calcPressureGradient (src/mps.cpp:505-533) for the
 // fluid ones, which use their own minimum: one kernel, two passes over the
 // particle's list (the second mostly from cache).
-template <bool PLANAR, bool MIXED>
+template <bool PLANAR, bool MIXED, bool SPLIT>
 __global__ void __launch_bounds__(kThreads) k_gradient(Consts c, StateBuf s, NbList nb, double* ax,
                                                        double* ay, double* az) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= c.n || s.bc[k] == BC_IGNORED) return;
-    const int np = nb.n_pad, m = nb.cnt[k];
+    static_assert(MIXED || !SPLIT, "the FP64 sum is serial");
+    const int kk = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool on = kk < c.n && s.bc[kk] != BC_IGNORED;
+    if (!SPLIT && !on) return;
+    const int k = SPLIT ? min(kk, c.n - 1) : kk;
+    // SPLIT: warp y takes every kListWarps-th group of four entries; the FP32 sums
+    // of the groups are added in warp order (mixed precision only)
+    __shared__ double s_min[SPLIT ? kListWarps : 1][32];
+    __shared__ float part[SPLIT ? kListWarps : 1][3][32];
+    const int lane = threadIdx.x & 31;
+    const int q_first = SPLIT ? 4 * threadIdx.y : 0, q_step = SPLIT ? 4 * kListWarps : 4;
+    const int np = nb.n_pad, m = on ? nb.cnt[k] : 0;
     // four neighbours' loads at a time (the columns of the list are one trip to
     // memory, the neighbours' fields a second), minima and sums in list order
     double pmin = s.p[k];
-    for (int q0 = 0; q0 < m; q0 += 4) {
+    for (int q0 = q_first; q0 < m; q0 += q_step) {
         int j[4];
         bool in[4];
 #pragma unroll
@@ -791,9 +1014,31 @@ __global__ void __launch_bounds__(kThreads) k_gradient(Consts c, StateBuf s, NbL
         for (int t = 0; t < 4; t++)
             if (in[t] && pmin > pj[t]) pmin = pj[t];
     }
-    s.minp[k] = pmin;
+    if (SPLIT) {
+        s_min[threadIdx.y][lane] = pmin;
+        __syncthreads();
+        for (int r = 0; r < kListWarps; r++)
+            if (pmin > s_min[r][lane]) pmin = s_min[r][lane];
+    }
+    if (on && (!SPLIT || threadIdx.y == 0)) s.minp[k] = pmin;
     // a fluid particle is never Ignored (only dummies and ghosts are)
-    if (s.type[k] != T_FLUID) return;
+    const bool fluid = on && s.type[k] == T_FLUID;
+    if (!SPLIT && !fluid) return;
+    // the sums of a particle's warps, in warp order; true: this thread writes
+    auto join = [&](float& gx, float& gy, float& gz) {
+        if (!SPLIT) return true;
+        part[threadIdx.y][0][lane] = gx;
+        part[threadIdx.y][1][lane] = gy;
+        part[threadIdx.y][2][lane] = gz;
+        __syncthreads();
+        if (threadIdx.y != 0) return false;
+        for (int r = 1; r < kListWarps; r++) {
+            gx += part[r][0][lane];
+            gy += part[r][1][lane];
+            gz += part[r][2][lane];
+        }
+        return fluid;
+    };
     const double xi = s.x[k], yi = s.y[k], zi = PLANAR ? 0.0 : s.z[k];
     if (!MIXED) {
         double gx = 0.0, gy = 0.0, gz = 0.0;
@@ -842,10 +1087,10 @@ __global__ void __launch_bounds__(kThreads) k_gradient(Consts c, StateBuf s, NbL
         // FP32 pairs (hi, lo), each within FP32 rounding of the exact
         // difference (the FP64 subtractions they replace were most of this
         // kernel's FP64 pipe time)
-        float gx = 0.f, gy = 0.f;
+        float gx = 0.f, gy = 0.f, gz = 0.f;
         const float2 hk = s.xyf[k], lk = s.xylo[k];
         const float pmh = f32(pmin), pml = f32(pmin - (double)pmh);
-        for (int q0 = 0; q0 < m; q0 += 4) {
+        for (int q0 = q_first; q0 < (fluid ? m : 0); q0 += q_step) {
             int j[4];
             double dist[4];
             float2 hj[4], lj[4], pj[4];
@@ -873,22 +1118,41 @@ __global__ void __launch_bounds__(kThreads) k_gradient(Consts c, StateBuf s, NbL
                 gy = fmaf((hj[t].y - hk.y) + (lj[t].y - lk.y), coef, gy);
             }
         }
+        if (!join(gx, gy, gz)) return;
         const float sc = -c.fgrad_scale / f32(c.rho);
         ax[k] = (double)(gx * sc);
         ay[k] = (double)(gy * sc);
     } else {
         float gx = 0.f, gy = 0.f, gz = 0.f;
-        for (int q = 0; q < m; q++) {
-            int j = nb.slot[(size_t)q * np + k];
-            if (s.type[j] == T_DUMMY) continue;
-            double dist = nb.dist[(size_t)q * np + k];
-            if (!lt_cut(dist, c.re_p)) continue;
-            float fd = f32(dist);
-            float coef = f32(s.p[j] - pmin) * (c.fre_p / fd - 1.f) / (fd * fd);
-            gx = fmaf(f32(s.x[j] - xi), coef, gx);
-            gy = fmaf(f32(s.y[j] - yi), coef, gy);
-            gz = fmaf(f32(s.z[j] - zi), coef, gz);
+        for (int q0 = q_first; q0 < (fluid ? m : 0); q0 += q_step) {
+            int j[4];
+            double dist[4], dp[4], tx[4], ty[4], tz[4];
+            bool in[4];
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                const size_t e = (size_t)min(q0 + t, m - 1) * np + k;
+                j[t] = nb.slot[e];
+                dist[t] = nb.dist[e];
+            }
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                in[t] = q0 + t < m && lt_cut(dist[t], c.re_p) && s.type[j[t]] != T_DUMMY;
+                dp[t] = s.p[j[t]];
+                tx[t] = s.x[j[t]];
+                ty[t] = s.y[j[t]];
+                tz[t] = s.z[j[t]];
+            }
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                if (!in[t]) continue;
+                const float fd = f32(dist[t]);
+                const float coef = f32(dp[t] - pmin) * (c.fre_p / fd - 1.f) / (fd * fd);
+                gx = fmaf(f32(tx[t] - xi), coef, gx);
+                gy = fmaf(f32(ty[t] - yi), coef, gy);
+                gz = fmaf(f32(tz[t] - zi), coef, gz);
+            }
         }
+        if (!join(gx, gy, gz)) return;
         const float sc = -c.fgrad_scale / f32(c.rho);
         ax[k] = (double)(gx * sc);
         ay[k] = (double)(gy * sc);
@@ -949,37 +1213,36 @@ __global__ void k_number_density(Consts c, StateBuf s) {
 
 void launch_explicit(const Consts& c, const StateBuf& in, const StateBuf& out,
                      const SortScratch& sc, int mixed, DevStats* ds, cudaStream_t st) {
-    int nb = block_count(c.n);
-    if (c.planar) {
-        if (mixed) {
-            k_explicit<true, true><<<nb, block_threads(c.n), 0, st>>>(c, in, out, sc.skey, sc.cell_start, sc.key, sc.rank, sc.cell_count, ds);
-            ++g_launches;
-        } else {
-            k_explicit<true, false><<<nb, block_threads(c.n), 0, st>>>(c, in, out, sc.skey, sc.cell_start, sc.key, sc.rank, sc.cell_count, ds);
-            ++g_launches;
-        }
-    } else {
-        if (mixed) {
-            k_explicit<false, true><<<nb, block_threads(c.n), 0, st>>>(c, in, out, sc.skey, sc.cell_start, sc.key, sc.rank, sc.cell_count, ds);
-            ++g_launches;
-        } else {
-            k_explicit<false, false><<<nb, block_threads(c.n), 0, st>>>(c, in, out, sc.skey, sc.cell_start, sc.key, sc.rank, sc.cell_count, ds);
-            ++g_launches;
-        }
-    }
+    const bool split = mixed && c.n <= kRowSplit;
+    auto launch = [&](auto kernel, int rows) {
+        const dim3 block = split ? dim3(32, rows) : dim3(block_threads(c.n));
+        kernel<<<split ? (c.n + 31) / 32 : block_count(c.n), block, 0, st>>>(c, in, out, sc.skey, sc.cell_start, sc.key,
+                                                                           sc.rank, sc.cell_count, ds);
+        ++g_launches;
+    };
+    if (c.planar)
+        launch(split ? k_explicit<true, true, true> : (mixed ? k_explicit<true, true, false> : k_explicit<true, false, false>),
+               kRows<true>);
+    else
+        launch(split ? k_explicit<false, true, true>
+                     : (mixed ? k_explicit<false, true, false> : k_explicit<false, false, false>),
+               kRows<false>);
 }
 
 void launch_collision(const Consts& c, const StateBuf& s, const SortScratch& sc,
                       int32_t* cand_cnt, int32_t* cand_base, const CollWork& cw, CollPair* pairs,
                       int32_t pair_cap, int32_t* scan_tmp, DevStats* ds, cudaStream_t st) {
     int nb = block_count(c.n);
-    if (c.planar) {
-        k_coll_count<true><<<nb, block_threads(c.n), 0, st>>>(c, s, sc.skey, sc.cell_start, cand_cnt, cw);
+    const bool split = c.n <= kRowSplit;
+    auto count = [&](auto kernel, int rows) {
+        const dim3 block = split ? dim3(32, rows) : dim3(block_threads(c.n));
+        kernel<<<split ? (c.n + 31) / 32 : nb, block, 0, st>>>(c, s, sc.skey, sc.cell_start, cand_cnt, cw);
         ++g_launches;
-    } else {
-        k_coll_count<false><<<nb, block_threads(c.n), 0, st>>>(c, s, sc.skey, sc.cell_start, cand_cnt, cw);
-        ++g_launches;
-    }
+    };
+    if (c.planar)
+        count(split ? k_coll_count<true, true> : k_coll_count<true, false>, kRows<true>);
+    else
+        count(split ? k_coll_count<false, true> : k_coll_count<false, false>, kRows<false>);
     launch_exclusive_scan(cand_cnt, cand_base, c.n, scan_tmp, false, st);
     const int32_t* total = cand_base + c.n;
     const int T = block_threads(c.n);
@@ -997,7 +1260,10 @@ void launch_collision(const Consts& c, const StateBuf& s, const SortScratch& sc,
 template <bool PLANAR, bool BC>
 static void build_list(const Consts& c, const StateBuf& s, const SortScratch& sc, const NbList& nb, const Ppe& A,
                        DevStats* ds, cudaStream_t st) {
-    if (c.n <= kBatchedList)
+    if (c.n <= kRowSplit)
+        k_build_rows<PLANAR, BC><<<(c.n + 31) / 32, dim3(32, kRows<PLANAR>), 0, st>>>(c, s, sc.skey, sc.cell_start, nb, A,
+                                                                                   ds);
+    else if (c.n <= kBatchedList)
         k_build_list<PLANAR, BC, 4><<<block_count(c.n), block_threads(c.n), 0, st>>>(c, s, sc.skey, sc.cell_start, nb,
                                                                                     A, ds);
     else
@@ -1065,27 +1331,21 @@ void launch_pressure_post(const Consts& c, const StateBuf& s, const NbList& nb, 
     int g = block_count(c.n);
     k_pressure_out<<<g, block_threads(c.n), 0, st>>>(c.n, x, s.p, s.pf, s.id, x_prev, ds);
     ++g_launches;
+    const bool split = mixed && c.n <= kRowSplit;
+    auto gradient = [&](auto kernel) {
+        const dim3 block = split ? dim3(32, kListWarps) : dim3(block_threads(c.n));
+        kernel<<<split ? (c.n + 31) / 32 : g, block, 0, st>>>(c, s, nb, ax, ay, az);
+        ++g_launches;
+    };
     if (c.planar) {
-        if (mixed) {
-            k_gradient<true, true><<<g, block_threads(c.n), 0, st>>>(c, s, nb, ax, ay, az);
-            ++g_launches;
-        } else {
-            k_gradient<true, false><<<g, block_threads(c.n), 0, st>>>(c, s, nb, ax, ay, az);
-            ++g_launches;
-        }
+        gradient(split ? k_gradient<true, true, true> : (mixed ? k_gradient<true, true, false> : k_gradient<true, false, false>));
         k_move2<true><<<g, block_threads(c.n), 0, st>>>(c, s, ax, ay, az, ds);
-        ++g_launches;
     } else {
-        if (mixed) {
-            k_gradient<false, true><<<g, block_threads(c.n), 0, st>>>(c, s, nb, ax, ay, az);
-            ++g_launches;
-        } else {
-            k_gradient<false, false><<<g, block_threads(c.n), 0, st>>>(c, s, nb, ax, ay, az);
-            ++g_launches;
-        }
+        gradient(split ? k_gradient<false, true, true>
+                       : (mixed ? k_gradient<false, true, false> : k_gradient<false, false, false>));
         k_move2<false><<<g, block_threads(c.n), 0, st>>>(c, s, ax, ay, az, ds);
-        ++g_launches;
     }
+    ++g_launches;
 }
 
 void launch_number_density(const Consts& c, const StateBuf& s, const NbList& /*nb*/,
