@@ -67,27 +67,6 @@ __device__ __forceinline__ void for_each_near(const Consts& c, const StateBuf& s
     }
 }
 
-// As for_each_near, over one of the sweep's slot ranges.
-template <bool PLANAR, class F>
-__device__ __forceinline__ void for_each_near_row(const Consts& c, const StateBuf& s,
-                                                  const int32_t* __restrict__ cs, int32_t key, int k, int row,
-                                                  float bound, F&& f) {
-    const float2 fk = s.xyf[k];
-    int b, e, ns = 0;
-    row_range<PLANAR>(c, cs, key, row, b, e);
-    int cand[kRowNear<PLANAR>];
-    survivors_of_range<PLANAR>(s, b, e, k, fk.x, fk.y, PLANAR ? 0.f : s.zf[k], bound, [&](int j) {
-        if (ns < kRowNear<PLANAR>) cand[ns] = j;
-        ns++;
-    });
-    if (ns <= kRowNear<PLANAR>) {
-        for (int q = 0; q < ns; q++) f(cand[q]);
-    } else {
-        for (int j = b; j < e; j++)
-            if (j != k) f(j);
-    }
-}
-
 // Number density at re_p over a particle's current neighbours (d < re_max),
 // in sweep order: the value a later setNumberDensity reads from the stale
 // list of a particle that has just become a ghost (src/mps.cpp:590-593).
@@ -107,8 +86,8 @@ __device__ double sweep_number_density_p(const Consts& c, const StateBuf& s, con
 // calcGravity + calcViscosity + moveParticles (+ checkBoundaryViolation),
 // src/mps.cpp:165-215 and 643-667, fused with the first neighbour sweep.
 // Reads `in`, writes the moved state to `out` (same slot order).  SPLIT: warp y of
-// a block of 32 particles sums slot range y, the ranges' FP32 sums are added in
-// range order (mixed precision only: the FP64 sum rounds like the reference's,
+// a block of 32 particles pre-filters slot range y, the warps share the survivors and
+// their FP32 sums are added in warp order (mixed precision only: the FP64 sum rounds like the reference's,
 // neighbour by neighbour).
 template <bool PLANAR, bool MIXED, bool SPLIT>
 __global__ void __launch_bounds__(SPLIT ? 32 * kRows<PLANAR> : kThreads) k_explicit(Consts c, StateBuf in, StateBuf out,
@@ -122,14 +101,43 @@ __global__ void __launch_bounds__(SPLIT ? 32 * kRows<PLANAR> : kThreads) k_expli
     __shared__ float part[SPLIT ? kRows<PLANAR> : 1][3][32];
     const int lane = threadIdx.x & 31;
     if (SPLIT) k = min(k, c.n - 1);
-    // pairs (j) over this thread's part of the sweep
+    // pairs (j) over this thread's part of the sweep; SPLIT: called by every thread
+    // of the block, which then shares the survivors of all ranges
+    constexpr int kShared = SPLIT ? (PLANAR ? 64 : 256) : 1;
+    __shared__ int s_list[kShared][32], s_cnt[SPLIT ? kRows<PLANAR> : 1][32];
     auto sweep = [&](int32_t key, auto&& pair) {
-        if constexpr (SPLIT)
-            for_each_near_row<PLANAR>(c, in, cs, key, k, threadIdx.y, c.ft_v, pair);
-        else
+        if constexpr (SPLIT) {
+            constexpr int R = kRows<PLANAR>;
+            const int row = threadIdx.y;
+            int cand[kRowNear<PLANAR>], b = 0, e = 0, ns = 0;
+            if (in.type[k] == T_FLUID) {
+                const float2 fk = in.xyf[k];
+                row_range<PLANAR>(c, cs, key, row, b, e);
+                survivors_of_range<PLANAR>(in, b, e, k, fk.x, fk.y, PLANAR ? 0.f : in.zf[k], c.ft_v, [&](int j) {
+                    if (ns < kRowNear<PLANAR>) cand[ns] = j;
+                    ns++;
+                });
+            }
+            s_cnt[row][lane] = ns;
+            __syncthreads();
+            int at = 0, m = 0;
+            for (int r = 0; r < R; r++) {
+                if (r == row) at = m;
+                m += s_cnt[r][lane];
+            }
+            if (__syncthreads_or(ns > kRowNear<PLANAR> || m > kShared)) {
+                for (int j = b; j < e; j++)
+                    if (j != k) pair(j);
+            } else {
+                for (int q = 0; q < ns; q++) s_list[at + q][lane] = cand[q];
+                __syncthreads();
+                for (int q = row; q < m; q += R) pair(s_list[q][lane]);
+            }
+        } else {
             for_each_near<PLANAR>(c, in, cs, key, k, c.ft_v, pair);
+        }
     };
-    // the ranges' sums, in range order
+    // the warps' sums, in warp order
     auto total = [&](int d) {
         float v = part[0][d][lane];
         for (int r = 1; r < kRows<PLANAR>; r++) v += part[r][d][lane];
@@ -142,7 +150,7 @@ __global__ void __launch_bounds__(SPLIT ? 32 * kRows<PLANAR> : kThreads) k_expli
     const bool fluid = t == T_FLUID;
     const int32_t key = fluid ? skey[k] : 0;
     float tx = 0.f, ty = 0.f, tz = 0.f;
-    if (MIXED && fluid) {
+    if (MIXED && (SPLIT || fluid)) {
         if (PLANAR) {
             // FP32 weights and FP32 accumulation; the neighbour set is the
             // exact FP64 one: the FP32 squared distance of the coordinate
