@@ -325,7 +325,8 @@ void enqueue_step(mps_engine* e, bool do_export) {
 // Algorithmic bytes of one pressure solve: each array a solver pass streams,
 // counted once at its stored width (gathered vector entries count once, as
 // the row's own entry).  Per stored off-diagonal entry and pass: FP64 12 B
-// (column + value), compact FP32 5 B (value + index byte).  Per row and
+// (column + value; the one-kernel CG streams 10, with 16-bit window indices, and
+// small scenes none), compact FP32 5 B (value + index byte).  Per row and
 // iteration: FP64 CG 116 B (8 vectors); MIXED inner iteration 69 B with the
 // Jacobi preconditioner; with the multigrid V-cycle, per cell of level 1
 // 72 B (segment bounds, the up pass's 9-point stencil and 8 vector words)

@@ -14,7 +14,6 @@ namespace mpsg {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kBatchedList = 80000;  // most particles of the batched list build (k_build_list)
 // Up to kRowSplit particles the sweeps run with one warp per slot range of a
 // particle's 27 (9) cells: one warp for all of them leaves a scene of 17,000
 // particles fewer warps than SM quarters, each bound by one particle's serial
@@ -86,9 +85,8 @@ __device__ double sweep_number_density_p(const Consts& c, const StateBuf& s, con
 // calcGravity + calcViscosity + moveParticles (+ checkBoundaryViolation),
 // src/mps.cpp:165-215 and 643-667, fused with the first neighbour sweep.
 // Reads `in`, writes the moved state to `out` (same slot order).  SPLIT: warp y of
-// a block of 32 particles pre-filters slot range y, the warps share the survivors and
-// their FP32 sums are added in warp order (mixed precision only: the FP64 sum rounds like the reference's,
-// neighbour by neighbour).
+// a block of 32 particles pre-filters slot range y, the warps share the survivors'
+// terms, and the sums run in sweep order (the same bits; mixed precision only).
 template <bool PLANAR, bool MIXED, bool SPLIT>
 __global__ void __launch_bounds__(SPLIT ? 32 * kRows<PLANAR> : kThreads) k_explicit(Consts c, StateBuf in, StateBuf out,
                                                        const int32_t* __restrict__ skey,
@@ -98,107 +96,113 @@ __global__ void __launch_bounds__(SPLIT ? 32 * kRows<PLANAR> : kThreads) k_expli
     static_assert(MIXED || !SPLIT, "the FP64 sum is serial");
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (!SPLIT && k >= c.n) return;
-    __shared__ float part[SPLIT ? kRows<PLANAR> : 1][3][32];
-    const int lane = threadIdx.x & 31;
     if (SPLIT) k = min(k, c.n - 1);
-    // pairs (j) over this thread's part of the sweep; SPLIT: called by every thread
-    // of the block, which then shares the survivors of all ranges
-    constexpr int kShared = SPLIT ? (PLANAR ? 64 : 256) : 1;
-    __shared__ int s_list[kShared][32], s_cnt[SPLIT ? kRows<PLANAR> : 1][32];
-    auto sweep = [&](int32_t key, auto&& pair) {
-        if constexpr (SPLIT) {
-            constexpr int R = kRows<PLANAR>;
-            const int row = threadIdx.y;
-            int cand[kRowNear<PLANAR>], b = 0, e = 0, ns = 0;
-            if (in.type[k] == T_FLUID) {
-                const float2 fk = in.xyf[k];
-                row_range<PLANAR>(c, cs, key, row, b, e);
-                survivors_of_range<PLANAR>(in, b, e, k, fk.x, fk.y, PLANAR ? 0.f : in.zf[k], c.ft_v, [&](int j) {
-                    if (ns < kRowNear<PLANAR>) cand[ns] = j;
-                    ns++;
-                });
-            }
-            s_cnt[row][lane] = ns;
-            __syncthreads();
-            int at = 0, m = 0;
-            for (int r = 0; r < R; r++) {
-                if (r == row) at = m;
-                m += s_cnt[r][lane];
-            }
-            if (__syncthreads_or(ns > kRowNear<PLANAR> || m > kShared)) {
-                for (int j = b; j < e; j++)
-                    if (j != k) pair(j);
-            } else {
-                for (int q = 0; q < ns; q++) s_list[at + q][lane] = cand[q];
-                __syncthreads();
-                for (int q = row; q < m; q += R) pair(s_list[q][lane]);
-            }
-        } else {
-            for_each_near<PLANAR>(c, in, cs, key, k, c.ft_v, pair);
-        }
-    };
-    // the warps' sums, in warp order
-    auto total = [&](int d) {
-        float v = part[0][d][lane];
-        for (int r = 1; r < kRows<PLANAR>; r++) v += part[r][d][lane];
-        return v;
-    };
     int8_t t = in.type[k];
     double x = in.x[k], y = in.y[k], vx = in.vx[k], vy = in.vy[k];
     double z = PLANAR ? c.z0 : in.z[k], vz = PLANAR ? 0.0 : in.vz[k];
     double nd_last = in.nd_last[k];
     const bool fluid = t == T_FLUID;
     const int32_t key = fluid ? skey[k] : 0;
-    float tx = 0.f, ty = 0.f, tz = 0.f;
-    if (MIXED && (SPLIT || fluid)) {
-        if (PLANAR) {
-            // FP32 weights and FP32 accumulation; the neighbour set is the
-            // exact FP64 one: the FP32 squared distance of the coordinate
-            // pairs decides outside the band [fv_in, fv_out] around the
-            // threshold (its error is far inside the band), the exact FP64
-            // test inside it
-            const float2 hk = in.xyf[k], lk = in.xylo[k], vk = in.vf[k];
-            sweep(key, [&](int j) {
-                const float2 hj = in.xyf[j], lj = in.xylo[j];
-                const float dx = (hj.x - hk.x) + (lj.x - lk.x);
-                const float dy = (hj.y - hk.y) + (lj.y - lk.y);
-                const float d2f = dx * dx + dy * dy;
-                bool inside = d2f < c.fv_in;
-                if (!inside && !(d2f > c.fv_out)) {
-                    const double d2 = dist2<PLANAR>(in, k, j, x, y, z);
-                    inside = lt_cut(d2, c.t_max) && lt_cut(d2, c.t_v);
-                }
-                if (inside) {
-                    const float2 vj = in.vf[j];
-                    const float w = c.fre_v * rsqrtf(d2f) - 1.f;
-                    tx = fmaf(vj.x - vk.x, w, tx);
-                    ty = fmaf(vj.y - vk.y, w, ty);
-                }
-            });
+    // Mixed: FP32 weights and FP32 accumulation over the exact FP64 neighbour set.
+    // The term of candidate j: velocity differences and weight (0 outside the radius).
+    // Planar: the FP32 squared distance of the coordinate pairs decides outside the
+    // band [fv_in, fv_out] around the threshold (its error is far inside the band),
+    // the exact FP64 test inside it.
+    const float2 hk = PLANAR && MIXED ? in.xyf[k] : float2{}, lk = PLANAR && MIXED ? in.xylo[k] : float2{},
+                 vk = PLANAR && MIXED ? in.vf[k] : float2{};
+    const float fvx = f32(vx), fvy = f32(vy), fvz = f32(vz);
+    auto term = [&](int j) {
+        float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+        if constexpr (PLANAR) {
+            const float2 hj = in.xyf[j], lj = in.xylo[j];
+            const float dx = (hj.x - hk.x) + (lj.x - lk.x);
+            const float dy = (hj.y - hk.y) + (lj.y - lk.y);
+            const float d2f = dx * dx + dy * dy;
+            bool inside = d2f < c.fv_in;
+            if (!inside && !(d2f > c.fv_out)) {
+                const double d2 = dist2<PLANAR>(in, k, j, x, y, z);
+                inside = lt_cut(d2, c.t_max) && lt_cut(d2, c.t_v);
+            }
+            if (inside) {
+                const float2 vj = in.vf[j];
+                r = make_float4(vj.x - vk.x, vj.y - vk.y, 0.f, c.fre_v * rsqrtf(d2f) - 1.f);
+            }
         } else {
-            // FP32 weights and FP32 accumulation; the neighbour set is the
-            // exact FP64 one.
-            const float fvx = f32(vx), fvy = f32(vy), fvz = f32(vz);
-            sweep(key, [&](int j) {
-                double d2 = dist2<PLANAR>(in, k, j, x, y, z);
-                if (lt_cut(d2, c.t_max) && lt_cut(d2, c.t_v)) {
-                    float w = c.fre_v * rsqrtf(f32(d2)) - 1.f;
-                    tx = fmaf(f32(in.vx[j]) - fvx, w, tx);
-                    ty = fmaf(f32(in.vy[j]) - fvy, w, ty);
-                    if (!PLANAR) tz = fmaf(f32(in.vz[j]) - fvz, w, tz);
-                }
+            const double d2 = dist2<PLANAR>(in, k, j, x, y, z);
+            if (lt_cut(d2, c.t_max) && lt_cut(d2, c.t_v))
+                r = make_float4(f32(in.vx[j]) - fvx, f32(in.vy[j]) - fvy, f32(in.vz[j]) - fvz,
+                                c.fre_v * rsqrtf(f32(d2)) - 1.f);
+        }
+        return r;
+    };
+    float tx = 0.f, ty = 0.f, tz = 0.f;
+    if constexpr (SPLIT) {
+        constexpr int R = kRows<PLANAR>, kShared = PLANAR ? 64 : 232;  // (48 KB in all)
+        __shared__ int s_list[kShared][32], s_cnt[R][32];
+        __shared__ float4 s_term[32][32];
+        __shared__ float s_sum[3][32];
+        const int lane = threadIdx.x, row = threadIdx.y;
+        int cand[kRowNear<PLANAR>], ns = 0;
+        if (fluid) {
+            const float2 fk = in.xyf[k];
+            int b, e;
+            row_range<PLANAR>(c, cs, key, row, b, e);
+            survivors_of_range<PLANAR>(in, b, e, k, fk.x, fk.y, PLANAR ? 0.f : in.zf[k], c.ft_v, [&](int j) {
+                if (ns < kRowNear<PLANAR>) cand[ns] = j;
+                ns++;
             });
         }
-    }
-    if constexpr (SPLIT) {
-        part[threadIdx.y][0][lane] = tx;
-        part[threadIdx.y][1][lane] = ty;
-        part[threadIdx.y][2][lane] = tz;
+        s_cnt[row][lane] = ns;
         __syncthreads();
-        if (threadIdx.y != 0 || blockIdx.x * blockDim.x + threadIdx.x >= c.n) return;
-        tx = total(0);
-        ty = total(1);
-        tz = PLANAR ? 0.f : total(2);
+        int at = 0, m = 0;
+        for (int r = 0; r < R; r++) {
+            if (r == row) at = m;
+            m += s_cnt[r][lane];
+        }
+        if (__syncthreads_or(ns > kRowNear<PLANAR> || m > kShared)) {
+            // more survivors than the lists hold: one warp, every candidate
+            if (row == 0 && fluid)
+                for_each_candidate<PLANAR>(c, cs, key, [&](int j) {
+                    if (j == k) return;
+                    const float4 q = term(j);
+                    tx = fmaf(q.x, q.w, tx);
+                    ty = fmaf(q.y, q.w, ty);
+                    tz = fmaf(q.z, q.w, tz);
+                });
+        } else {
+            for (int q = 0; q < ns; q++) s_list[at + q][lane] = cand[q];
+            __syncthreads();
+            // 32 survivors at a time: the warps share the terms, then one warp per
+            // component adds them in sweep order
+            const int wmax = __reduce_max_sync(0xffffffffu, m);
+            float sum = 0.f;
+            for (int q0 = 0; q0 < wmax; q0 += 32) {
+                for (int q = row; q < 32; q += R)
+                    s_term[q][lane] = q0 + q < m ? term(s_list[q0 + q][lane]) : make_float4(0.f, 0.f, 0.f, 0.f);
+                __syncthreads();
+                if (row < (PLANAR ? 2 : 3)) {
+#pragma unroll 8
+                    for (int q = 0; q < 32; q++) {
+                        const float* p = reinterpret_cast<const float*>(&s_term[q][lane]);
+                        sum = fmaf(p[row], p[3], sum);
+                    }
+                }
+                __syncthreads();
+            }
+            if (row < 3) s_sum[row][lane] = sum;
+            __syncthreads();
+            tx = s_sum[0][lane];
+            ty = s_sum[1][lane];
+            tz = PLANAR ? 0.f : s_sum[2][lane];
+        }
+        if (row != 0 || blockIdx.x * blockDim.x + threadIdx.x >= c.n) return;
+    } else if (MIXED && fluid) {
+        for_each_near<PLANAR>(c, in, cs, key, k, c.ft_v, [&](int j) {
+            const float4 q = term(j);
+            tx = fmaf(q.x, q.w, tx);
+            ty = fmaf(q.y, q.w, ty);
+            if (!PLANAR) tz = fmaf(q.z, q.w, tz);
+        });
     }
     if (fluid) {
         double ax, ay, az;
@@ -506,13 +510,7 @@ __global__ void __launch_bounds__(kThreads) k_coll_wave(Consts c, StateBuf s, co
 // and the classic setSourceTerm (src/mps.cpp:262-320): the surface number
 // density summed over the list entries within re_s, in list order (the
 // order in which the reference's getNumberDensity reads the stored list).
-//
-// Batches of B candidates in pass 2: their loads, square roots and divisions
-// are independent, only the append and the sums go in order.  With few warps
-// per SM quarter the kernel is bound by the latency of one particle's chain
-// (2,000 particles: 47 -> 27 us with B = 4); at 1M it is bound by issue, where
-// the batch's registers cost more than they give, and B = 1 stays.
-template <bool PLANAR, bool BC, int B>
+template <bool PLANAR, bool BC>
 __device__ __forceinline__ void list_serial(const Consts& c, const StateBuf& s, const int32_t* __restrict__ skey,
                                             const int32_t* __restrict__ cs, const NbList& nb, int k, int& m,
                                             double& nd, double& nsurf) {
@@ -529,32 +527,19 @@ __device__ __forceinline__ void list_serial(const Consts& c, const StateBuf& s, 
     });
     if (ns <= c.K) {
         // exact test, compacting in place (order kept): src/mps.cpp:585-619
-        for (int q0 = 0; q0 < ns; q0 += B) {
-            int j[B];
-            double dist[B], w[B], ws[B];
-            bool in[B];
-#pragma unroll
-            for (int t = 0; t < B; t++) j[t] = nb.slot[(size_t)min(q0 + t, ns - 1) * np + k];
-#pragma unroll
-            for (int t = 0; t < B; t++) {
-                const double d2 = dist2<PLANAR>(s, k, j[t], xi, yi, zi);
-                in[t] = q0 + t < ns && lt_cut(d2, c.t_max);
-                if (B == 1 && !in[t]) continue;
-                dist[t] = dsqrt(d2);
-                w[t] = weight(dist[t], c.re_p);
-                ws[t] = BC ? weight(dist[t], c.re_s) : 0.0;
-            }
-#pragma unroll
-            for (int t = 0; t < B; t++) {
-                if (!in[t]) continue;
-                if (lt_cut(dist[t], c.re_p)) nd = dadd(nd, w[t]);  // src/mps.cpp:573-583
-                if (BC && lt_cut(dist[t], c.re_s)) nsurf = dadd(nsurf, ws[t]);
-                const size_t e = (size_t)m * np + k;
-                nb.slot[e] = j[t];
-                nb.dist[e] = dist[t];
-                nb.wp[e] = w[t];
-                m++;
-            }
+        for (int q = 0; q < ns; q++) {
+            const int j = nb.slot[(size_t)q * np + k];
+            const double d2 = dist2<PLANAR>(s, k, j, xi, yi, zi);
+            if (!lt_cut(d2, c.t_max)) continue;
+            const double dist = dsqrt(d2);
+            const double w = weight(dist, c.re_p);
+            if (lt_cut(dist, c.re_p)) nd = dadd(nd, w);  // src/mps.cpp:573-583
+            if (BC && lt_cut(dist, c.re_s)) nsurf = dadd(nsurf, weight(dist, c.re_s));
+            const size_t e = (size_t)m * np + k;
+            nb.slot[e] = j;
+            nb.dist[e] = dist;
+            nb.wp[e] = w;
+            m++;
         }
     } else {
         // more survivors than the list holds: the exact one-pass sweep
@@ -606,7 +591,7 @@ __device__ __forceinline__ void list_finish(const Consts& c, const StateBuf& s, 
     if ((threadIdx.x & 31) == 0 && wmax > 0) atomicMax(&ds->max_neighbors, wmax);
 }
 
-template <bool PLANAR, bool BC, int B>
+template <bool PLANAR, bool BC>
 __global__ void __launch_bounds__(kThreads) k_build_list(Consts c, StateBuf s,
                                                          const int32_t* __restrict__ skey,
                                                          const int32_t* __restrict__ cs, NbList nb,
@@ -615,7 +600,7 @@ __global__ void __launch_bounds__(kThreads) k_build_list(Consts c, StateBuf s,
     const bool valid = k < c.n && s.type[k] != T_GHOST;
     int m = 0;
     double nd = 0.0, nsurf = 0.0;  // number densities at re_p and (BC) re_s
-    if (valid) list_serial<PLANAR, BC, B>(c, s, skey, cs, nb, k, m, nd, nsurf);
+    if (valid) list_serial<PLANAR, BC>(c, s, skey, cs, nb, k, m, nd, nsurf);
     list_finish<BC>(c, s, nb, A, ds, k, valid, m, nd, nsurf);
 }
 
@@ -660,7 +645,7 @@ __global__ void __launch_bounds__(32 * kRows<PLANAR>) k_build_rows(Consts c, Sta
     if (__syncthreads_or(ns > kRowNear<PLANAR> || m > c.K)) {
         if (row != 0) return;
         m = 0;
-        if (valid) list_serial<PLANAR, BC, 1>(c, s, skey, cs, nb, k, m, nd, nsurf);
+        if (valid) list_serial<PLANAR, BC>(c, s, skey, cs, nb, k, m, nd, nsurf);
         list_finish<BC>(c, s, nb, A, ds, k, valid, m, nd, nsurf);
         return;
     }
@@ -993,10 +978,12 @@ __global__ void __launch_bounds__(kThreads) k_gradient(Consts c, StateBuf s, NbL
     const bool on = kk < c.n && s.bc[kk] != BC_IGNORED;
     if (!SPLIT && !on) return;
     const int k = SPLIT ? min(kk, c.n - 1) : kk;
-    // SPLIT: warp y takes every kListWarps-th group of four entries; the FP32 sums
-    // of the groups are added in warp order (mixed precision only)
+    // SPLIT: warp y takes every kListWarps-th group of four entries; the terms of 32
+    // entries meet in shared memory, where one warp per component adds them in list
+    // order (the same bits; mixed precision only)
     __shared__ double s_min[SPLIT ? kListWarps : 1][32];
-    __shared__ float part[SPLIT ? kListWarps : 1][3][32];
+    __shared__ float4 s_term[SPLIT ? 4 * kListWarps : 1][32];
+    __shared__ float s_sum[SPLIT ? 3 : 1][32];
     const int lane = threadIdx.x & 31;
     const int q_first = SPLIT ? 4 * threadIdx.y : 0, q_step = SPLIT ? 4 * kListWarps : 4;
     const int np = nb.n_pad, m = on ? nb.cnt[k] : 0;
@@ -1032,20 +1019,47 @@ __global__ void __launch_bounds__(kThreads) k_gradient(Consts c, StateBuf s, NbL
     // a fluid particle is never Ignored (only dummies and ghosts are)
     const bool fluid = on && s.type[k] == T_FLUID;
     if (!SPLIT && !fluid) return;
-    // the sums of a particle's warps, in warp order; true: this thread writes
-    auto join = [&](float& gx, float& gy, float& gz) {
-        if (!SPLIT) return true;
-        part[threadIdx.y][0][lane] = gx;
-        part[threadIdx.y][1][lane] = gy;
-        part[threadIdx.y][2][lane] = gz;
-        __syncthreads();
-        if (threadIdx.y != 0) return false;
-        for (int r = 1; r < kListWarps; r++) {
-            gx += part[r][0][lane];
-            gy += part[r][1][lane];
-            gz += part[r][2][lane];
+    // The FP32 sums of the particle's list; terms(q0, r): the coordinate differences
+    // and coefficients of entries q0 .. q0 + 3 (0 for those that do not count).
+    // false: another thread writes the result.
+    auto sums = [&](float (&g)[3], auto&& terms) {
+        float4 r[4];
+        if constexpr (!SPLIT) {
+            for (int q0 = 0; q0 < m; q0 += 4) {
+                terms(q0, r);
+#pragma unroll
+                for (int t = 0; t < 4; t++) {
+                    g[0] = fmaf(r[t].x, r[t].w, g[0]);
+                    g[1] = fmaf(r[t].y, r[t].w, g[1]);
+                    if (!PLANAR) g[2] = fmaf(r[t].z, r[t].w, g[2]);
+                }
+            }
+            return true;
         }
-        return fluid;
+        const int mine = fluid ? m : 0, wmax = __reduce_max_sync(0xffffffffu, mine);
+        const int row = threadIdx.y;
+        float sum = 0.f;
+        for (int q0 = 0; q0 < wmax; q0 += 4 * kListWarps) {
+#pragma unroll
+            for (int t = 0; t < 4; t++) r[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (q0 + q_first < mine) terms(q0 + q_first, r);
+#pragma unroll
+            for (int t = 0; t < 4; t++) s_term[q_first + t][lane] = r[t];
+            __syncthreads();
+            if (row < (PLANAR ? 2 : 3)) {
+#pragma unroll 8
+                for (int q = 0; q < 4 * kListWarps; q++) {
+                    const float* p = reinterpret_cast<const float*>(&s_term[q][lane]);
+                    sum = fmaf(p[row], p[3], sum);
+                }
+            }
+            __syncthreads();
+        }
+        if (row < 3) s_sum[row][lane] = sum;
+        __syncthreads();
+        if (row != 0 || !fluid) return false;
+        for (int d = 0; d < 3; d++) g[d] = s_sum[d][lane];
+        return true;
     };
     const double xi = s.x[k], yi = s.y[k], zi = PLANAR ? 0.0 : s.z[k];
     if (!MIXED) {
@@ -1095,10 +1109,10 @@ __global__ void __launch_bounds__(kThreads) k_gradient(Consts c, StateBuf s, NbL
         // FP32 pairs (hi, lo), each within FP32 rounding of the exact
         // difference (the FP64 subtractions they replace were most of this
         // kernel's FP64 pipe time)
-        float gx = 0.f, gy = 0.f, gz = 0.f;
+        float g[3] = {0.f, 0.f, 0.f};
         const float2 hk = s.xyf[k], lk = s.xylo[k];
         const float pmh = f32(pmin), pml = f32(pmin - (double)pmh);
-        for (int q0 = q_first; q0 < (fluid ? m : 0); q0 += q_step) {
+        const bool writes = sums(g, [&](int q0, float4 (&r)[4]) {
             int j[4];
             double dist[4];
             float2 hj[4], lj[4], pj[4];
@@ -1118,21 +1132,21 @@ __global__ void __launch_bounds__(kThreads) k_gradient(Consts c, StateBuf s, NbL
             }
 #pragma unroll
             for (int t = 0; t < 4; t++) {
-                if (!in[t]) continue;
                 const float fd = f32(dist[t]);
                 const float dp = (pj[t].x - pmh) + (pj[t].y - pml);
                 const float coef = dp * (c.fre_p / fd - 1.f) / (fd * fd);
-                gx = fmaf((hj[t].x - hk.x) + (lj[t].x - lk.x), coef, gx);
-                gy = fmaf((hj[t].y - hk.y) + (lj[t].y - lk.y), coef, gy);
+                r[t] = in[t] ? make_float4((hj[t].x - hk.x) + (lj[t].x - lk.x), (hj[t].y - hk.y) + (lj[t].y - lk.y),
+                                           0.f, coef)
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
             }
-        }
-        if (!join(gx, gy, gz)) return;
+        });
+        if (!writes) return;
         const float sc = -c.fgrad_scale / f32(c.rho);
-        ax[k] = (double)(gx * sc);
-        ay[k] = (double)(gy * sc);
+        ax[k] = (double)(g[0] * sc);
+        ay[k] = (double)(g[1] * sc);
     } else {
-        float gx = 0.f, gy = 0.f, gz = 0.f;
-        for (int q0 = q_first; q0 < (fluid ? m : 0); q0 += q_step) {
+        float g[3] = {0.f, 0.f, 0.f};
+        const bool writes = sums(g, [&](int q0, float4 (&r)[4]) {
             int j[4];
             double dist[4], dp[4], tx[4], ty[4], tz[4];
             bool in[4];
@@ -1152,19 +1166,17 @@ __global__ void __launch_bounds__(kThreads) k_gradient(Consts c, StateBuf s, NbL
             }
 #pragma unroll
             for (int t = 0; t < 4; t++) {
-                if (!in[t]) continue;
                 const float fd = f32(dist[t]);
                 const float coef = f32(dp[t] - pmin) * (c.fre_p / fd - 1.f) / (fd * fd);
-                gx = fmaf(f32(tx[t] - xi), coef, gx);
-                gy = fmaf(f32(ty[t] - yi), coef, gy);
-                gz = fmaf(f32(tz[t] - zi), coef, gz);
+                r[t] = in[t] ? make_float4(f32(tx[t] - xi), f32(ty[t] - yi), f32(tz[t] - zi), coef)
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
             }
-        }
-        if (!join(gx, gy, gz)) return;
+        });
+        if (!writes) return;
         const float sc = -c.fgrad_scale / f32(c.rho);
-        ax[k] = (double)(gx * sc);
-        ay[k] = (double)(gy * sc);
-        if (!PLANAR) az[k] = (double)(gz * sc);
+        ax[k] = (double)(g[0] * sc);
+        ay[k] = (double)(g[1] * sc);
+        if (!PLANAR) az[k] = (double)(g[2] * sc);
     }
 }
 
@@ -1271,12 +1283,8 @@ static void build_list(const Consts& c, const StateBuf& s, const SortScratch& sc
     if (c.n <= kRowSplit)
         k_build_rows<PLANAR, BC><<<(c.n + 31) / 32, dim3(32, kRows<PLANAR>), 0, st>>>(c, s, sc.skey, sc.cell_start, nb, A,
                                                                                    ds);
-    else if (c.n <= kBatchedList)
-        k_build_list<PLANAR, BC, 4><<<block_count(c.n), block_threads(c.n), 0, st>>>(c, s, sc.skey, sc.cell_start, nb,
-                                                                                    A, ds);
     else
-        k_build_list<PLANAR, BC, 1><<<block_count(c.n), block_threads(c.n), 0, st>>>(c, s, sc.skey, sc.cell_start, nb,
-                                                                                    A, ds);
+        k_build_list<PLANAR, BC><<<block_count(c.n), block_threads(c.n), 0, st>>>(c, s, sc.skey, sc.cell_start, nb, A, ds);
     ++g_launches;
 }
 
