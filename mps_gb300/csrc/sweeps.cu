@@ -19,7 +19,7 @@ constexpr int kThreads = 256;
 // particles fewer warps than SM quarters, each bound by one particle's serial
 // chain.  Split and not, the sweeps' kernels and all
 // of a step but the solve: 3-D box of 17,343 particles 0.92 -> 0.48 ms, dam of 2,162
-// 0.19 -> 0.14 (mixed) and 0.23 -> 0.20 (FP64); nothing at 50,469 (0.26 ms both) and
+// 0.19 -> 0.14 (mixed) and 0.23 -> 0.15 (FP64); nothing at 50,469 (0.26 ms both) and
 // a loss at 109,202 (0.44 -> 0.50).
 constexpr int kRowSplit = 20000;
 template <bool PLANAR>
@@ -86,14 +86,13 @@ __device__ double sweep_number_density_p(const Consts& c, const StateBuf& s, con
 // src/mps.cpp:165-215 and 643-667, fused with the first neighbour sweep.
 // Reads `in`, writes the moved state to `out` (same slot order).  SPLIT: warp y of
 // a block of 32 particles pre-filters slot range y, the warps share the survivors'
-// terms, and the sums run in sweep order (the same bits; mixed precision only).
+// terms, and the sums run in sweep order (the same bits).
 template <bool PLANAR, bool MIXED, bool SPLIT>
 __global__ void __launch_bounds__(SPLIT ? 32 * kRows<PLANAR> : kThreads) k_explicit(Consts c, StateBuf in, StateBuf out,
                                                        const int32_t* __restrict__ skey,
                                                        const int32_t* __restrict__ cs,
                                                        int32_t* __restrict__ nkey, int32_t* __restrict__ nrank,
                                                        int32_t* __restrict__ ncount, DevStats* ds) {
-    static_assert(MIXED || !SPLIT, "the FP64 sum is serial");
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (!SPLIT && k >= c.n) return;
     if (SPLIT) k = min(k, c.n - 1);
@@ -135,12 +134,33 @@ __global__ void __launch_bounds__(SPLIT ? 32 * kRows<PLANAR> : kThreads) k_expli
         }
         return r;
     };
+    // FP64: the products themselves, rounded as the reference's
+    auto term64 = [&](int j, double (&r)[3]) {
+        r[0] = r[1] = r[2] = 0.0;
+        const double d2 = dist2<PLANAR>(in, k, j, x, y, z);
+        if (!(lt_cut(d2, c.t_max) && lt_cut(d2, c.t_v))) return;
+        const double w = weight(dsqrt(d2), c.re_v);
+        r[0] = dmul(dsub(in.vx[j], vx), w);
+        r[1] = dmul(dsub(in.vy[j], vy), w);
+        if (!PLANAR) r[2] = dmul(dsub(in.vz[j], vz), w);
+    };
     float tx = 0.f, ty = 0.f, tz = 0.f;
+    double sx = 0.0, sy = 0.0, sz = 0.0;
+    auto add64 = [&](int j) {
+        double r[3];
+        term64(j, r);
+        sx = dadd(sx, r[0]);
+        sy = dadd(sy, r[1]);
+        if (!PLANAR) sz = dadd(sz, r[2]);
+    };
     if constexpr (SPLIT) {
         constexpr int R = kRows<PLANAR>, kShared = PLANAR ? 64 : 232;  // (48 KB in all)
         __shared__ int s_list[kShared][32], s_cnt[R][32];
-        __shared__ float4 s_term[32][32];
+        constexpr int kChunk = MIXED ? 32 : 16, D = PLANAR ? 2 : 3;
+        __shared__ float4 s_term[MIXED ? kChunk : 1][32];
+        __shared__ double s_term64[MIXED ? 1 : kChunk][D][32];
         __shared__ float s_sum[3][32];
+        __shared__ double s_sum64[3][32];
         const int lane = threadIdx.x, row = threadIdx.y;
         int cand[kRowNear<PLANAR>], ns = 0;
         if (fluid) {
@@ -164,36 +184,60 @@ __global__ void __launch_bounds__(SPLIT ? 32 * kRows<PLANAR> : kThreads) k_expli
             if (row == 0 && fluid)
                 for_each_candidate<PLANAR>(c, cs, key, [&](int j) {
                     if (j == k) return;
-                    const float4 q = term(j);
-                    tx = fmaf(q.x, q.w, tx);
-                    ty = fmaf(q.y, q.w, ty);
-                    tz = fmaf(q.z, q.w, tz);
+                    if constexpr (MIXED) {
+                        const float4 q = term(j);
+                        tx = fmaf(q.x, q.w, tx);
+                        ty = fmaf(q.y, q.w, ty);
+                        tz = fmaf(q.z, q.w, tz);
+                    } else {
+                        add64(j);
+                    }
                 });
         } else {
             for (int q = 0; q < ns; q++) s_list[at + q][lane] = cand[q];
             __syncthreads();
-            // 32 survivors at a time: the warps share the terms, then one warp per
-            // component adds them in sweep order
+            // a chunk of survivors at a time: the warps share the terms, then one warp
+            // per component adds them in sweep order (zeros add nothing)
             const int wmax = __reduce_max_sync(0xffffffffu, m);
             float sum = 0.f;
-            for (int q0 = 0; q0 < wmax; q0 += 32) {
-                for (int q = row; q < 32; q += R)
-                    s_term[q][lane] = q0 + q < m ? term(s_list[q0 + q][lane]) : make_float4(0.f, 0.f, 0.f, 0.f);
+            double sum64 = 0.0;
+            for (int q0 = 0; q0 < wmax; q0 += kChunk) {
+                for (int q = row; q < kChunk; q += R) {
+                    const bool used = q0 + q < m;
+                    if constexpr (MIXED) {
+                        s_term[q][lane] = used ? term(s_list[q0 + q][lane]) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    } else {
+                        double r[3] = {0.0, 0.0, 0.0};
+                        if (used) term64(s_list[q0 + q][lane], r);
+                        for (int d = 0; d < D; d++) s_term64[q][d][lane] = r[d];
+                    }
+                }
                 __syncthreads();
-                if (row < (PLANAR ? 2 : 3)) {
+                if (row < D) {
 #pragma unroll 8
-                    for (int q = 0; q < 32; q++) {
-                        const float* p = reinterpret_cast<const float*>(&s_term[q][lane]);
-                        sum = fmaf(p[row], p[3], sum);
+                    for (int q = 0; q < kChunk; q++) {
+                        if constexpr (MIXED) {
+                            const float* p = reinterpret_cast<const float*>(&s_term[q][lane]);
+                            sum = fmaf(p[row], p[3], sum);
+                        } else {
+                            sum64 = dadd(sum64, s_term64[q][row][lane]);
+                        }
                     }
                 }
                 __syncthreads();
             }
-            if (row < 3) s_sum[row][lane] = sum;
+            if (MIXED && row < 3) s_sum[row][lane] = sum;
+            if (!MIXED && row < 3) s_sum64[row][lane] = sum64;
             __syncthreads();
-            tx = s_sum[0][lane];
-            ty = s_sum[1][lane];
-            tz = PLANAR ? 0.f : s_sum[2][lane];
+            if (MIXED) {
+                tx = s_sum[0][lane];
+                ty = s_sum[1][lane];
+                tz = PLANAR ? 0.f : s_sum[2][lane];
+            } else {
+                sx = s_sum64[0][lane];
+                sy = s_sum64[1][lane];
+                sz = s_sum64[2][lane];
+            }
         }
         if (row != 0 || blockIdx.x * blockDim.x + threadIdx.x >= c.n) return;
     } else if (MIXED && fluid) {
@@ -203,20 +247,12 @@ __global__ void __launch_bounds__(SPLIT ? 32 * kRows<PLANAR> : kThreads) k_expli
             ty = fmaf(q.y, q.w, ty);
             if (!PLANAR) tz = fmaf(q.z, q.w, tz);
         });
+    } else if (fluid) {
+        for_each_near<PLANAR>(c, in, cs, key, k, c.ft_v, add64);
     }
     if (fluid) {
         double ax, ay, az;
         if (!MIXED) {
-            double sx = 0.0, sy = 0.0, sz = 0.0;
-            for_each_near<PLANAR>(c, in, cs, key, k, c.ft_v, [&](int j) {
-                double d2 = dist2<PLANAR>(in, k, j, x, y, z);
-                if (lt_cut(d2, c.t_max) && lt_cut(d2, c.t_v)) {
-                    double w = weight(dsqrt(d2), c.re_v);
-                    sx = dadd(sx, dmul(dsub(in.vx[j], vx), w));
-                    sy = dadd(sy, dmul(dsub(in.vy[j], vy), w));
-                    if (!PLANAR) sz = dadd(sz, dmul(dsub(in.vz[j], vz), w));
-                }
-            });
             ax = dadd(c.g[0], dmul(sx, c.visc_a));
             ay = dadd(c.g[1], dmul(sy, c.visc_a));
             az = PLANAR ? 0.0 : dadd(c.g[2], dmul(sz, c.visc_a));
@@ -973,17 +1009,19 @@ __global__ void k_pressure_out(int n, const double* __restrict__ x, double* __re
 template <bool PLANAR, bool MIXED, bool SPLIT>
 __global__ void __launch_bounds__(kThreads) k_gradient(Consts c, StateBuf s, NbList nb, double* ax,
                                                        double* ay, double* az) {
-    static_assert(MIXED || !SPLIT, "the FP64 sum is serial");
     const int kk = blockIdx.x * blockDim.x + threadIdx.x;
     const bool on = kk < c.n && s.bc[kk] != BC_IGNORED;
     if (!SPLIT && !on) return;
     const int k = SPLIT ? min(kk, c.n - 1) : kk;
     // SPLIT: warp y takes every kListWarps-th group of four entries; the terms of 32
     // entries meet in shared memory, where one warp per component adds them in list
-    // order (the same bits; mixed precision only)
+    // order (the same bits)
+    constexpr int D = PLANAR ? 2 : 3;
     __shared__ double s_min[SPLIT ? kListWarps : 1][32];
-    __shared__ float4 s_term[SPLIT ? 4 * kListWarps : 1][32];
+    __shared__ float4 s_term[SPLIT && MIXED ? 4 * kListWarps : 1][32];
+    __shared__ double s_term64[SPLIT && !MIXED ? 4 * kListWarps : 1][D][32];
     __shared__ float s_sum[SPLIT ? 3 : 1][32];
+    __shared__ double s_sum64[SPLIT ? 3 : 1][32];
     const int lane = threadIdx.x & 31;
     const int q_first = SPLIT ? 4 * threadIdx.y : 0, q_step = SPLIT ? 4 * kListWarps : 4;
     const int np = nb.n_pad, m = on ? nb.cnt[k] : 0;
@@ -1064,9 +1102,9 @@ __global__ void __launch_bounds__(kThreads) k_gradient(Consts c, StateBuf s, NbL
     const double xi = s.x[k], yi = s.y[k], zi = PLANAR ? 0.0 : s.z[k];
     if (!MIXED) {
         double gx = 0.0, gy = 0.0, gz = 0.0;
-        for (int q0 = 0; q0 < m; q0 += 4) {
+        auto terms = [&](int q0, double (&tx)[4], double (&ty)[4], double (&tz)[4]) {
             int j[4];
-            double dist[4], w[4], dp[4], tx[4], ty[4], tz[4];
+            double dist[4], w[4], dp[4];
             bool in[4];
 #pragma unroll
             for (int t = 0; t < 4; t++) {
@@ -1092,12 +1130,46 @@ __global__ void __launch_bounds__(kThreads) k_gradient(Consts c, StateBuf s, NbL
                 if (!PLANAR) tz[t] = ddiv(dmul(dmul(dsub(tz[t], zi), dp[t]), w[t]), d2);
             }
 #pragma unroll
-            for (int t = 0; t < 4; t++) {
-                if (!in[t]) continue;
-                gx = dadd(gx, tx[t]);
-                gy = dadd(gy, ty[t]);
-                if (!PLANAR) gz = dadd(gz, tz[t]);
+            for (int t = 0; t < 4; t++)
+                if (!in[t]) tx[t] = ty[t] = tz[t] = 0.0;  // adds nothing
+        };
+        double tx[4], ty[4], tz[4];
+        if constexpr (!SPLIT) {
+            for (int q0 = 0; q0 < m; q0 += 4) {
+                terms(q0, tx, ty, tz);
+#pragma unroll
+                for (int t = 0; t < 4; t++) {
+                    gx = dadd(gx, tx[t]);
+                    gy = dadd(gy, ty[t]);
+                    if (!PLANAR) gz = dadd(gz, tz[t]);
+                }
             }
+        } else {
+            const int mine = fluid ? m : 0, wmax = __reduce_max_sync(0xffffffffu, mine), row = threadIdx.y;
+            double sum = 0.0;
+            for (int q0 = 0; q0 < wmax; q0 += 4 * kListWarps) {
+#pragma unroll
+                for (int t = 0; t < 4; t++) tx[t] = ty[t] = tz[t] = 0.0;
+                if (q0 + q_first < mine) terms(q0 + q_first, tx, ty, tz);
+#pragma unroll
+                for (int t = 0; t < 4; t++) {
+                    s_term64[q_first + t][0][lane] = tx[t];
+                    s_term64[q_first + t][1][lane] = ty[t];
+                    if (!PLANAR) s_term64[q_first + t][D - 1][lane] = tz[t];
+                }
+                __syncthreads();
+                if (row < D) {
+#pragma unroll 8
+                    for (int q = 0; q < 4 * kListWarps; q++) sum = dadd(sum, s_term64[q][row][lane]);
+                }
+                __syncthreads();
+            }
+            if (row < 3) s_sum64[row][lane] = sum;
+            __syncthreads();
+            if (row != 0 || !fluid) return;
+            gx = s_sum64[0][lane];
+            gy = s_sum64[1][lane];
+            gz = s_sum64[2][lane];
         }
         gx = dmul(gx, c.grad_scale);
         gy = dmul(gy, c.grad_scale);
@@ -1233,7 +1305,7 @@ __global__ void k_number_density(Consts c, StateBuf s) {
 
 void launch_explicit(const Consts& c, const StateBuf& in, const StateBuf& out,
                      const SortScratch& sc, int mixed, DevStats* ds, cudaStream_t st) {
-    const bool split = mixed && c.n <= kRowSplit;
+    const bool split = c.n <= kRowSplit;
     auto launch = [&](auto kernel, int rows) {
         const dim3 block = split ? dim3(32, rows) : dim3(block_threads(c.n));
         kernel<<<split ? (c.n + 31) / 32 : block_count(c.n), block, 0, st>>>(c, in, out, sc.skey, sc.cell_start, sc.key,
@@ -1241,11 +1313,12 @@ void launch_explicit(const Consts& c, const StateBuf& in, const StateBuf& out,
         ++g_launches;
     };
     if (c.planar)
-        launch(split ? k_explicit<true, true, true> : (mixed ? k_explicit<true, true, false> : k_explicit<true, false, false>),
+        launch(mixed ? (split ? k_explicit<true, true, true> : k_explicit<true, true, false>)
+                     : (split ? k_explicit<true, false, true> : k_explicit<true, false, false>),
                kRows<true>);
     else
-        launch(split ? k_explicit<false, true, true>
-                     : (mixed ? k_explicit<false, true, false> : k_explicit<false, false, false>),
+        launch(mixed ? (split ? k_explicit<false, true, true> : k_explicit<false, true, false>)
+                     : (split ? k_explicit<false, false, true> : k_explicit<false, false, false>),
                kRows<false>);
 }
 
@@ -1347,18 +1420,19 @@ void launch_pressure_post(const Consts& c, const StateBuf& s, const NbList& nb, 
     int g = block_count(c.n);
     k_pressure_out<<<g, block_threads(c.n), 0, st>>>(c.n, x, s.p, s.pf, s.id, x_prev, ds);
     ++g_launches;
-    const bool split = mixed && c.n <= kRowSplit;
+    const bool split = c.n <= kRowSplit;
     auto gradient = [&](auto kernel) {
         const dim3 block = split ? dim3(32, kListWarps) : dim3(block_threads(c.n));
         kernel<<<split ? (c.n + 31) / 32 : g, block, 0, st>>>(c, s, nb, ax, ay, az);
         ++g_launches;
     };
     if (c.planar) {
-        gradient(split ? k_gradient<true, true, true> : (mixed ? k_gradient<true, true, false> : k_gradient<true, false, false>));
+        gradient(mixed ? (split ? k_gradient<true, true, true> : k_gradient<true, true, false>)
+                       : (split ? k_gradient<true, false, true> : k_gradient<true, false, false>));
         k_move2<true><<<g, block_threads(c.n), 0, st>>>(c, s, ax, ay, az, ds);
     } else {
-        gradient(split ? k_gradient<false, true, true>
-                       : (mixed ? k_gradient<false, true, false> : k_gradient<false, false, false>));
+        gradient(mixed ? (split ? k_gradient<false, true, true> : k_gradient<false, true, false>)
+                       : (split ? k_gradient<false, false, true> : k_gradient<false, false, false>));
         k_move2<false><<<g, block_threads(c.n), 0, st>>>(c, s, ax, ay, az, ds);
     }
     ++g_launches;
