@@ -1,7 +1,7 @@
 """The mixed solver's split V-cycle over its forms: one cluster (every level in
 every block's shared memory), grid-wide with shared coarse levels, patches that
 do not fit and live in global memory (two bodies of water at the ends of a very
-wide domain), and the streaming form above 300,000 rows.  Against the FP64 solver
+wide domain), and the streaming form above 150,000 rows.  Against the FP64 solver
 from the same state: the mixed solve stops at a relative residual of 1e-10 and
 its FP32 sums round at 6e-8, so pressures agree to 1e-6 and surface flags are
 identical.
