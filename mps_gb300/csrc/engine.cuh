@@ -359,6 +359,7 @@ struct BatchSolve {
     int32_t* gsize = nullptr;       // per scene: blocks in its group
     unsigned int* bars = nullptr;   // per scene: barrier counter (128-byte stride)
     int32_t block = 0, grid = 0;
+    int32_t smem = 0;               // dynamic shared memory of a block
     double alpha = 0.0;
     std::vector<int32_t> group_blocks;
 };

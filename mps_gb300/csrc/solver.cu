@@ -452,48 +452,115 @@ __device__ __forceinline__ uint32_t ldg_once(const uint32_t* p) {
 }
 
 // FP32 SELL row (rows without a compact form): int32 columns of the FP64
-// matrix, FP32 values in the quad layout.
+// matrix, FP32 values in the quad layout.  One running sum in the order of the
+// neighbour list; two groups of four entries' loads and gathers at a time
+// (padding adds 0, the columns past the slice's width are not set).
 __device__ __forceinline__ float spmv32_sell_row(const Ppe& A, int K, int row,
                                                  const float* __restrict__ u, float ui) {
-    const int sl = row >> 5, lane = row & 31;
-    const int w = __ldg(A.slice_w + sl);
-    const int32_t* cp = A.col + (size_t)sl * K * 32 + lane;
-    const float* vq = A.val32 + qsell_index(row, 0, K);
+    const int w = __ldg(A.slice_w + (row >> 5)), groups = (w + 3) >> 2;
+    const int32_t* cp = A.col + (size_t)(row >> 5) * K * 32 + (row & 31);
+    const float4* vq = reinterpret_cast<const float4*>(A.val32) + (qsell_index(row, 0, K) >> 2);
     float s = 0.f;
-    for (int m = 0; m < w; m++)
-        s = fmaf(__ldg(vq + (m >> 2) * 128 + (m & 3)), __ldca(u + __ldg(cp + m * 32)) - ui, s);
+    for (int g = 0; g < groups; g += 2) {
+        int c[8];
+        float x[8];
+        const float4 a = ldg_once(vq + g * 32),
+                     b = g + 1 < groups ? ldg_once(vq + (g + 1) * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int t = 0; t < 8; t++) c[t] = 4 * g + t < w ? __ldg(cp + (4 * g + t) * 32) : row;
+#pragma unroll
+        for (int t = 0; t < 8; t++) x[t] = __ldca(u + c[t]) - ui;
+        s = fmaf(a.x, x[0], s);
+        s = fmaf(a.y, x[1], s);
+        s = fmaf(a.z, x[2], s);
+        s = fmaf(a.w, x[3], s);
+        s = fmaf(b.x, x[4], s);
+        s = fmaf(b.y, x[5], s);
+        s = fmaf(b.z, x[6], s);
+        s = fmaf(b.w, x[7], s);
+    }
     return s;
 }
 
-// Groups [g0, g1) of four entries of such a row, two groups' loads and gathers
-// at a time.
-__device__ __forceinline__ float sell_part_sum(const Ppe& A, int K, int row, int w, int g0, int g1,
-                                               const float* __restrict__ u, float ui) {
-    const int32_t* cp = A.col + (size_t)(row >> 5) * K * 32 + (row & 31);
+// Warps that share a slice of such rows: while a scene leaves most warps without a
+// slice, a row by one thread is a chain of ten or more trips to L1 and L2.
+__host__ __device__ __forceinline__ int row_parts(int nslices, int64_t warps) {
+    int parts = 8;
+    while (parts > 1 && (int64_t)parts * nslices > warps) parts >>= 1;
+    return parts;
+}
+// Entries per warp and round of a shared row, and the block's room for their values
+// and differences.
+constexpr int kPartTerms = 16;
+constexpr int terms_smem(int block) { return block * kPartTerms * (int)sizeof(float2); }
+
+// The same sum by `parts` warps: they gather the entries' differences, groups of four
+// dealt in turn, and the slice's warp `lead` adds the terms in list order, so that the
+// row has the same bits for any number of warps (a sum per warp, added afterwards,
+// moved velocities of a 3-D step by 4e-8).  The serial chain of ~100 additions and its
+// barrier take 0.5 of the 11.5 us of an inner iteration at 17,343 rows (a sum per warp:
+// 11.0).  All threads of the block; the sum is the lead warp's.  w: the row's width, 0
+// for a thread without a row; t: the slice's terms.
+__device__ __forceinline__ float shared_row_sum(const Ppe& A, int K, int row, int w, int part, int parts, bool lead,
+                                                const float* __restrict__ u, float ui, float2* t) {
+    const int lane = threadIdx.x & 31, groups = (w + 3) >> 2, round = parts * (kPartTerms / 4);
+    const int32_t* cp = A.col + (size_t)(row >> 5) * K * 32 + lane;
     const float4* vq = reinterpret_cast<const float4*>(A.val32) + (qsell_index(row, 0, K) >> 2);
-    float s0 = 0.f, s1 = 0.f;
-    for (int g = g0; g < g1; g += 2) {
-        int c[8];
-        float x[8];
-        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 a = ldg_once(vq + g * 32), b = g + 1 < g1 ? ldg_once(vq + (g + 1) * 32) : zero;
+    t += lane;
+    float s = 0.f;
+    for (int g0 = 0;; g0 += round) {
 #pragma unroll
-        for (int t = 0; t < 8; t++) {
-            const int m = 4 * g + t;  // (the columns past the slice's width are not set)
-            c[t] = m < w && m < 4 * g1 ? __ldg(cp + m * 32) : row;
+        for (int h = 0; h < kPartTerms / 8; h++) {
+            const int ga = g0 + part + 2 * h * parts, gb = ga + parts;
+            if (ga >= groups) break;
+            int c[8];
+            float x[8];
+            const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 a = ldg_once(vq + ga * 32), b = gb < groups ? ldg_once(vq + gb * 32) : zero;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const int m = 4 * (q < 4 ? ga : gb) + (q & 3);
+                c[q] = m < w ? __ldg(cp + m * 32) : row;
+            }
+#pragma unroll
+            for (int q = 0; q < 8; q++) x[q] = __ldca(u + c[q]) - ui;
+            float2* ta = t + (ga - g0) * 128;
+            ta[0] = make_float2(a.x, x[0]);
+            ta[32] = make_float2(a.y, x[1]);
+            ta[64] = make_float2(a.z, x[2]);
+            ta[96] = make_float2(a.w, x[3]);
+            if (gb < groups) {
+                float2* tb = t + (gb - g0) * 128;
+                tb[0] = make_float2(b.x, x[4]);
+                tb[32] = make_float2(b.y, x[5]);
+                tb[64] = make_float2(b.z, x[6]);
+                tb[96] = make_float2(b.w, x[7]);
+            }
         }
+        const int more = __syncthreads_or(g0 + round < groups);
+        if (lead) {
+            // (the next eight terms' loads behind this eight's additions)
+            const int m = min(w - 4 * g0, 4 * round);
+            float2 a[8], b[8];
+            auto load = [&](float2 (&v)[8], int q0) {
 #pragma unroll
-        for (int t = 0; t < 8; t++) x[t] = __ldca(u + c[t]) - ui;
-        s0 = fmaf(a.x, x[0], s0);
-        s1 = fmaf(a.y, x[1], s1);
-        s0 = fmaf(a.z, x[2], s0);
-        s1 = fmaf(a.w, x[3], s1);
-        s0 = fmaf(b.x, x[4], s0);
-        s1 = fmaf(b.y, x[5], s1);
-        s0 = fmaf(b.z, x[6], s0);
-        s1 = fmaf(b.w, x[7], s1);
+                for (int q = 0; q < 8; q++) v[q] = q0 + q < m ? t[(q0 + q) * 32] : make_float2(0.f, 0.f);
+            };
+            auto add = [&](const float2 (&v)[8]) {
+#pragma unroll
+                for (int q = 0; q < 8; q++) s = fmaf(v[q].x, v[q].y, s);
+            };
+            load(a, 0);
+            for (int q0 = 0; q0 < m; q0 += 16) {
+                load(b, q0 + 8);
+                add(a);
+                load(a, q0 + 16);
+                add(b);
+            }
+        }
+        if (!more) return s;
+        __syncthreads();
     }
-    return s0 + s1;
 }
 
 // Compact FP32 row: per group of four entries one 16-byte value word and one
@@ -616,11 +683,6 @@ __device__ __forceinline__ void compact_pair(const Ppe& A, const MatFree& mf, in
 __device__ __forceinline__ void off_rows(const Ppe& A, const MatFree& mf, int K, int i, int i2,
                                          const float* __restrict__ v, float vi, float vi2, float& o,
                                          float& o2) {
-    if (!mf.enabled) {
-        o = spmv32_sell_row(A, K, i, v, vi);
-        o2 = i2 >= 0 ? spmv32_sell_row(A, K, i2, v, vi2) : 0.f;
-        return;
-    }
     const int j2 = i2 >= 0 ? i2 : i;
     const int8_t fa = mf.sell_row[i], fb = mf.sell_row[j2];
     const int wa = __ldg(A.slice_w + (i >> 5)), wb = __ldg(A.slice_w + (j2 >> 5));
@@ -1484,11 +1546,12 @@ __device__ __forceinline__ bool mg_vcycle(const Mg& mg, uint32_t& swp, const Ppe
 }
 
 // The mixed-precision solve of one scene by one group of BS-thread blocks
-// (the whole grid for a single scene, or one scene's share of a batch).
+// (the whole grid for a single scene, or one scene's share of a batch).  terms:
+// terms_smem(BS) bytes of shared memory if a 3-D scene's warps share rows.
 template <int BS>
 __device__ __forceinline__ void solve_mixed(const Ppe& A, const MatFree& mf, const Mg& mg,
                                             const Krylov& kv, const SolveArgs& a, DevStats* ds,
-                                            GridBar& gb) {
+                                            GridBar& gb, float2* __restrict__ terms) {
     if (*(volatile int32_t*)&ds->status & ST_ASYMMETRIC) {  // the reference exits here
         if (gb.rank == 0 && threadIdx.x == 0) {
             ds->cg_iterations = 0;
@@ -1599,35 +1662,28 @@ __device__ __forceinline__ void solve_mixed(const Ppe& A, const MatFree& mf, con
                 }
             }
             if (!mf.enabled) {
-                // rows without the compact form (3-D scenes: ~100 entries a
-                // row).  A small scene leaves most warps without a row, and a
-                // row by one thread is a chain of dependent gathers: `parts`
-                // warps share a slice, each with a run of its groups of four
-                // entries, and the first adds their sums in order.
+                // rows without the compact form (3-D scenes: ~100 entries a row): one
+                // slice per warp in turn, or `parts` warps for each of the block's slices
+                // (which then fit one pass)
                 constexpr int kW = BS / 32;
                 const int warp = threadIdx.x >> 5;
-                int parts = 8;
-                while (parts > 1 && (int64_t)parts * a.nslices > (int64_t)gb.size * kW) parts >>= 1;
-                const int per = kW / parts, part = warp & (parts - 1);
+                const int parts = row_parts(a.nslices, (int64_t)gb.size * kW), per = kW / parts;
+                const int own = warp / parts, part = warp & (parts - 1);
+                // (the lead warps of a block's slices on different SM quarters)
+                const bool lead = parts == 1 || part == (parts == 2 ? (own >> 1) & 1 : own & 3);
                 const int mine = (a.nslices - gb.rank + gb.size - 1) / gb.size;  // the group's slices of this block
-                __shared__ float s_part[kW][32];
                 for (int q0 = 0; q0 < mine; q0 += per) {
-                    const int q = q0 + warp / parts;
+                    const int q = q0 + own;
                     const int i = (q * gb.size + gb.rank) * 32 + lane;
                     const bool row = q < mine && i < a.n;
-                    float ui = 0.f, o = 0.f;
-                    if (row) {
-                        ui = __ldcg(kv.u32 + i);
-                        const int w = __ldg(A.slice_w + (i >> 5)), groups = (w + 3) >> 2;
-                        o = sell_part_sum(A, a.K, i, w, groups * part / parts, groups * (part + 1) / parts, kv.u32, ui);
-                    }
-                    if (parts > 1) {
-                        s_part[warp][lane] = o;
-                        __syncthreads();
-                        if (part == 0)
-                            for (int t = 1; t < parts; t++) o += s_part[warp + t][lane];
-                    }
-                    if (row && part == 0) {
+                    const float ui = row ? __ldcg(kv.u32 + i) : 0.f;
+                    float o = 0.f;
+                    if (parts > 1)
+                        o = shared_row_sum(A, a.K, row ? i : 0, row ? __ldg(A.slice_w + (i >> 5)) : 0, part, parts, lead,
+                                           kv.u32, ui, terms + own * parts * kPartTerms * 32);
+                    else if (row)
+                        o = spmv32_sell_row(A, a.K, i, kv.u32, ui);
+                    if (row && lead) {
                         const float dg = A.diag32[i], rv = kv.r32[i];
                         const float w = dg > 0.f ? fmaf(A.rsum32[i], ui, o) : 0.f;
                         kv.w32[i] = w;
@@ -1635,7 +1691,6 @@ __device__ __forceinline__ void solve_mixed(const Ppe& A, const MatFree& mf, con
                         acc_prod(dl, w, ui);
                         acc_prod(rr, rv, rv);
                     }
-                    if (parts > 1) __syncthreads();
                 }
             }
             const F2 v3[3] = {g, dl, rr};
@@ -1715,8 +1770,9 @@ __device__ __forceinline__ void solve_mixed(const Ppe& A, const MatFree& mf, con
 __global__ void __launch_bounds__(kMixedBlock, 1)
     k_cg_mixed(__grid_constant__ const Ppe A, __grid_constant__ const MatFree mf, __grid_constant__ const Mg mg,
                __grid_constant__ const Krylov kv, __grid_constant__ const SolveArgs a, DevStats* ds) {
+    extern __shared__ __align__(16) unsigned char s_dyn[];
     GridBar gb = whole_grid(kv);
-    solve_mixed<kMixedBlock>(A, mf, mg, kv, a, ds, gb);
+    solve_mixed<kMixedBlock>(A, mf, mg, kv, a, ds, gb, reinterpret_cast<float2*>(s_dyn));
 }
 
 // ----------------------------------------------- overlapped additive cycle
@@ -2044,9 +2100,9 @@ template <int NV>
 __global__ void __launch_bounds__(kMixedBlock, 1)
     k_cg_mixed_ov(__grid_constant__ const Ppe A, __grid_constant__ const MatFree mf, __grid_constant__ const Mg mg,
                   __grid_constant__ const Krylov kv, __grid_constant__ const SolveArgs a, DevStats* ds, int floats) {
-    extern __shared__ float s_levels[];
+    extern __shared__ __align__(16) unsigned char s_dyn[];
     GridBar gb = whole_grid(kv);
-    solve_mixed_overlap<kMixedBlock, NV, false>(A, mf, mg, kv, a, ds, gb, s_levels, floats);
+    solve_mixed_overlap<kMixedBlock, NV, false>(A, mf, mg, kv, a, ds, gb, reinterpret_cast<float*>(s_dyn), floats);
 }
 
 // The same solve by one cluster, for small scenes whose level 1 fits a
@@ -2054,9 +2110,10 @@ __global__ void __launch_bounds__(kMixedBlock, 1)
 __global__ void __launch_bounds__(kMixedBlock, 1)
     k_cg_mixed_cl(__grid_constant__ const Ppe A, __grid_constant__ const MatFree mf, __grid_constant__ const Mg mg,
                   __grid_constant__ const Krylov kv, __grid_constant__ const SolveArgs a, DevStats* ds, int floats) {
-    extern __shared__ float s_levels[];
+    extern __shared__ __align__(16) unsigned char s_dyn[];
     GridBar gb = whole_grid(kv);
-    solve_mixed_overlap<kMixedBlock, kCycleThreads, true>(A, mf, mg, kv, a, ds, gb, s_levels, floats);
+    solve_mixed_overlap<kMixedBlock, kCycleThreads, true>(A, mf, mg, kv, a, ds, gb, reinterpret_cast<float*>(s_dyn),
+                                                          floats);
     cluster_barrier();  // no block leaves while another may still store into its slots
 }
 
@@ -2083,15 +2140,16 @@ __global__ void __launch_bounds__(BS, MINB) k_cg_mixed_batched(const SceneSolve*
         reinterpret_cast<int32_t*>(&s)[k] = reinterpret_cast<const int32_t*>(scenes + m.x)[k];
     __syncthreads();
     GridBar gb{bars + 32 * m.x, 0u, 0, m.y, gsize[m.x], s.kv.partials};
+    extern __shared__ __align__(16) unsigned char s_dyn[];
     if constexpr (BS == kMixedBlock) {
         // one block per SM: the overlapped arrangement within each group
-        extern __shared__ float s_levels[];
         if (s.mg.enabled && s.mg.overlap) {
-            solve_mixed_overlap<BS, kBatchCycle, false>(s.A, s.mf, s.mg, s.kv, s.a, s.ds, gb, s_levels, floats);
+            solve_mixed_overlap<BS, kBatchCycle, false>(s.A, s.mf, s.mg, s.kv, s.a, s.ds, gb,
+                                                        reinterpret_cast<float*>(s_dyn), floats);
             return;
         }
     }
-    solve_mixed<BS>(s.A, s.mf, s.mg, s.kv, s.a, s.ds, gb);
+    solve_mixed<BS>(s.A, s.mf, s.mg, s.kv, s.a, s.ds, gb, reinterpret_cast<float2*>(s_dyn));
 }
 
 // Mixed-solver setup: FP32 values of the matrix and their compact index
@@ -2267,7 +2325,7 @@ int cluster_blocks() {
 
 void solver_setup(Krylov& k, int32_t /*n_pad*/, int device) {
     int g1 = cg64_grid(device);
-    int g2 = coop_grid((const void*)k_cg_mixed, device, kMixedBlock, 0, 1);
+    int g2 = coop_grid((const void*)k_cg_mixed, device, kMixedBlock, terms_smem(kMixedBlock), 1);
     int g3 = std::min(coop_grid((const void*)k_cg_mixed_ov<kCycleThreads>, device, kMixedBlock, kSplitSmem, 1),
                       coop_grid((const void*)k_cg_mixed_ov<kStreamCycle>, device, kMixedBlock, kStreamSmem, 1));
     k.grid = std::min({g1, g2, g3});
@@ -2340,11 +2398,14 @@ namespace {
 // 3.3 ms in its plain form; 64 scenes of 2,000 - 60,000, where every SM streams
 // all the time: 18.9 against 16.7), the others the plain form; the autotuner
 // times both.
-size_t batch_smem(int block) { return block == kMixedBlock ? kStreamSmem : 0; }
+// With a 3-D scene among them, every block has room for shared rows' terms.
+size_t batch_smem(int block, bool space) {
+    return std::max<size_t>(block == kMixedBlock ? kStreamSmem : 0, space ? terms_smem(block) : 0);
+}
 
 template <int BS, int MINB>
 int resident_grid(int device) {
-    return coop_grid((const void*)k_cg_mixed_batched<BS, MINB>, device, BS, batch_smem(BS), MINB);
+    return coop_grid((const void*)k_cg_mixed_batched<BS, MINB>, device, BS, batch_smem(BS, true), MINB);
 }
 }  // namespace
 
@@ -2415,6 +2476,8 @@ int batch_solve_setup(const std::vector<BatchScene>& scenes, int block, double a
     cudaMemcpy(b.gsize, gs.data(), sizeof(int32_t) * ns, cudaMemcpyHostToDevice);
     b.n_scenes = ns;
     b.block = block;
+    b.smem = (int32_t)batch_smem(block, std::any_of(scenes.begin(), scenes.end(),
+                                                    [](const BatchScene& q) { return !q.mf.enabled; }));
     b.grid = (int32_t)bmap.size();
     b.alpha = alpha;
     b.group_blocks = gs;
@@ -2434,13 +2497,13 @@ void launch_solve_mixed_batched(const BatchSolve& b, cudaStream_t st) {
     const int2* bm = b.bmap;
     const int32_t* gs = b.gsize;
     unsigned int* bars = b.bars;
-    int floats = (int)batch_smem(b.block) / 4;
+    int floats = b.smem / 4;
     void* args[] = {&sc, &bm, &gs, &bars, &floats};
     cudaMemsetAsync(b.bars, 0, sizeof(unsigned int) * 32 * b.n_scenes, st);
     const void* fn = b.block == 256   ? (const void*)k_cg_mixed_batched<256, 4>
                      : b.block == 512 ? (const void*)k_cg_mixed_batched<512, 2>
                                       : (const void*)k_cg_mixed_batched<1024, 1>;
-    cudaLaunchCooperativeKernel(fn, dim3(b.grid), dim3(b.block), args, batch_smem(b.block), st);
+    cudaLaunchCooperativeKernel(fn, dim3(b.grid), dim3(b.block), args, b.smem, st);
     ++g_launches;
 }
 
@@ -2484,7 +2547,9 @@ void launch_solve_mixed(const Consts& c, const Ppe& A, const MatFree& mf, const 
         ++g_launches;
         return;
     }
-    cudaLaunchCooperativeKernel((const void*)k_cg_mixed, dim3(k.grid), dim3(kMixedBlock), args, 0, st);
+    const bool shared_rows = !mf.enabled && row_parts(a.nslices, (int64_t)k.grid * (kMixedBlock / 32)) > 1;
+    cudaLaunchCooperativeKernel((const void*)k_cg_mixed, dim3(k.grid), dim3(kMixedBlock), args,
+                                shared_rows ? terms_smem(kMixedBlock) : 0, st);
     ++g_launches;
 }
 
