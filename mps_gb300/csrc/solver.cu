@@ -23,6 +23,7 @@
 #include <utility>
 #include <vector>
 
+#include "cellpack.cuh"
 #include "devutil.cuh"
 #include "engine.cuh"
 
@@ -976,7 +977,8 @@ struct CyclePatch {
     // (first float, -1: read from global memory): the dense inverse; per level
     // > lr the restriction weights of its cells, dn = [16 weights, invd, (x, y)]
     // by position in the level's list; per level the stencils of the block's
-    // cells, up = [9 taps, invd, (x, y)] by position in the block's list.  The
+    // cells, up = [9 taps, invd, (x, y)] by position in the block's list (neither on
+    // a level too wide for packed coordinates).  The
     // cycle's phases are short chains of dependent loads, several times as
     // long from L2 behind the operator pass's traffic as from here.
     int dense, dn[kMgMaxLevels], up[kMgMaxLevels];
@@ -1102,24 +1104,24 @@ __device__ __forceinline__ void plan_patches(const Ppe& A, const Mg& mg, const M
     for (int l = mg.nlev - 1; l >= 1; l--) {
         const MgLevel &L = mg.lev[l], &C = mg.lev[l + 1];
         const int na = __ldg(mg.nact + l + 1), nc = C.nx * C.ny, n1 = L.nx * L.ny;
-        const int dn = l >= mg.lred ? take(18 * na) : -1;
+        const int dn = l >= mg.lred && packs(C.nx, C.ny) ? take(18 * na) : -1;
         if (dn >= 0)
             for (int q = tid; q < na; q += BS) {
                 const int I = __ldg(C.act + q);
 #pragma unroll
                 for (int k = 0; k < 16; k++) sm[dn + k * na + q] = ldc(C.rw, (size_t)k * nc + I);
                 sm[dn + 16 * na + q] = ldc(C.invd, I);
-                sm[dn + 17 * na + q] = __int_as_float((I / C.ny) << 16 | (I % C.ny));
+                sm[dn + 17 * na + q] = __uint_as_float(pack_cell(I / C.ny, I % C.ny));
             }
         const int cnt = cp.count[l];
-        const int up = cp.list[l] >= 0 ? take(11 * cnt) : -1;
+        const int up = cp.list[l] >= 0 && packs(L.nx, L.ny) ? take(11 * cnt) : -1;
         if (up >= 0)
             for (int q = tid; q < cnt; q += BS) {
                 const int I = list[cp.list[l] + q];
 #pragma unroll
                 for (int d = 0; d < 9; d++) sm[up + d * cnt + q] = ldc(L.st, (size_t)d * n1 + I);
                 sm[up + 9 * cnt + q] = ldc(L.invd, I);
-                sm[up + 10 * cnt + q] = __int_as_float((I / L.ny) << 16 | (I % L.ny));
+                sm[up + 10 * cnt + q] = __uint_as_float(pack_cell(I / L.ny, I % L.ny));
             }
         if (tid == 0) {
             cp.dn[l + 1] = dn;
@@ -1159,8 +1161,8 @@ __device__ __forceinline__ void smooth_level(const Mg& mg, int l, const CyclePat
     if (cp.up[l] >= 0) {
         const float* W = sm + cp.up[l];
         for (int q = threadIdx.x; q < cnt; q += NT) {
-            const int xy = __float_as_int(W[10 * cnt + q]);
-            const int x = xy >> 16, y = xy & 0xffff, I = x * L.ny + y;
+            const uint32_t xy = __float_as_uint(W[10 * cnt + q]);
+            const int x = cell_x(xy), y = cell_y(xy), I = x * L.ny + y;
             t[I] = smooth_cell(mg, L, cny, corr, x, y, W[9 * cnt + q], r(I), [&](int d) { return W[d * cnt + q]; }, e);
         }
     } else {
@@ -1232,8 +1234,8 @@ __device__ __forceinline__ bool mg_split_cycle(const Mg& mg, GridBar& gb, DevSta
         if (cp.dn[l + 1] >= 0) {
             const float* W = sm + cp.dn[l + 1];
             for (int q = tid; q < na; q += NT) {
-                const int xy = __float_as_int(W[17 * na + q]);
-                cell(xy >> 16, xy & 0xffff, W[16 * na + q], [&](int k) { return W[k * na + q]; });
+                const uint32_t xy = __float_as_uint(W[17 * na + q]);
+                cell(cell_x(xy), cell_y(xy), W[16 * na + q], [&](int k) { return W[k * na + q]; });
             }
         } else {
             for (int q = tid; q < na; q += NT) {
