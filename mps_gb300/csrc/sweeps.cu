@@ -485,9 +485,11 @@ __global__ void __launch_bounds__(kThreads) k_coll_wave(Consts c, StateBuf s, co
                                                         const int32_t* __restrict__ cnt_by_id,
                                                         const int32_t* __restrict__ base_by_id, CollWork cw,
                                                         DevStats* ds) {
-    const int32_t total = min(*total_p, cap);
-    if (blockIdx.x == 0 && threadIdx.x == 0) ds->n_cand = *total_p;
-    if (total == 0) return;
+    const int32_t total = *total_p;
+    if (blockIdx.x == 0 && threadIdx.x == 0) ds->n_cand = total;
+    // more pairs than the table holds: those of the first particle that did not fit are
+    // not set, and the step reports the overflow (k_coll_write)
+    if (total == 0 || total > cap) return;
     const double inv_rho = ddiv(1.0, c.rho);
     if (cw.serial || *(volatile int32_t*)(cw.ctl + 1)) {
         // the serial pass: every pair in order by one thread (verification mode, or
