@@ -345,7 +345,11 @@ int mps_number_density_static(const mps_params* prm, int32_t n, const double* d_
  * blocks are split into a group per scene (each group converges on its own
  * scene's tolerance).  The solve launch's block size (256/512/1024) and the
  * exponent alpha of its group-size model (blocks ~ rows^alpha) are picked by
- * an autotuner on the first step unless set with mps_batch_set_launch.
+ * an autotuner on the first step unless set with mps_batch_set_launch.  Blocks
+ * of 1,024 threads order the multigrid iteration another way than smaller ones
+ * (mps_set_multigrid, modes 1 and 4), so pressures depend on the autotuner's
+ * choice at the level of the solve's tolerance: a launch set by the caller
+ * gives the same results in every process.
  * ------------------------------------------------------------------------ */
 typedef struct mps_batch mps_batch;
 

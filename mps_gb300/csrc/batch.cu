@@ -326,7 +326,7 @@ int mps_batch_step(mps_batch* b, int32_t n_steps, mps_step_stats* stats, float* 
             mps_step_stats* o = stats ? &stats[s] : &tmp;
             e->last_step_graphed = graphed ? 1 : 0;
             e->step_launches = graphed ? b->graph_launches : 0;
-            int rc = engine_collect(e, o);
+            int rc = engine_collect(e, o, !batch_overlaps(b->block));
             o->ms_step = b->last_ms;
             o->ms_solve = 0.f;
             if (rc && !first_rc) first_rc = rc;

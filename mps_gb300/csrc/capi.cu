@@ -341,15 +341,16 @@ void enqueue_step(mps_engine* e, bool do_export) {
 // refinement the FP64 residual (12 B/entry + 36 B/row) and once the FP32
 // operator setup (17 B/entry + 28 B/row written and read; 36 B/row more for
 // the row-to-cell sums of the multigrid modes, from which level 1's stencils
-// are summed).
-double solve_bytes(const mps_engine* e, const DevStats& h) {
+// are summed).  plain: mode 1 ran in its plain form (batch launches of 256 and 512
+// threads).
+double solve_bytes(const mps_engine* e, const DevStats& h, bool plain) {
     const double nnz = (double)h.nnz_off, n = (double)e->n, it = (double)h.cg_iterations;
     if (e->precision == MPS_PRECISION_FP64) return it * (12.0 * nnz + 116.0 * n) + 36.0 * n;
     const Mg g = active_mg(e);
     const bool mg = g.enabled != 0;
     const bool additive = mg && g.additive;
     const double ent = e->c.planar ? 5.0 : 8.0;
-    const double row_add = g.smooth ? 165.0 : g.overlap ? 145.0 : 85.0;
+    const double row_add = g.smooth ? 165.0 : g.overlap && !plain ? 145.0 : 85.0;
     double per_it = !mg ? (ent * nnz + 69.0 * n)
                         : additive ? (ent * nnz + row_add * n) : (3.0 * ent * nnz + 155.0 * n);
     if (mg)
@@ -360,7 +361,7 @@ double solve_bytes(const mps_engine* e, const DevStats& h) {
     return it * per_it + ref * (12.0 * nnz + 36.0 * n) + setup;
 }
 
-void fill_stats(mps_engine* e, mps_step_stats* out) {
+void fill_stats(mps_engine* e, mps_step_stats* out, bool plain = false) {
     DevStats& h = *e->hs;
     double cour = 0.0;
     unsigned long long b = h.courant_bits;
@@ -390,7 +391,7 @@ void fill_stats(mps_engine* e, mps_step_stats* out) {
     out->nnz_offdiag = (int64_t)h.nnz_off;
     out->max_neighbors = h.max_neighbors;
     out->graph_replayed = e->last_step_graphed;
-    out->solve_bytes = solve_bytes(e, h);
+    out->solve_bytes = solve_bytes(e, h, plain);
 }
 
 void drop_graphs(mps_engine* e) {
@@ -1051,8 +1052,8 @@ void engine_pre_solve(mps_engine* e) { enqueue_pre_solve(e); }
 void engine_solver_setup(mps_engine* e) { enqueue_solver_setup(e); }
 void engine_post_solve(mps_engine* e, bool do_export) { enqueue_post_solve(e, do_export); }
 Mg engine_active_mg(const mps_engine* e) { return active_mg(e); }
-int engine_collect(mps_engine* e, mps_step_stats* stats) {
-    fill_stats(e, stats);
+int engine_collect(mps_engine* e, mps_step_stats* stats, bool plain) {
+    fill_stats(e, stats, plain);
     return check_status(e);
 }
 }  // namespace mpsg

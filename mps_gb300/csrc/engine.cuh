@@ -365,6 +365,8 @@ struct BatchSolve {
 };
 // Blocks of `block` threads (256, 512 or 1024) co-resident on the device.
 int batch_resident_grid(int block, int device);
+// Whether blocks of that size run mode 1 in its overlapped arrangement.
+bool batch_overlaps(int block);
 void batch_group_sizes(const std::vector<int32_t>& rows, double alpha, int grid,
                        std::vector<int32_t>& out);
 // 0 on success; 1 if the device holds fewer blocks than scenes; 2 on a CUDA error.

@@ -148,7 +148,8 @@ MPSG_HIDDEN void engine_post_solve(mps_engine* e, bool do_export);
 // The multigrid hierarchy as the mixed solver uses it (disabled if not requested).
 MPSG_HIDDEN Mg engine_active_mg(const mps_engine* e);
 // After the step's device stats reached e->hs: fills stats, returns the status.
-MPSG_HIDDEN int engine_collect(mps_engine* e, mps_step_stats* stats);
+// plain: the solve ran mode 1 in its plain form.
+MPSG_HIDDEN int engine_collect(mps_engine* e, mps_step_stats* stats, bool plain);
 // Records a phase of the running step into e->tape (adjoint.cu).
 MPSG_HIDDEN void tape_phase(mps_engine* e, TapePhase ph);
 // The reference's message for the first asymmetric pair of the last step's

@@ -2411,6 +2411,8 @@ int resident_grid(int device) {
 }
 }  // namespace
 
+bool batch_overlaps(int block) { return block == kMixedBlock; }
+
 int batch_resident_grid(int block, int device) {
     switch (block) {
         case 256: return resident_grid<256, 4>(device);
