@@ -92,7 +92,8 @@ typedef struct {
     int32_t graph_replayed;         /* 1: the step ran as one CUDA graph replay */
     double solve_bytes;             /* algorithmic HBM bytes of the pressure solve (model:
                                        every array the solver kernels stream counted once
-                                       per pass at its stored width) */
+                                       per pass at its stored width, FP64 rows that stay
+                                       in shared memory too) */
 } mps_step_stats;
 
 typedef struct mps_engine mps_engine;

@@ -324,10 +324,13 @@ void enqueue_step(mps_engine* e, bool do_export) {
 
 // Algorithmic bytes of one pressure solve: each array a solver pass streams,
 // counted once at its stored width (gathered vector entries count once, as
-// the row's own entry).  Per stored off-diagonal entry and pass: FP64 12 B
-// (column + value; the one-kernel CG streams 10, with 16-bit window indices, and
-// small scenes none), compact FP32 5 B (value + index byte).  Per row and
-// iteration: FP64 CG 116 B (8 vectors); MIXED inner iteration 69 B with the
+// the row's own entry).  Per stored off-diagonal entry and pass: FP64 CG 10 B
+// (value + 16-bit window index, made once from the column), FP64 residual 12 B
+// (column + value), compact FP32 5 B (value + index byte).  Per row and
+// iteration: FP64 CG 80 B (diagonal, its inverse, x, r and q read and written, z
+// written and read; blocks that keep their rows in shared memory, scenes of up to
+// ~60,000 rows, stream z alone and are counted like the others), and once 10 B
+// per entry and 56 B per row; MIXED inner iteration 69 B with the
 // Jacobi preconditioner; with the multigrid V-cycle, per cell of level 1
 // 72 B (segment bounds, the up pass's 9-point stencil and 8 vector words)
 // and of levels >= 2 132 B (the same plus the 4x4 restriction weights), and,
@@ -345,7 +348,7 @@ void enqueue_step(mps_engine* e, bool do_export) {
 // threads).
 double solve_bytes(const mps_engine* e, const DevStats& h, bool plain) {
     const double nnz = (double)h.nnz_off, n = (double)e->n, it = (double)h.cg_iterations;
-    if (e->precision == MPS_PRECISION_FP64) return it * (12.0 * nnz + 116.0 * n) + 36.0 * n;
+    if (e->precision == MPS_PRECISION_FP64) return it * (10.0 * nnz + 80.0 * n) + 10.0 * nnz + 56.0 * n;
     const Mg g = active_mg(e);
     const bool mg = g.enabled != 0;
     const bool additive = mg && g.additive;
