@@ -151,6 +151,8 @@ int mps_set_initial_guess(mps_engine* e, int32_t previous);
  * normally, leaving the context usable.
  * MPS_OK when all 8 gave up with that status. */
 int mps_selftest_wait_limit(int32_t* blocks_gave_up, double* seconds);
+/* The same for the exchange of the FP64 solve's blocks (polled slots). */
+int mps_selftest_exchange_limit(int32_t* blocks_gave_up, double* seconds);
 
 /* How the collision pass (src/mps.cpp:217-250) applies its candidate pairs.
  * serial = 0 (default): in parallel, each pair after exactly the earlier

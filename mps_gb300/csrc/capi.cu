@@ -804,17 +804,25 @@ int mps_set_multigrid(mps_engine* e, int32_t mode, float omega, float scale) {
     return MPS_OK;
 }
 
-int mps_selftest_wait_limit(int32_t* blocks_gave_up, double* seconds) {
+static int selftest_waits(const char* name, bool exchange, int32_t* blocks_gave_up, double* seconds) {
     int gave = 0, status = 0;
     float ms = 0.f;
     constexpr int kBlocks = 8;
-    if (selftest_wait_limit(kBlocks, &gave, &status, &ms) != 0)
-        return fail(MPS_ERR_CUDA, "mps_selftest_wait_limit: CUDA call failed");
+    if (selftest_wait_limit(kBlocks, exchange, &gave, &status, &ms) != 0)
+        return fail(MPS_ERR_CUDA, std::string(name) + ": CUDA call failed");
     if (blocks_gave_up) *blocks_gave_up = gave;
     if (seconds) *seconds = ms * 1e-3;
     if (gave != kBlocks || !(status & ST_TIMEOUT))
-        return fail(MPS_ERR_TIMEOUT, "mps_selftest_wait_limit: not every block gave up with the timeout status");
+        return fail(MPS_ERR_TIMEOUT, std::string(name) + ": not every block gave up with the timeout status");
     return MPS_OK;
+}
+
+int mps_selftest_wait_limit(int32_t* blocks_gave_up, double* seconds) {
+    return selftest_waits("mps_selftest_wait_limit", false, blocks_gave_up, seconds);
+}
+
+int mps_selftest_exchange_limit(int32_t* blocks_gave_up, double* seconds) {
+    return selftest_waits("mps_selftest_exchange_limit", true, blocks_gave_up, seconds);
 }
 
 int mps_set_collisions(mps_engine* e, int32_t serial) {

@@ -71,6 +71,7 @@ struct Exchange {
     unsigned long long* slots;
     unsigned int number;
     int rank, size;
+    long long limit = kSpinLimit64;  // polls before an exchange gives up
 };
 
 __device__ __forceinline__ void st_slot(unsigned long long* p, unsigned long long a, unsigned long long b) {
@@ -195,7 +196,7 @@ __device__ __forceinline__ bool exchange(Exchange& ex, const double (&v)[M], boo
         for (long long it = 0; __any_sync(0xffffffffu, todo != 0); it++) {
             if (it > 256) {
                 __nanosleep(16);
-                bool stop = it > kSpinLimit64;
+                bool stop = it > ex.limit;
                 if (stop) atomicOr(&ds->status, ST_TIMEOUT);
                 if ((it & 1023) == 0 && (*(volatile int*)&ds->status & ST_TIMEOUT)) stop = true;
                 if (__any_sync(0xffffffffu, stop)) {
@@ -616,6 +617,16 @@ __global__ void __launch_bounds__(BS, 1) k_cg64(Ppe A, Krylov kv, Cg64Args a, De
     }
 }
 
+// One exchange in a group that counts a block more than the launch has.
+__global__ void __launch_bounds__(512) k_selftest_exchange(unsigned long long* slots, unsigned int* gave_up,
+                                                          DevStats* ds) {
+    Exchange ex{slots, 0u, (int)blockIdx.x, (int)gridDim.x + 1, 1ll << 16};
+    double tot[2], aux[2];
+    const double v[2] = {1.0, 2.0};
+    const bool ok = exchange<2, true, 512, false>(ex, v, true, tot, aux, ds, [](int, double) { return 0.0; });
+    if (threadIdx.x == 0 && !ok) atomicAdd(gave_up, 1u);
+}
+
 // Dynamic shared memory of a block: all of an SM's but the static arrays above.
 constexpr int kSmem64 = 224 * 1024;
 // More slices per block than this: 1024 threads (their loads are in flight
@@ -641,6 +652,10 @@ int grid64(int device) {
 }
 
 }  // namespace
+
+void launch_selftest_exchange(int blocks, unsigned long long* slots, unsigned int* gave_up, DevStats* ds) {
+    k_selftest_exchange<<<blocks, 512>>>(slots, gave_up, ds);
+}
 
 int cg64_grid(int device) { return std::min(grid64<512>(device), grid64<1024>(device)); }
 

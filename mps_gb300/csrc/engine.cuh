@@ -321,12 +321,15 @@ struct Krylov {
     int32_t block;
 };
 void solver_setup(Krylov& k, int32_t n_pad, int device);
-// Runs the grid barrier with one block that never arrives on `blocks`
-// blocks; reports how many gave up, the status word and the kernel time.
-int selftest_wait_limit(int blocks, int* gave_up, int* status, float* ms);
+// Runs the grid barrier, or with `exchange` the FP64 solve's exchange, with one block
+// that never arrives on `blocks` blocks; reports how many gave up, the status word and
+// the kernel time.
+int selftest_wait_limit(int blocks, bool exchange, int* gave_up, int* status, float* ms);
 // ----------------------------------------------------------------- cg64.cu
 // Blocks the FP64 solve may use on the device (0: it does not fit).
 int cg64_grid(int device);
+// One exchange of a group of blocks + 1 (slots: 16 words per member, zeroed).
+void launch_selftest_exchange(int blocks, unsigned long long* slots, unsigned int* gave_up, DevStats* ds);
 // Blocks of its one-cluster form (0: the device runs none).
 int cg64_cluster();
 // Solves A x = b; returns through DevStats (iterations, residual, status).

@@ -2346,8 +2346,9 @@ void launch_mixed_setup(const Consts& c, const SortScratch& sc, const Ppe& A, Ma
     ++g_launches;
 }
 
-// Self-test of the bounded waits: the solver's grid barrier in a group that
-// counts one block more than the launch has, so no block can pass.  Every
+// Self-test of the bounded waits: the solver's grid barrier, or the FP64 solve's
+// exchange, in a group that counts one block more than the launch has, so no block can
+// pass.  Every
 // block gives up (at its spin limit, here 2^16 polls instead of the solver's
 // 2^23, or on the flag of the first that did), records it and ends; nothing
 // faults and nothing is left waiting.
@@ -2359,20 +2360,25 @@ __global__ void k_selftest_barrier(unsigned int* words, DevStats* ds) {
 }
 }  // namespace
 
-int selftest_wait_limit(int blocks, int* gave_up, int* status, float* ms) {
+int selftest_wait_limit(int blocks, bool exchange, int* gave_up, int* status, float* ms) {
     unsigned int* words = nullptr;
     DevStats* ds = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     int rc = 0;
-    if (cudaMalloc(&words, 2 * sizeof(unsigned int)) != cudaSuccess ||
+    // two words, then the exchange's slots
+    const size_t bytes = 64 + sizeof(unsigned long long) * 16 * (blocks + 1);
+    if (cudaMalloc(&words, bytes) != cudaSuccess ||
         cudaMalloc(&ds, sizeof(DevStats)) != cudaSuccess || cudaEventCreate(&e0) != cudaSuccess ||
         cudaEventCreate(&e1) != cudaSuccess) {
         rc = -1;
     } else {
-        cudaMemset(words, 0, 2 * sizeof(unsigned int));
+        cudaMemset(words, 0, bytes);
         cudaMemset(ds, 0, sizeof(DevStats));
         cudaEventRecord(e0);
-        k_selftest_barrier<<<blocks, 64>>>(words, ds);
+        if (exchange)
+            launch_selftest_exchange(blocks, reinterpret_cast<unsigned long long*>(words + 16), words + 1, ds);
+        else
+            k_selftest_barrier<<<blocks, 64>>>(words, ds);
         cudaEventRecord(e1);
         unsigned int h[2] = {0, 0};
         DevStats hs{};

@@ -167,8 +167,9 @@ def load(build_if_missing: bool = False):
         getattr(L, name).restype = C.c_int
     L.mps_read_csv.argtypes = [C.c_char_p, C.c_int32, P(C.c_int32), P(C.c_double), vp, vp, vp]
     L.mps_read_csv.restype = C.c_int
-    L.mps_selftest_wait_limit.argtypes = [P(C.c_int32), P(C.c_double)]
-    L.mps_selftest_wait_limit.restype = C.c_int
+    for name in ("mps_selftest_wait_limit", "mps_selftest_exchange_limit"):
+        getattr(L, name).argtypes = [P(C.c_int32), P(C.c_double)]
+        getattr(L, name).restype = C.c_int
     L.mps_check_symmetry.argtypes = [C.c_int32, vp, vp, vp, P(C.c_int32), P(C.c_int32)]
     L.mps_check_symmetry.restype = C.c_int
     L.mps_selftest_exact64.argtypes = [C.c_uint64, C.c_uint64, P(C.c_uint64)]
@@ -217,13 +218,14 @@ def read_particles_csv(path):
     return tm.value, pos, vel, typ
 
 
-def selftest_wait_limit():
-    """Runs the device-side wait-limit self-test (include/mps_gb300.h):
-    (return code, blocks that gave up, seconds)."""
+def selftest_wait_limit(exchange=False):
+    """Runs the device-side wait-limit self-test (include/mps_gb300.h) of the grid
+    barrier or of the FP64 solve's exchange: (return code, blocks that gave up, seconds)."""
     L = load()
     g = C.c_int32(0)
     sec = C.c_double(0.0)
-    rc = L.mps_selftest_wait_limit(C.byref(g), C.byref(sec))
+    fn = L.mps_selftest_exchange_limit if exchange else L.mps_selftest_wait_limit
+    rc = fn(C.byref(g), C.byref(sec))
     return rc, g.value, sec.value
 
 
