@@ -651,7 +651,7 @@ int mps_create(const mps_params* prm, int32_t n, const double* pos, const double
         e->alloc(&e->kv.s32, np) || e->alloc(&e->kv.w32, np) || e->alloc(&e->kv.x32, np) ||
         e->alloc(&e->kv.u32, np) ||
         e->alloc(&e->kv.inv_diag32, np) || e->alloc(&e->kv.barrier, 64) ||
-        e->alloc(&e->kv.totals, 8) || e->alloc(&e->mf.idx8, np * K) ||
+        e->alloc(&e->mf.idx8, np * K) ||
         e->alloc(&e->mf.sell_row, np) || e->alloc(&e->mf.rs, 3 * np) ||
         e->alloc(&e->cand_cnt, np + 1) || e->alloc(&e->cand_base, np + 2) ||
         e->alloc(&e->cw.jn, np) || e->alloc(&e->cw.jl, np * kCollJList) || e->alloc(&e->cw.ver, np) ||

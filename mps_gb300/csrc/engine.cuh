@@ -314,11 +314,9 @@ struct Krylov {
     float *r32, *p32, *s32, *w32, *x32, *u32, *inv_diag32;
     double* partials;       // 2 x grid x 8 per-block partial sums
     unsigned int* barrier;  // monotonically increasing arrival counter
-    double* totals;         // unused scratch (8 doubles)
     int32_t grid;           // cooperative grid size
     int32_t cluster;        // blocks of a one-cluster mixed solve (0: the device runs none)
     int32_t cluster64;      // the same for the FP64 solve
-    int32_t block;
 };
 void solver_setup(Krylov& k, int32_t n_pad, int device);
 // Runs the grid barrier, or with `exchange` the FP64 solve's exchange, with one block

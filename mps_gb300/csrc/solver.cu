@@ -4,9 +4,8 @@
 // cooperative kernels: one launch per solve, the
 // blocks stay resident and meet at grid barriers between the phases of an
 // iteration, and the convergence test runs on the device.  A dot product is
-// reduced per block, written as one partial per block, and summed in a fixed
-// order by the last block to reach the barrier, which publishes the total
-// before it releases the others; results are therefore run-to-run
+// reduced per block, written as one partial per block, and after the barrier
+// summed in the same order by every block; results are therefore run-to-run
 // deterministic and every block takes the same branch.
 //
 //  * MIXED (k_cg_mixed): iterative refinement.  x and the residual
@@ -34,7 +33,6 @@ namespace {
 // Single-scene solves: one 1024-thread block per SM, 152 blocks meet at
 // each grid barrier.  Batched solves (many scenes in one launch) run the same
 // code on groups of blocks, each group with its own barrier and partials.
-constexpr int kBlock = 1024;
 constexpr int kMixedBlock = 1024;  // k_cg_mixed: one block per SM
 // Polls before a barrier wait gives up: one poll (an acquire load plus the
 // back-off) takes ~0.28 us on GB300 (measured by mps_selftest_wait_limit),
@@ -140,9 +138,7 @@ __device__ __forceinline__ bool grid_sync(GridBar& gb, DevStats* ds) {
 // The two halves of that: publish_partials reduces the block's M values
 // and writes its partials into the next buffer (returned); sum_partials,
 // after a grid barrier that every block passed after publishing, sums the
-// partials in block order.  Between the two any number of phases and
-// barriers may run (the pipelined solve overlaps its reduction with the
-// preconditioner that way).
+// partials in block order.
 template <int M, int BS>
 __device__ __forceinline__ const double* publish_partials(GridBar& gb, const double (&v)[M]) {
     constexpr int kW = BS / 32;
@@ -834,13 +830,12 @@ __device__ __forceinline__ float* level1_presmooth(const Mg& mg, uint32_t swp) {
 
 // Levels lo..nlev of the V-cycle, run by the group's first block alone (they
 // are small): down smoothing + restriction, the dense coarsest solve, up
-// smoothing with the prolongation folded in.  Only block-level barriers of
-// the group NT inside; the caller brackets it with grid barriers.  Level lo's
+// smoothing with the prolongation folded in.  Only block-level barriers
+// inside; the caller brackets it with grid barriers.  Level lo's
 // r and pre-smoothing were written by the grid pass; its correction goes to
 // its t array.
-template <int NT>
 __device__ void mg_block_cycle(const Mg& mg, int lo) {
-    const int tid = threadIdx.x, nt = NT == 0 ? (int)blockDim.x : NT;
+    const int tid = threadIdx.x, nt = (int)blockDim.x;
     uint32_t bsw = 0;  // role swaps of the levels below lo in this cycle
     for (int l = lo; l < mg.nlev; l++) {
         const MgLevel L = l == lo ? mg.lev[lo] : lev_view(mg, l, bsw);
@@ -853,7 +848,7 @@ __device__ void mg_block_cycle(const Mg& mg, int lo) {
             C.r[I] = rr;
             if (smooth) C.e[I] = mg.omega * iv * rr;
         }
-        group_bar<NT>();
+        __syncthreads();
     }
     {
         // coarsest level: e = A_c^-1 r, one warp per row (lanes split the
@@ -885,14 +880,14 @@ __device__ void mg_block_cycle(const Mg& mg, int lo) {
                 if (lane == 0 && i < n) out[i] = ldc(L.invd, i) > 0.f ? a : 0.f;
             }
         }
-        group_bar<NT>();
+        __syncthreads();
     }
     for (int l = mg.nlev - 1; l >= lo; l--) {
         const MgLevel L = l == lo ? mg.lev[lo] : lev_view(mg, l, bsw);
         const MgLevel C = lev_view(mg, l + 1, bsw);
         const int n = L.nx * L.ny;
         for (int I = tid; I < n; I += nt) L.t[I] = ldc(L.invd, I) > 0.f ? smooth_up_cell(mg, L, C, I) : 0.f;
-        group_bar<NT>();
+        __syncthreads();
         if (l > lo) bsw ^= 1u << l;
     }
 }
@@ -1291,14 +1286,11 @@ __device__ __forceinline__ const float* split_correction(const Mg& mg, const flo
 // were written: a grid barrier, the grid-wide levels down (restriction
 // fused with the next level's pre-smoothing), the small levels in the
 // group's first block, the grid-wide levels up (prolongation folded into the post-smoothing), each
-// phase closed by a grid barrier of the thread group NT (0: whole blocks).
-// Afterwards level 1's correction is complete for every block
-// (level1_correction).  sync_first = false skips the first barrier where
-// the caller passed one since level 1 was written.  swp: the role swaps.
-template <int NT>
+// phase closed by a grid barrier.  Afterwards level 1's correction is complete for
+// every block (level1_correction).  swp: the role swaps.
 __device__ __forceinline__ bool mg_cell_levels(const Mg& mg, uint32_t& swp, GridBar& gb, DevStats* ds,
-                                               int gcell, int gsz, bool sync_first = true) {
-    if (sync_first && !grid_sync<NT>(gb, ds)) return false;
+                                               int gcell, int gsz) {
+    if (!grid_sync(gb, ds)) return false;
     const int lo = mg.ngrid + 1;
     // grid-wide levels, down: restrict level l into l+1 and pre-smooth there
     // (every level but the coarsest, whose e comes from its dense inverse),
@@ -1316,11 +1308,11 @@ __device__ __forceinline__ bool mg_cell_levels(const Mg& mg, uint32_t& swp, Grid
             C.r[I] = rr;
             if (smooth) C.e[I] = mg.omega * iv * rr;
         }
-        if (!grid_sync<NT>(gb, ds)) return false;
+        if (!grid_sync(gb, ds)) return false;
     }
     // small levels in the group's first block
-    if (gb.rank == 0) mg_block_cycle<NT>(mg, lo);
-    if (!grid_sync<NT>(gb, ds)) return false;
+    if (gb.rank == 0) mg_block_cycle(mg, lo);
+    if (!grid_sync(gb, ds)) return false;
     // grid-wide levels, up: prolongation folded into the post-smoothing
     for (int l = mg.ngrid; l >= 1; l--) {
         const MgLevel L = lev_view(mg, l, swp);
@@ -1330,7 +1322,7 @@ __device__ __forceinline__ bool mg_cell_levels(const Mg& mg, uint32_t& swp, Grid
             const int I = __ldg(L.act + a);
             L.t[I] = smooth_up_cell(mg, L, C, I);
         }
-        if (!grid_sync<NT>(gb, ds)) return false;
+        if (!grid_sync(gb, ds)) return false;
         swp ^= 1u << l;
     }
     return true;
@@ -1436,7 +1428,7 @@ __device__ __forceinline__ bool mg_vcycle(const Mg& mg, uint32_t& swp, const Ppe
     } else {
         mg_level1_plain(mg, mf, src0, gcell, gsz, level1_presmooth(mg, swp));
     }
-    if (!mg_cell_levels<0>(mg, swp, gb, ds, gcell, gsz)) return false;
+    if (!mg_cell_levels(mg, swp, gb, ds, gcell, gsz)) return false;
     // level 1's correction
     const float* __restrict__ e1 = level1_correction(mg, swp);
     if (mg.additive && mg.smooth) {
@@ -2331,7 +2323,6 @@ void solver_setup(Krylov& k, int32_t /*n_pad*/, int device) {
     int g3 = std::min(coop_grid((const void*)k_cg_mixed_ov<kCycleThreads>, device, kMixedBlock, kSplitSmem, 1),
                       coop_grid((const void*)k_cg_mixed_ov<kStreamCycle>, device, kMixedBlock, kStreamSmem, 1));
     k.grid = std::min({g1, g2, g3});
-    k.block = kBlock;
     k.cluster = cluster_blocks();
     k.cluster64 = cg64_cluster();
 }
