@@ -127,8 +127,7 @@ int mps_set_solver(mps_engine* e, int32_t precision, double tol, int64_t max_ite
  * the multiplicative V(1,1) cycle from the particle level (three operator
  * passes per iteration).  omega = Jacobi weight in (0,1], scale =
  * coarse-correction weight in [1,2); 0 picks the mode's default (modes 1,
- * 3 and 4: 1.0, 1.4, between the cell levels 1.6 in modes 1 and 4; mode 2:
- * 0.9, 1.5).  No counterpart in the reference (its
+ * 3 and 4: 1.0, 1.4; mode 2: 0.9, 1.5).  No counterpart in the reference (its
  * CG is Jacobi-preconditioned). */
 int mps_set_multigrid(mps_engine* e, int32_t mode, float omega, float scale);
 

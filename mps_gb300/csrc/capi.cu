@@ -478,20 +478,15 @@ int run_one_step(mps_engine* e, bool do_export, mps_step_stats* stats) {
 // the same omega on Galerkin 9-point stencils, whose Jacobi spectrum
 // D^-1 A_c stays well below 2, so undamped Jacobi still smooths there;
 // omega 1, s 1.4 took the fewest CG iterations on the 1M dam break (69 vs
-// 73 at 0.9/1.5).  Between the cell levels, where an aggregate is a plain 2x2
-// of a 9-point grid, a larger scale fits: 1.6 against 1.4 takes 40 instead of
-// 44 iterations (45,000-particle dam break) and 44 instead of 49 (200,000-
-// particle tank); 1.7 saves one more there but costs 4 % on a shaken column.
-// Multiplicative (mode 2) smooths the particle matrix itself, whose D^-1 A can
-// approach 2: there the damped 0.9 stays.
-void mg_default_weights(int mode, float* omega, float* scale, float* cscale) {
+// 73 at 0.9/1.5).  Multiplicative (mode 2) smooths the particle matrix
+// itself, whose D^-1 A can approach 2: there the damped 0.9 stays.
+void mg_default_weights(int mode, float* omega, float* scale) {
     if (mode == 2) {
         *omega = 0.9f;
-        *scale = *cscale = 1.5f;
+        *scale = 1.5f;
     } else {
         *omega = 1.0f;
         *scale = 1.4f;
-        *cscale = mode == 3 ? 1.4f : 1.6f;
     }
 }
 
@@ -669,7 +664,7 @@ int mps_create(const mps_params* prm, int32_t n, const double* pos, const double
     if (c.planar) {
         Mg& g = e->mg;
         g.enabled = 1;
-        mg_default_weights(1, &g.omega, &g.scale, &g.cscale);
+        mg_default_weights(1, &g.omega, &g.scale);
         g.additive = 1;
         int nx = c.numX, ny = c.numY, l = 1;
         for (;;) {
@@ -789,9 +784,8 @@ int mps_set_multigrid(mps_engine* e, int32_t mode, float omega, float scale) {
     if (mode < 0 || mode > 4) return fail(MPS_ERR_ARG, "multigrid mode must be 0, 1, 2, 3 or 4");
     if (mode && !e->mg.enabled)
         return fail(MPS_ERR_ARG, "multigrid needs a planar scene (2-D, constant z)");
-    float dw, ds, dc;
-    mg_default_weights(mode, &dw, &ds, &dc);
-    const float cscale = scale == 0.f ? dc : scale;  // a scale of the caller's holds on every level
+    float dw, ds;
+    mg_default_weights(mode, &dw, &ds);
     if (omega == 0.f) omega = dw;
     if (scale == 0.f) scale = ds;
     if (!(omega > 0.f && omega <= 1.f) || !(scale >= 1.f && scale < 2.f))
@@ -800,7 +794,6 @@ int mps_set_multigrid(mps_engine* e, int32_t mode, float omega, float scale) {
     e->mg_requested = mode;
     e->mg.omega = omega;
     e->mg.scale = scale;
-    e->mg.cscale = cscale;
     return MPS_OK;
 }
 

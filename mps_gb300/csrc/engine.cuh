@@ -279,8 +279,7 @@ struct Mg {
     float* res0;    // level-0 residual (per slot)
     float* dense;   // inverse of the coarsest operator (cells x cells of level nlev)
     float omega;    // damped-Jacobi weight
-    float scale;    // scale of the cells' correction at the particles
-    float cscale;   // scale of a coarser level's correction at the cells
+    float scale;    // coarse-correction scale
     // 0: multiplicative V(1,1) from level 0 (Jacobi pre- and post-smoothing
     // around the coarse correction); 1: additive at level 0, u = omega D^-1 r
     // + scale P V1(P^T r) (no level-0 operator pass; still SPD)

@@ -766,14 +766,14 @@ __device__ __forceinline__ float restrict_cell(const MgLevel& F, const MgLevel& 
 }
 
 // Post-smoothing of a level with the prolongation folded in: the corrected
-// value of a cell is e + cscale * e_parent, computed on the fly for the cell and
+// value of a cell is e + s * e_parent, computed on the fly for the cell and
 // its 8 neighbours, so prolongation needs no pass or barrier of its own.
 // Taps clamped and masked: all loads in one batch.
 __device__ __forceinline__ float smooth_up_cell(const Mg& mg, const MgLevel& L, const MgLevel& C,
                                                 int I) {
     const int n = L.nx * L.ny;
     const int x = I / L.ny, y = I - x * L.ny;
-    const float ei = fmaf(mg.cscale, ldv(C.e, (x / 2) * C.ny + y / 2), ldv(L.e, I));
+    const float ei = fmaf(mg.scale, ldv(C.e, (x / 2) * C.ny + y / 2), ldv(L.e, I));
     float st[9], ej[9];
     bool ok[9];
 #pragma unroll
@@ -781,7 +781,7 @@ __device__ __forceinline__ float smooth_up_cell(const Mg& mg, const MgLevel& L, 
         const int j = tap(L, x, y, d, ok[d]);
         const int jx = j / L.ny, jy = j - jx * L.ny;
         st[d] = ldc(L.st, (size_t)d * n + I);
-        ej[d] = fmaf(mg.cscale, ldv(C.e, (jx / 2) * C.ny + jy / 2), ldv(L.e, j));
+        ej[d] = fmaf(mg.scale, ldv(C.e, (jx / 2) * C.ny + jy / 2), ldv(L.e, j));
     }
     const float iv = ldc(L.invd, I), ri = ldv(L.r, I);
     float acc = 0.f;
@@ -1135,7 +1135,7 @@ __device__ __forceinline__ float smooth_cell(const Mg& mg, const MgLevel& L, int
     for (int d = 0; d < 9; d++) {
         const int jx = min(max(x + d / 3 - 1, 0), L.nx - 1), jy = min(max(y + d % 3 - 1, 0), L.ny - 1);
         w[d] = st(d);
-        ej[d] = fmaf(mg.cscale, corr[(jx >> 1) * cny + (jy >> 1)], e(jx * L.ny + jy));
+        ej[d] = fmaf(mg.scale, corr[(jx >> 1) * cny + (jy >> 1)], e(jx * L.ny + jy));
     }
     float acc = 0.f;
 #pragma unroll
