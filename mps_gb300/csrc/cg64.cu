@@ -633,9 +633,9 @@ constexpr int kSmem64 = 224 * 1024;
 // together); fewer: 512 (cheaper block barriers).
 constexpr int kWideSlices = 32;
 
-// Largest scene of the one-cluster form: per iteration 5.2 to 5.5 us up to 2,000
-// rows and 6.5 at 3,400 (16 SMs issue all the FP64 work) against 7.5 to 8.2 us
-// for one block per SM at 4,500 to 11,000.
+// Largest scene of the one-cluster form (16 SMs issue all the FP64 work), per iteration
+// against one block per SM: 5.5 and 7.5 us at 2,006 rows, 6.4 and 7.6 at 3,172, 6.9 and
+// 7.7 at 4,078, 8.0 and 7.9 at 4,805, 8.5 and 8.1 at 5,902, 10.2 and 8.0 at 8,068.
 constexpr int kClusterRows64 = 4000;
 
 template <int BS>

@@ -14,7 +14,10 @@ namespace mpsg {
 // instruction holds its SM quarter for 64 cycles: while there are no more warps
 // than SM quarters (608), one-warp blocks give every warp a quarter of its own
 // (2,000 particles: 68 SMs instead of 9; all of an FP64 step but the solve 0.43 ->
-// 0.40 ms when the blocks changed).
+// 0.40 ms when the blocks changed).  The lines are flat: the same with blocks of 32, 64 and
+// 256 threads, planar tanks in us, mixed: 16,606 particles 174, 165, 180; 23,988: 224, 210,
+// 216; 47,688: 260, 261, 277; 75,564: 317, 302, 303; 114,164: 378, 384, 362; FP64: 9,190:
+// 162, 165, 164; 16,606: 196, 193, 208; 47,688: 315, 312, 360; 93,872: 450, 442, 490.
 inline int block_threads(int n) { return n <= 20000 ? 32 : n <= 80000 ? 64 : 256; }
 inline int block_count(int n) { return (n + block_threads(n) - 1) / block_threads(n); }
 

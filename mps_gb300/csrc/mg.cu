@@ -1,5 +1,5 @@
 // Setup of the aggregation multigrid preconditioner used by the mixed
-// pressure solver (the V-cycle itself runs inside k_cg_mixed, solver.cu).
+// pressure solver (the V-cycle itself runs inside the mixed solves, solver.cu).
 //
 // Level 1: one unknown per bucket cell (numX x numY, cell index
 // cx * numY + cy, the planar cell key).  Its operator is the Galerkin

@@ -434,7 +434,7 @@ __device__ __forceinline__ double spmv64_row(const Ppe& A, int K, int sl, int la
 // complete before a barrier's acquire), and the operator's pass it by.  Per inner
 // iteration, gathers from L2 -> from L1 -> and operator past L1: 1.02 M
 // rows 100.9 -> 100.7 -> 96.3 us, 109,202 rows 31.0 -> 30.0 -> 30.0, a 3-D box of
-// 17,343 rows 13.2 -> 11.2 -> 11.1.
+// 17,343 rows 13.2 -> 11.2 -> 11.1 (before its rows' list-order sums).
 __device__ __forceinline__ float4 ldg_once(const float4* p) {
     float4 v;
     asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
@@ -2253,8 +2253,9 @@ SolveArgs make_args(const Consts& c, double tol, int64_t max_iter) {
 
 namespace {
 // Largest scene of the one-cluster solve.  Its 16 SMs take, per inner iteration,
-// 15.0 us at 2,162 rows, 17.5 at 4,400, 16.7 at 7,456, 20.4 at 11,312 and 27.6 at
-// 21,424, against 17.0, 18.4, 16.9, 17.9 and 20.1 for the grid of 152 blocks: the
+// 15.0 us at 2,162 rows, 16.0 at 3,765, 16.6 at 7,540, 17.1 at 8,068, 17.8 at 9,672, 20.2
+// at 11,312 and 27.6 at 21,424, against 17.0, 17.1, 17.2, 17.5, 17.6, 18.2 and 20.1 for
+// the grid of 152 blocks (whole steps at 8,068 rows 0.907 and 0.919 ms): the
 // line lies where the operator pass on 16 SMs has eaten up what the cluster's
 // barriers save.
 constexpr int kClusterRows = 8000;
@@ -2266,8 +2267,9 @@ constexpr int kSplitLevels = 136 * 1024;
 // Above kStreamRows rows the iteration is bound by the operator pass rather
 // than by the cycle's latency, and its loads in flight and gathered vector need
 // the L1 that shared memory takes away: less shared memory (one more grid-wide
-// level) and fewer cycle warps.  Per inner iteration, without and with: 109,202
-// rows 30.0 and 34.0 us, 208,240 rows 35.8 and 32.8, 1M rows 171 and 108 when the
+// level) and fewer cycle warps.  Per inner iteration, without and with: 93,872 rows
+// 24.6 and 26.0 us, 124,534: 28.7 and 29.1, 150,069: 31.7 and 32.2, 165,152: 34.3 and
+// 34.3, 205,565: 35.2 and 32.8, 306,796: 41.3 and 40.7, 1M rows 171 and 108 when the
 // line was first drawn.
 constexpr int kStreamRows = 150000;
 constexpr int kStreamLevels = 40 * 1024;

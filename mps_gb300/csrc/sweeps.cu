@@ -17,10 +17,13 @@ constexpr int kThreads = 256;
 // Up to kRowSplit particles the sweeps run with one warp per slot range of a
 // particle's 27 (9) cells: one warp for all of them leaves a scene of 17,000
 // particles fewer warps than SM quarters, each bound by one particle's serial
-// chain.  Split and not, the sweeps' kernels and all
-// of a step but the solve: 3-D box of 17,343 particles 0.92 -> 0.48 ms, dam of 2,162
-// 0.19 -> 0.14 (mixed) and 0.23 -> 0.15 (FP64); nothing at 50,469 (0.26 ms both) and
-// a loss at 109,202 (0.44 -> 0.50).
+// chain.  All of a step but the solve, one thread per particle and split: 3-D box of
+// 17,343 particles 0.92 and 0.48 ms; dam of 2,162 0.19 and 0.14 (mixed), 0.23 and 0.15
+// (FP64); planar tanks, mixed / FP64, of 9,190 particles 194 and 148 / 225 and 166 us,
+// 16,606: 214 and 173 / 246 and 196, 20,272: 203 and 180 / 243 and 206, 23,988: 212 and
+// 189 / 250 and 217, 32,173: 218 and 213 / 265 and 252, 47,688: 258 and 274 / 319 and
+// 318, 93,872 mixed 348 and 396.  The gain is gone between 32,000 and 48,000; from 20,000
+// on it is below 3 % of a mixed step and 1 % of an FP64 one.
 constexpr int kRowSplit = 20000;
 template <bool PLANAR>
 constexpr int kRows = PLANAR ? 3 : 9;
